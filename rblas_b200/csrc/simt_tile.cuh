@@ -232,29 +232,57 @@ __device__ __forceinline__ bool dmma_mainloop(double (&acc)[8][4], int num_kt, c
     return true;
 }
 
-// Compute warps: consume num_kt stages from ring iteration it into the
-// thread's 8 x TN accumulator. Returns false if a wait gave up.
-template <typename T, bool A_K, bool B_K, int V = 0>
-__device__ __forceinline__ bool simt_mainloop(T (&acc)[8][SimtCfg<T, V>::TN], int num_kt, const uint8_t* smem,
-                                              int stage_stride, uint64_t* full, uint64_t* empty, uint32_t& it,
-                                              uint32_t* err, int warp, int lane) {
-    if constexpr (sizeof(T) == 8) {
-        return dmma_mainloop<A_K, B_K>(acc, num_kt, smem, stage_stride, full, empty, it, err, warp, lane);
-    }
-    using Cfg = SimtCfg<T, V>;
+// ---- f32 on the CUDA cores ---------------------------------------------------
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack_f32x2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack_f32x2(f32x2 v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ void fma_f32x2(f32x2& c, f32x2 a, f32x2 b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+}
+
+template <bool PACKED> struct PairAcc { using type = f32x2; };
+template <> struct PairAcc<false> { using type = float; };
+
+template <bool A_K, bool B_K, int V>
+__device__ __forceinline__ bool f32_mainloop(float (&acc)[8][SimtCfg<float, V>::TN], int num_kt, const uint8_t* smem,
+                                               int stage_stride, uint64_t* full, uint64_t* empty, uint32_t& it,
+                                               uint32_t* err, int warp, int lane) {
+    using Cfg = SimtCfg<float, V>;
     constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, TN = Cfg::TN, ST = Cfg::STAGES;
-    constexpr int VEC = Vec16<T>::N;  // elements per 16-byte load
-    constexpr int A_BYTES = simt_a_bytes<T, V>();
-    static_assert(BK * sizeof(T) == 128, "a K-major tile row must be one 128-byte swizzle row");
+    constexpr int VEC = Vec16<float>::N;  // elements per 16-byte load
+    constexpr int A_BYTES = simt_a_bytes<float, V>();
+    static_assert(BK * sizeof(float) == 128, "a K-major tile row must be one 128-byte swizzle row");
     static_assert(A_BYTES % 1024 == 0, "swizzled tiles need 1 KiB alignment");
     const int wm = warp & 1, wn = warp >> 1;          // 2 x 4 warps
     const int lane_m = lane & 7, lane_n = lane >> 3;  // 8 x 4 lanes
     const int wm0 = wm * 64, wn0 = wn * (4 * TN);
 
+    // FFMA2 (fma.rn.f32x2) does two of a lane's FMAs per instruction. A
+    // lane's FMAs and the instructions around them share the issue and
+    // register-read slots, so half as many instructions per FMA is what it
+    // saves: each element's chain is the same fma sequence in k order and the
+    // bits are those of scalar FFMA. The accumulators are register pairs
+    // along the dimension of an MN-major operand, whose 16-byte reads are
+    // such pairs already; the other operand's value is repeated into both
+    // halves (one move). With both operands K-major the pairs of both would
+    // have to be assembled by moves, which cost more than FFMA2 saves (29
+    // against 43 TFLOP/s at 4096^3): that case stays on scalar FFMA.
+    // 4096^3, TFLOP/s, scalar -> FFMA2: A / B MN / MN-major 50.4 -> 60.4,
+    // MN / K 47.7 -> 55.3, K / MN 48.3 -> 52.8.
+    constexpr bool PACKED = !(A_K && B_K);
+    constexpr bool PAIR_M = !A_K;
+    constexpr int PI = PACKED && PAIR_M ? 4 : 8, PJ = PACKED && !PAIR_M ? TN / 2 : TN;
+    typename PairAcc<PACKED>::type acc2[PI][PJ];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < PI; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = T(0);
+        for (int j = 0; j < PJ; ++j) acc2[i][j] = 0;
 
     for (int kt = 0; kt < num_kt; ++kt, ++it) {
         const int s = it % ST;
@@ -263,8 +291,8 @@ __device__ __forceinline__ bool simt_mainloop(T (&acc)[8][SimtCfg<T, V>::TN], in
         const uint8_t* sb = sa + A_BYTES;
 #pragma unroll
         for (int kk = 0; kk < BK; kk += VEC) {
-            T a[VEC][8];
-            T b[VEC][TN];
+            float a[VEC][8];
+            float b[VEC][TN];
             const int chunk = kk / VEC;  // 16-byte chunk along k within a 128-byte row
             if constexpr (A_K) {
                 // [m][k] swizzled: a quarter-warp (same lane_n, lane_m 0..7)
@@ -272,8 +300,8 @@ __device__ __forceinline__ bool simt_mainloop(T (&acc)[8][SimtCfg<T, V>::TN], in
 #pragma unroll
                 for (int r = 0; r < 8; ++r) {
                     const int row = wm0 + lane_m + 8 * r;
-                    T v[VEC];
-                    lds16<T>(sa + row * 128 + ((chunk ^ (row & 7)) << 4), v);
+                    float v[VEC];
+                    lds16<float>(sa + row * 128 + ((chunk ^ (row & 7)) << 4), v);
 #pragma unroll
                     for (int q = 0; q < VEC; ++q) a[q][r] = v[q];
                 }
@@ -284,8 +312,8 @@ __device__ __forceinline__ bool simt_mainloop(T (&acc)[8][SimtCfg<T, V>::TN], in
 #pragma unroll
                     for (int g = 0; g < 8 / VEC; ++g) {
                         const int col = wm0 + g * 8 * VEC + lane_m * VEC;
-                        T v[VEC];
-                        lds16<T>(sa + ((kk + q) * BM + col) * sizeof(T), v);
+                        float v[VEC];
+                        lds16<float>(sa + ((kk + q) * BM + col) * sizeof(float), v);
 #pragma unroll
                         for (int e = 0; e < VEC; ++e) a[q][g * VEC + e] = v[e];
                     }
@@ -295,8 +323,8 @@ __device__ __forceinline__ bool simt_mainloop(T (&acc)[8][SimtCfg<T, V>::TN], in
 #pragma unroll
                 for (int j = 0; j < TN; ++j) {
                     const int row = wn0 + lane_n * TN + j;
-                    T v[VEC];
-                    lds16<T>(sb + row * 128 + ((chunk ^ (row & 7)) << 4), v);
+                    float v[VEC];
+                    lds16<float>(sb + row * 128 + ((chunk ^ (row & 7)) << 4), v);
 #pragma unroll
                     for (int q = 0; q < VEC; ++q) b[q][j] = v[q];
                 }
@@ -306,18 +334,33 @@ __device__ __forceinline__ bool simt_mainloop(T (&acc)[8][SimtCfg<T, V>::TN], in
 #pragma unroll
                     for (int g = 0; g < TN / VEC; ++g) {
                         const int col = wn0 + g * 4 * VEC + lane_n * VEC;
-                        T v[VEC];
-                        lds16<T>(sb + ((kk + q) * BN + col) * sizeof(T), v);
+                        float v[VEC];
+                        lds16<float>(sb + ((kk + q) * BN + col) * sizeof(float), v);
 #pragma unroll
                         for (int e = 0; e < VEC; ++e) b[q][g * VEC + e] = v[e];
                     }
             }
 #pragma unroll
-            for (int q = 0; q < VEC; ++q)
+            for (int q = 0; q < VEC; ++q) {
+                if constexpr (PACKED) {
+                    f32x2 ap[PI], bp[PJ];
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
+                    for (int i = 0; i < PI; ++i)
+                        ap[i] = PAIR_M ? pack_f32x2(a[q][2 * i], a[q][2 * i + 1]) : pack_f32x2(a[q][i], a[q][i]);
 #pragma unroll
-                    for (int j = 0; j < TN; ++j) acc[i][j] = fma(a[q][i], b[q][j], acc[i][j]);
+                    for (int j = 0; j < PJ; ++j)
+                        bp[j] = PAIR_M ? pack_f32x2(b[q][j], b[q][j]) : pack_f32x2(b[q][2 * j], b[q][2 * j + 1]);
+#pragma unroll
+                    for (int i = 0; i < PI; ++i)
+#pragma unroll
+                        for (int j = 0; j < PJ; ++j) fma_f32x2(acc2[i][j], ap[i], bp[j]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < PI; ++i)
+#pragma unroll
+                        for (int j = 0; j < PJ; ++j) acc2[i][j] = fmaf(a[q][i], b[q][j], acc2[i][j]);
+                }
+            }
         }
         // every lane's shared-memory reads of the stage are ordered before
         // the warp's release (lane 0's arrive orders only its own accesses,
@@ -327,7 +370,32 @@ __device__ __forceinline__ bool simt_mainloop(T (&acc)[8][SimtCfg<T, V>::TN], in
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[s]);
     }
+#pragma unroll
+    for (int i = 0; i < PI; ++i)
+#pragma unroll
+        for (int j = 0; j < PJ; ++j) {
+            if constexpr (!PACKED)     acc[i][j] = acc2[i][j];
+            else if constexpr (PAIR_M) unpack_f32x2(acc2[i][j], acc[2 * i][j], acc[2 * i + 1][j]);
+            else                       unpack_f32x2(acc2[i][j], acc[i][2 * j], acc[i][2 * j + 1]);
+        }
     return true;
+}
+
+// Compute warps: consume num_kt stages from ring iteration it into the
+// thread's 8 x TN accumulator. Returns false if a wait gave up.
+template <typename T, bool A_K, bool B_K, int V = 0>
+__device__ __forceinline__ bool simt_mainloop(T (&acc)[8][SimtCfg<T, V>::TN], int num_kt, const uint8_t* smem,
+                                              int stage_stride, uint64_t* full, uint64_t* empty, uint32_t& it,
+                                              uint32_t* err, int warp, int lane) {
+    if constexpr (sizeof(T) == 8)
+        return dmma_mainloop<A_K, B_K>(acc, num_kt, smem, stage_stride, full, empty, it, err, warp, lane);
+    else
+        return f32_mainloop<A_K, B_K, V>(acc, num_kt, smem, stage_stride, full, empty, it, err, warp, lane);
+}
+// Whether element (r, c) of C is this problem's to write (and C0's to read).
+template <typename T>
+__device__ __forceinline__ bool simt_live(const SimtOut<T>& o, int r, int c) {
+    return r < o.m && c < o.n && !(o.tri == 1 && r > c) && !(o.tri == 2 && r < c);
 }
 
 // Compute warps: C = alpha*acc + beta*Cin for the tile at (m0, n0).
@@ -342,44 +410,60 @@ __device__ __forceinline__ void simt_epilogue(const SimtOut<T>& o, const T (&acc
         const int g = lane >> 2, tq = lane & 3;
         const int wm0 = wm * 64, wn0 = wn * 16;
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int ig = 0; ig < 8; ig += 4) {  // 16 C0 values requested at a time
+            T cv[4][4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int r = m0 + wm0 + dmma_row<A_K>(i >> 1, q, g);
-                const int cidx = n0 + wn0 + dmma_col<B_K>(i & 1, q, tq);
-                if (r >= o.m || cidx >= o.n) continue;
-                if ((o.tri == 1 && r > cidx) || (o.tri == 2 && r < cidx)) continue;
-                T* cp = o.c + r + static_cast<size_t>(cidx) * o.ldc;
-                T tv = T(0);
-                if (o.beta_mode != 0) {
-                    const T cv = o.cin[r + static_cast<size_t>(cidx) * o.ldcin];
-                    tv = (o.beta_mode == 1) ? cv : o.beta * cv;
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int r = m0 + wm0 + dmma_row<A_K>((ig + i) >> 1, q, g);
+                    const int cidx = n0 + wn0 + dmma_col<B_K>((ig + i) & 1, q, tq);
+                    cv[i][q] = (o.beta_mode != 0 && simt_live(o, r, cidx))
+                                   ? o.cin[r + static_cast<size_t>(cidx) * o.ldcin] : T(0);
                 }
-                *cp = fma(o.alpha, acc[i][q], tv);
-            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int r = m0 + wm0 + dmma_row<A_K>((ig + i) >> 1, q, g);
+                    const int cidx = n0 + wn0 + dmma_col<B_K>((ig + i) & 1, q, tq);
+                    if (!simt_live(o, r, cidx)) continue;
+                    const T tv = (o.beta_mode == 2) ? o.beta * cv[i][q] : cv[i][q];
+                    o.c[r + static_cast<size_t>(cidx) * o.ldc] = fma(o.alpha, acc[ig + i][q], tv);
+                }
+        }
         return;
     }
     const int lane_m = lane & 7, lane_n = lane >> 3;
     const int wm0 = wm * 64, wn0 = wn * (4 * TN);
+    auto row = [&](int i) {
+        return m0 + (A_K ? (wm0 + lane_m + 8 * i) : (wm0 + (i / VEC) * 8 * VEC + lane_m * VEC + (i % VEC)));
+    };
+    auto col = [&](int j) {
+        return n0 + (B_K ? (wn0 + lane_n * TN + j) : (wn0 + (j / VEC) * 4 * VEC + lane_n * VEC + (j % VEC)));
+    };
+    // two rows at a time: their C0 values are requested together, before the
+    // stores (which might alias them, so the compiler keeps that order)
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int r = m0 + (A_K ? (wm0 + lane_m + 8 * i)
-                                : (wm0 + (i / VEC) * 8 * VEC + lane_m * VEC + (i % VEC)));
-        if (r >= o.m) continue;
+    for (int ig = 0; ig < 8; ig += 2) {
+        T cv[2][TN];
 #pragma unroll
-        for (int j = 0; j < TN; ++j) {
-            const int cidx = n0 + (B_K ? (wn0 + lane_n * TN + j)
-                                       : (wn0 + (j / VEC) * 4 * VEC + lane_n * VEC + (j % VEC)));
-            if (cidx >= o.n) continue;
-            if ((o.tri == 1 && r > cidx) || (o.tri == 2 && r < cidx)) continue;
-            T* cp = o.c + r + static_cast<size_t>(cidx) * o.ldc;
-            T t = T(0);
-            if (o.beta_mode != 0) {
-                const T cv = o.cin[r + static_cast<size_t>(cidx) * o.ldcin];
-                t = (o.beta_mode == 1) ? cv : o.beta * cv;
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+                const int r = row(ig + i), cidx = col(j);
+                cv[i][j] = (o.beta_mode != 0 && simt_live(o, r, cidx))
+                               ? o.cin[r + static_cast<size_t>(cidx) * o.ldcin] : T(0);
             }
-            *cp = fma(o.alpha, acc[i][j], t);
-        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+                const int r = row(ig + i), cidx = col(j);
+                if (!simt_live(o, r, cidx)) continue;
+                const T t = (o.beta_mode == 2) ? o.beta * cv[i][j] : cv[i][j];
+                o.c[r + static_cast<size_t>(cidx) * o.ldc] = fma(o.alpha, acc[ig + i][j], t);
+            }
     }
 }
 
