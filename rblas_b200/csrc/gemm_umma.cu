@@ -369,6 +369,348 @@ __global__ void __launch_bounds__(UCfg<MODE>::THREADS, 1)
 }
 
 // ------------------------------------------------------------------------------
+// The BF16-split GEMM on CTA pairs: 256 x 256 tiles, M = 256 N = 256 MMAs.
+//
+// An M = 128 N = 128 MMA reads both operands from shared memory at the full
+// 128 bytes per clock, and TMA's writes of the next stage come on top, so
+// umma_gemm_kernel's tensor pipe waits for shared memory. A pair's MMA reads
+// 128 rows of A and 128 of B per SM for twice the products: 64 bytes per
+// clock, and half the TMA bytes per product. Each CTA loads its 128 rows of
+// A and its 128 of B; the even CTA's warp 1 issues for both.
+// 3xBF16 alternates two accumulators of 256 columns. BF16X6 keeps hi*hi apart
+// (as umma_body does), which fills TMEM with one accumulator of each kind. A
+// drain takes ~1200 clocks from the last MMA to the even CTA's knowing (the
+// commit 300, the reads 340, the odd CTA's arrival 460), so a unit issues
+// its small products first and its hi*hi ones (1024 clocks) last: the small
+// accumulator drains behind hi*hi, and hi*hi's behind the next unit's small
+// products. The hi planes then outlive the others of their stage and have a
+// ring of their own. Within each accumulator the products keep umma_body's
+// order, so the results are its bits.
+// Per CTA: warp 0 TMA producer; warp 1 TMEM owner and, in the even CTA, MMA
+// issuer (in the odd one it passes on to the even CTA that a stage has
+// landed); warps 2..17 epilogue (four per TMEM lane quarter, 64 columns each).
+// 8192^3, us a call (split pass included), 128 x 128 tiles -> pairs: 3xBF16
+// 3316 -> 2404, BF16X6 5256 -> 4482; the GEMMs then run at 1.48 and 1.55
+// PFLOP/s of bf16 products (cuBLAS's burst 1.68), held by the power cap (SM
+// clock 1.55 GHz). A cluster-scope release in the epilogue's arrival, which
+// waits for the thread's stores, had cost BF16X6 850 us of that.
+// ------------------------------------------------------------------------------
+// KB: K bytes per stage row. Ring H holds the hi planes (HP of them per
+// stage; every plane for 3xBF16), ring L the others.
+template <int MODE> struct PairCfg;
+template <> struct PairCfg<kModeBf16x3> { static constexpr int KB = 128, HP = 2, HS = 3, LP = 0, LS = 0; };  // 3 x 64 KiB
+template <> struct PairCfg<kModeBf16x6> { static constexpr int KB = 64, HP = 1, HS = 6, LP = 2, LS = 4; };   // 6 x 16, 4 x 32 KiB
+constexpr int kPairN = 256;
+constexpr int kPairEpiWarps = 16;
+constexpr int kPairCols = kPairN / (kPairEpiWarps / 4);  // columns per epilogue warp
+constexpr int kPairThreads = 64 + 32 * kPairEpiWarps;
+constexpr int kPairBarBytes = 512;
+template <int MODE>
+constexpr int pair_smem_bytes() {
+    using P = PairCfg<MODE>;
+    return 2 * 128 * P::KB * (P::HP * P::HS + P::LP * P::LS) + kPairBarBytes + 1024;
+}
+static_assert(pair_smem_bytes<kModeBf16x3>() <= 232448 && pair_smem_bytes<kModeBf16x6>() <= 232448,
+              "the pair kernels' rings must fit one CTA's shared memory");
+
+struct PairBar {
+    uint64_t h_full[6], h_empty[6];
+    uint64_t l_full[4], l_empty[4];
+    uint64_t peer_full[4];  // even CTA: the odd CTA's stage has landed
+    uint64_t acc_full[2];
+    uint64_t acc_empty[2];  // even CTA: both CTAs' epilogue warps
+    uint64_t drain;
+    uint32_t tmem_base;
+};
+static_assert(sizeof(PairBar) <= kPairBarBytes, "shared memory reserved for the pair kernels' barriers");
+
+using f32pair = unsigned long long;
+__device__ __forceinline__ void add_f32pair(f32pair& s, uint32_t lo, uint32_t hi) {
+    f32pair v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(lo), "r"(hi));
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(s) : "l"(v));
+}
+
+template <int MODE>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
+    umma_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                     const __grid_constant__ UParams p) {
+    using Cfg = UCfg<MODE>;
+    using Pc = PairCfg<MODE>;
+    constexpr int NP = Cfg::NA, KB = Pc::KB, HS = Pc::HS, LS = Pc::LS, HP = Pc::HP;
+    constexpr int PL = 128 * KB;            // one plane's 128 rows
+    constexpr int HSTAGE = 2 * HP * PL;     // A's planes, then B's
+    constexpr int LSTAGE = 2 * Pc::LP * PL;
+    constexpr bool TWO = LS > 0;            // two rings
+    constexpr int PS = TWO ? LS : HS;       // slots of peer_full
+    constexpr int SUB = kRowBytes / KB;     // stages per 64-element K tile
+    constexpr int KSTEPS = KB / 32;
+    constexpr uint32_t IDESC = umma_idesc(1, 1, 256, kPairN);  // f32 <- bf16
+    constexpr bool SPLIT_ACC = (MODE == kModeBf16x6);
+    static_assert(Cfg::NB == NP && HP + Pc::LP == NP && HS <= 6 && LS <= 4 && PS <= 4 && SPLIT_ACC == TWO, "rings");
+
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    uint8_t* lring = smem + HS * HSTAGE;
+    PairBar* bar = reinterpret_cast<PairBar*>(lring + LS * LSTAGE);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_rank();
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < HS; ++s) {
+            mbar_init(&bar->h_full[s], 1);
+            mbar_init(&bar->h_empty[s], 1);
+        }
+        for (int s = 0; s < 4; ++s) {
+            mbar_init(&bar->l_full[s], 1);
+            mbar_init(&bar->l_empty[s], 1);
+            mbar_init(&bar->peer_full[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&bar->acc_full[b], 1);
+            mbar_init(&bar->acc_empty[b], 2 * kPairEpiWarps);
+        }
+        mbar_init(&bar->drain, 1);
+        fence_barrier_init();
+    }
+    if (warp == 1) tmem_alloc_pair(&bar->tmem_base, 512);
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();  // the other CTA's barriers are initialised too
+    tc_fence_after();
+    const uint32_t tmem_base = bar->tmem_base;
+    uint32_t* const err = p.err;
+    const int items = p.num_tiles, first = blockIdx.x >> 1, step = gridDim.x >> 1;
+    const int stages = p.num_kt * SUB, per_unit = p.kt_per_chunk * SUB;
+    bool ok = true;
+
+    if (warp == 0 && lane == 0) {
+        // ------------------------------ TMA producer ------------------------------
+        prefetch_tmap(&tmA);
+        prefetch_tmap(&tmB);
+        uint32_t nh = 0, nl = 0;  // stages issued
+        for (int item = first; ok && item < items; item += step) {
+            int tm, tn;
+            raster_tile(item, p.tiles_m, p.tiles_n, tm, tn);
+            const int m0 = tm * 256 + rank * 128, n0 = tn * kPairN + rank * 128;
+            for (int kt = 0; kt < stages; ++kt) {
+                const int k0 = kt * (KB / 2);
+                const uint32_t hs = nh % HS;
+                if (nh >= HS && !mbar_wait_cluster(&bar->h_empty[hs], ((nh / HS) - 1) & 1, err, 0x221)) {
+                    ok = false;
+                    break;
+                }
+                uint8_t* sh = smem + hs * HSTAGE;
+                mbar_arrive_expect_tx(&bar->h_full[hs], HSTAGE);
+#pragma unroll
+                for (int q = 0; q < HP; ++q) tma_load_3d(sh + q * PL, &tmA, &bar->h_full[hs], k0, m0, q);
+#pragma unroll
+                for (int q = 0; q < HP; ++q) tma_load_3d(sh + (HP + q) * PL, &tmB, &bar->h_full[hs], k0, n0, q);
+                ++nh;
+                if constexpr (TWO) {
+                    const uint32_t ls = nl % LS;
+                    if (nl >= LS && !mbar_wait_cluster(&bar->l_empty[ls], ((nl / LS) - 1) & 1, err, 0x229)) {
+                        ok = false;
+                        break;
+                    }
+                    uint8_t* sl = lring + ls * LSTAGE;
+                    mbar_arrive_expect_tx(&bar->l_full[ls], LSTAGE);
+#pragma unroll
+                    for (int q = 0; q < Pc::LP; ++q) tma_load_3d(sl + q * PL, &tmA, &bar->l_full[ls], k0, m0, HP + q);
+#pragma unroll
+                    for (int q = 0; q < Pc::LP; ++q)
+                        tma_load_3d(sl + (Pc::LP + q) * PL, &tmB, &bar->l_full[ls], k0, n0, HP + q);
+                    ++nl;
+                }
+            }
+        }
+        if (!ok) {  // this CTA's copies land before it exits
+            for (uint32_t j = nh > (uint32_t)HS ? nh - HS : 0; j < nh; ++j)
+                mbar_wait_drain(&bar->h_full[j % HS], (j / HS) & 1);
+            if constexpr (TWO)
+                for (uint32_t j = nl > (uint32_t)LS ? nl - LS : 0; j < nl; ++j)
+                    mbar_wait_drain(&bar->l_full[j % LS], (j / LS) & 1);
+        }
+    } else if (warp == 1 && lane == 0 && rank == 1) {
+        // ------------------- odd CTA: landed stages, told to the even one -------------------
+        uint32_t it = 0;
+        for (int item = first; ok && item < items; item += step)
+            for (int kt = 0; kt < stages; ++kt, ++it) {
+                if (!mbar_wait(&bar->h_full[it % HS], (it / HS) & 1, err, 0x222)) {
+                    ok = false;
+                    break;
+                }
+                if constexpr (TWO) {
+                    if (!mbar_wait(&bar->l_full[it % LS], (it / LS) & 1, err, 0x22a)) {
+                        ok = false;
+                        break;
+                    }
+                }
+                mbar_arrive_rank(&bar->peer_full[it % PS], 0);
+            }
+    } else if (warp == 1 && lane == 0) {
+        // ------------------------- even CTA: MMA issuer -------------------------
+        uint32_t it = 0, uc = 0;
+        auto landed = [&](uint32_t i) -> bool {  // stage i, in both CTAs
+            if (!mbar_wait(&bar->h_full[i % HS], (i / HS) & 1, err, 0x223)) return false;
+            if constexpr (TWO) {
+                if (!mbar_wait(&bar->l_full[i % LS], (i / LS) & 1, err, 0x22b)) return false;
+            }
+            if (!mbar_wait_cluster(&bar->peer_full[i % PS], (i / PS) & 1, err, 0x224)) return false;
+            tc_fence_after();
+            return true;
+        };
+        // A descriptor's low word is the address / 16 (plus a constant field)
+        // and its high word constant: the issuing thread keeps low words and
+        // adds constants, since the address arithmetic of a descriptor made
+        // anew takes longer than the 128 clocks of an MMA.
+        const uint64_t d0 = KB == 128 ? sw128_kmajor_desc(smem_u32(smem)) : sw64_kmajor_desc(smem_u32(smem));
+        const uint32_t h_lo = static_cast<uint32_t>(d0), d_hi = static_cast<uint32_t>(d0 >> 32);
+        const uint32_t l_lo = h_lo + HS * HSTAGE / 16;
+        // the products Q0..Q1-1 of a stage (ring slots hs, ls) into d
+        auto products = [&](uint32_t hs, uint32_t ls, auto q0, auto q1, uint32_t d, bool fresh) {
+            const uint32_t hb = h_lo + hs * (HSTAGE / 16), lb = l_lo + ls * (LSTAGE / 16);
+#pragma unroll
+            for (int kk = 0; kk < KSTEPS; ++kk)
+#pragma unroll
+                for (int q = decltype(q0)::value; q < decltype(q1)::value; ++q) {
+                    const int qa = Cfg::pa(q), qb = Cfg::pb(q);
+                    const uint32_t a = (qa < HP ? hb + qa * (PL / 16) : lb + (qa - HP) * (PL / 16)) + 2 * kk;
+                    const uint32_t b =
+                        (qb < HP ? hb + (HP + qb) * (PL / 16) : lb + (Pc::LP + qb - HP) * (PL / 16)) + 2 * kk;
+                    umma_f16_pair(d, (static_cast<uint64_t>(d_hi) << 32) | a, (static_cast<uint64_t>(d_hi) << 32) | b,
+                                  IDESC, (kk == 0 && q == decltype(q0)::value) ? (fresh ? 0u : 1u) : 1u);
+                }
+        };
+        using Q0 = std::integral_constant<int, 0>;
+        using QB = std::integral_constant<int, Cfg::NPROD - 1>;
+        using QN = std::integral_constant<int, Cfg::NPROD>;
+        uint32_t hs = 0, ls = 0;  // ring slots of the next stage
+        for (int item = first; ok && item < items; item += step) {
+            for (int u = 0; ok && u < p.kchunks; ++u, ++uc) {
+                const int n_st = min(per_unit, stages - u * per_unit);
+                if constexpr (!SPLIT_ACC) {
+                    const uint32_t b = uc & 1;
+                    if (uc >= 2 && !mbar_wait_cluster(&bar->acc_empty[b], ((uc >> 1) - 1) & 1, err, 0x225)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    for (int j = 0; ok && j < n_st; ++j, ++it) {
+                        ok = landed(it);
+                        if (!ok) break;
+                        products(hs, 0, Q0{}, QN{}, tmem_base + b * kPairN, j == 0);
+                        tc_commit_pair(&bar->h_empty[hs]);
+                        hs = hs + 1 == HS ? 0 : hs + 1;
+                    }
+                    if (ok) tc_commit_pair(&bar->acc_full[b]);
+                } else {
+                    if (uc >= 1 && !mbar_wait_cluster(&bar->acc_empty[0], (uc - 1) & 1, err, 0x226)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    uint32_t hj = hs;
+                    for (int j = 0; ok && j < n_st; ++j) {
+                        ok = landed(it + j);
+                        if (!ok) break;
+                        products(hj, ls, Q0{}, QB{}, tmem_base, j == 0);
+                        tc_commit_pair(&bar->l_empty[ls]);
+                        hj = hj + 1 == HS ? 0 : hj + 1;
+                        ls = ls + 1 == LS ? 0 : ls + 1;
+                    }
+                    if (!ok) break;
+                    tc_commit_pair(&bar->acc_full[0]);
+                    if (uc >= 1 && !mbar_wait_cluster(&bar->acc_empty[1], (uc - 1) & 1, err, 0x227)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    for (int j = 0; j < n_st; ++j, ++it) {
+                        products(hs, 0, QB{}, QN{}, tmem_base + kPairN, j == 0);
+                        tc_commit_pair(&bar->h_empty[hs]);
+                        hs = hs + 1 == HS ? 0 : hs + 1;
+                    }
+                    tc_commit_pair(&bar->acc_full[1]);
+                }
+            }
+        }
+        // nothing of ours is in flight before TMEM is released (arrives on the
+        // odd CTA's copy too, which nobody waits on)
+        tc_commit_pair(&bar->drain);
+        mbar_wait_drain(&bar->drain, 0);
+    } else if (warp >= 2) {
+        // ------------------------------ epilogue ------------------------------
+        const int quarter = warp & 3, cq = (warp - 2) >> 2;
+        const int row_in_tile = quarter * 32 + lane;
+        const uint32_t tbase = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + cq * kPairCols;
+        uint32_t uc = 0;
+        for (int item = first; ok && item < items; item += step) {
+            int tm, tn;
+            raster_tile(item, p.tiles_m, p.tiles_n, tm, tn);
+            const int r = tm * 256 + static_cast<int>(rank) * 128 + row_in_tile, n0 = tn * kPairN + cq * kPairCols;
+            f32pair sum[kPairCols / 2];
+#pragma unroll
+            for (int j = 0; j < kPairCols / 2; ++j) sum[j] = 0ull;
+            for (int u = 0; ok && u < p.kchunks; ++u, ++uc) {
+                // the smaller products first, then hi*hi (SPLIT_ACC)
+#pragma unroll 1
+                for (int part = 0; part < (SPLIT_ACC ? 2 : 1); ++part) {
+                    const uint32_t b = SPLIT_ACC ? part : (uc & 1);
+                    const uint32_t ph = SPLIT_ACC ? (uc & 1) : ((uc >> 1) & 1);
+                    const bool got = mbar_wait_cluster(&bar->acc_full[b], ph, err, 0x228);
+                    if (!__all_sync(0xffffffffu, got)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+#pragma unroll
+                    for (int ch = 0; ch < kPairCols / 16; ++ch) {
+                        uint32_t v[16];
+                        tmem_ld16(tbase + b * kPairN + ch * 16, v);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) add_f32pair(sum[ch * 8 + j], v[2 * j], v[2 * j + 1]);
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_rank_relaxed(&bar->acc_empty[b], 0);
+                }
+            }
+            if (ok && r < p.m) {
+                // C0 read 16 values at a time, all requested before use
+#pragma unroll
+                for (int g = 0; g < kPairCols / 16; ++g) {
+                    float cv[16];
+#pragma unroll
+                    for (int jj = 0; jj < 16; ++jj) {
+                        const int col = n0 + g * 16 + jj;
+                        cv[jj] = (p.beta_mode != 0 && col < p.n) ? p.cin[r + static_cast<size_t>(col) * p.ldc] : 0.f;
+                    }
+#pragma unroll
+                    for (int jj = 0; jj < 16; ++jj) {
+                        const int col = n0 + g * 16 + jj;
+                        if (col < p.n) {
+                            float lo, hi;
+                            asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(sum[g * 8 + jj / 2]));
+                            const float tb = (p.beta_mode == 2) ? p.beta_f * cv[jj] : cv[jj];
+                            p.c[r + static_cast<size_t>(col) * p.ldc] = fmaf(p.alpha_f, (jj & 1) ? hi : lo, tb);
+                        }
+                    }
+                }
+            }
+        }
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();  // no CTA leaves while the other may still reach its memory
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc_pair(tmem_base, 512);
+    }
+}
+
+// ------------------------------------------------------------------------------
 // The BF16-split forms with A split inside the GEMM (A rows contiguous:
 // NoTrans).
 //
@@ -1653,9 +1995,10 @@ __global__ void __launch_bounds__(256) bf16_split_grouped_kernel(const BsOperand
 }
 
 CUresult make_tmap_planes(CUtensorMap* map, const void* base, CUtensorMapDataType dtype, size_t elem,
-                          uint64_t k, uint64_t rows, uint64_t planes, uint64_t kp, uint32_t box_rows) {
-    return make_tmap_3d(map, base, dtype, elem, k, rows, planes, kp, kp * rows, kRowBytes / elem,
-                        box_rows, 1, true);
+                          uint64_t k, uint64_t rows, uint64_t planes, uint64_t kp, uint32_t box_rows,
+                          int row_bytes = kRowBytes) {
+    return make_tmap_3d(map, base, dtype, elem, k, rows, planes, kp, kp * rows, row_bytes / elem,
+                        box_rows, 1, row_bytes);
 }
 
 template <int MODE>
@@ -1677,6 +2020,26 @@ cudaError_t launch_umma(const CUtensorMap& ta, const CUtensorMap& tb, const UPar
     KernelTimer tm;
     kernel_timing_begin(name, work, st, &tm);
     kern<<<grid, UCfg<MODE>::THREADS, smem, st>>>(ta, tb, p);
+    kernel_timing_end(&tm, st);
+    count_launch();
+    return cudaGetLastError();
+}
+
+template <int MODE>
+cudaError_t launch_umma_pair(const CUtensorMap& ta, const CUtensorMap& tb, const UParams& p, int sms, cudaStream_t st) {
+    auto kern = umma_pair_kernel<MODE>;
+    constexpr int smem = pair_smem_bytes<MODE>();
+    static bool attr = false;
+    if (!attr) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+        attr = true;
+    }
+    const int grid = 2 * std::min(p.num_tiles, sms / 2);
+    KernelTimer tm;
+    kernel_timing_begin((MODE == kModeBf16x3) ? "umma_bf16x3" : "umma_bf16x6",
+                        2.0 * p.m * p.n * static_cast<double>(p.k) * UCfg<MODE>::NPROD, st, &tm);
+    kern<<<grid, kPairThreads, smem, st>>>(ta, tb, p);
     kernel_timing_end(&tm, st);
     count_launch();
     return cudaGetLastError();
@@ -1776,6 +2139,19 @@ bool bf16_fused_a(bool ta, int n, const float* A, size_t lda) {
     return !ta && n <= 256 && (reinterpret_cast<uintptr_t>(A) & 15) == 0 && (lda & 3) == 0;
 }
 
+// Whether an m x n product runs on CTA pairs (256 x 256 tiles) rather than
+// 128 x 128 tiles: by the number of waves, one of pairs taking 1.7 times one of
+// small tiles (BF16X6; 3xBF16 1.4) for four times the C per pair of SMs.
+// Measured per wave: 8192^3 305 against 180 us (X6), 159 against 112 (3x);
+// 2048^3 88 against 52, 50 against 39. One wave of either (777 x 999 x 1234,
+// X6): 77 us on pairs, 56 on small tiles.
+bool bf16_pair_tiles(int planes, int m, int n, int sms) {
+    const long t128 = static_cast<long>((m + 127) / 128) * ((n + 127) / 128);
+    const long t256 = static_cast<long>((m + 255) / 256) * ((n + 255) / 256);
+    const long w128 = (t128 + sms - 1) / sms, w256 = (t256 + sms / 2 - 1) / std::max(sms / 2, 1);
+    return sms >= 2 && (planes == 2 ? 14 : 17) * w256 < 10 * w128;
+}
+
 template <int MODE>
 cudaError_t launch_bf16_fused(const CUtensorMap& ta32, const CUtensorMap& tb, const UParams& p, cudaStream_t st) {
     auto kern = umma_split_fused_kernel<MODE>;
@@ -1802,8 +2178,12 @@ cudaError_t launch_bf16_fused(const CUtensorMap& ta32, const CUtensorMap& tb, co
 cudaError_t launch_bf16_split_gemm(int planes, bool ta, bool tb, int m, int n, int k, float alpha,
                                    const float* A, size_t lda, const float* B, size_t ldb, float beta,
                                    float* C, size_t ldc, cudaStream_t st, CUresult* cu_err) {
-    constexpr int UN = 128;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const bool fused = bf16_fused_a(ta, n, A, lda);
+    const bool pair = !fused && bf16_pair_tiles(planes, m, n, sms);
+    const int UM = pair ? 256 : kUM, UN = pair ? kPairN : 128;
     const size_t kp = round_up(static_cast<size_t>(k), 8);  // 16-byte rows of bf16
     const size_t pa = fused ? 0 : static_cast<size_t>(m) * kp, pb = static_cast<size_t>(n) * kp;
     void* buf = nullptr;
@@ -1822,12 +2202,14 @@ cudaError_t launch_bf16_split_gemm(int planes, bool ta, bool tb, int m, int n, i
     }
     bf16_split_kernel<<<gb, 256, 0, st>>>(B, brs, bps, n, k, planes, sb, kp, pb);
     count_launch();
+    // rows of the plane boxes: one stage's K (BF16X6 pairs take half a K tile)
+    const int rb = (pair && planes == 3) ? PairCfg<kModeBf16x6>::KB : kRowBytes;
     CUtensorMap tma, tmb;
     // fused: A itself as an m x k f32 tensor, 128-row x 64-column boxes
     CUresult r = fused ? make_tmap_2d(&tma, A, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, sizeof(float), m, k, lda, kUM, 64,
                                       false)
-                       : make_tmap_planes(&tma, sa, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, k, m, planes, kp, kUM);
-    if (r == CUDA_SUCCESS) r = make_tmap_planes(&tmb, sb, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, k, n, planes, kp, UN);
+                       : make_tmap_planes(&tma, sa, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, k, m, planes, kp, 128, rb);
+    if (r == CUDA_SUCCESS) r = make_tmap_planes(&tmb, sb, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, k, n, planes, kp, 128, rb);
     if (r != CUDA_SUCCESS) {
         if (cu_err) *cu_err = r;
         cudaFreeAsync(buf, st);
@@ -1835,7 +2217,7 @@ cudaError_t launch_bf16_split_gemm(int planes, bool ta, bool tb, int m, int n, i
     }
     UParams p{};
     p.m = m; p.n = n; p.k = k;
-    p.tiles_m = (m + kUM - 1) / kUM;
+    p.tiles_m = (m + UM - 1) / UM;
     p.tiles_n = (n + UN - 1) / UN;
     p.num_tiles = p.tiles_m * p.tiles_n;
     p.num_kt = static_cast<int>((k + 63) / 64);
@@ -1846,7 +2228,10 @@ cudaError_t launch_bf16_split_gemm(int planes, bool ta, bool tb, int m, int n, i
     p.c = C; p.ldc = ldc;
     p.cin = C;
     p.err = device_error_word();
-    if (fused)
+    if (pair)
+        e = (planes == 2) ? launch_umma_pair<kModeBf16x3>(tma, tmb, p, sms, st)
+                          : launch_umma_pair<kModeBf16x6>(tma, tmb, p, sms, st);
+    else if (fused)
         e = (planes == 2) ? launch_bf16_fused<kModeBf16x3>(tma, tmb, p, st)
                           : launch_bf16_fused<kModeBf16x6>(tma, tmb, p, st);
     else

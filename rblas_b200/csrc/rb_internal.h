@@ -32,10 +32,11 @@ CUresult make_tmap_2d(CUtensorMap* map, const void* base, CUtensorMapDataType dt
                       uint32_t box_cols, bool swizzle128);
 
 // 3-D tiled tensor map: dims d0 (contiguous), d1, d2; strides s1, s2 in
-// elements between consecutive d1 / d2 indices; box b0 x b1 x b2.
+// elements between consecutive d1 / d2 indices; box b0 x b1 x b2. swizzle_bytes:
+// 128 or 64 (b0*elem bytes), else none.
 CUresult make_tmap_3d(CUtensorMap* map, const void* base, CUtensorMapDataType dtype, size_t elem,
                       uint64_t d0, uint64_t d1, uint64_t d2, uint64_t s1, uint64_t s2,
-                      uint32_t b0, uint32_t b1, uint32_t b2, bool swizzle128);
+                      uint32_t b0, uint32_t b1, uint32_t b2, int swizzle_bytes);
 
 // ---- launch bookkeeping ----------------------------------------------------------
 

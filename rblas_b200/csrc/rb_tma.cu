@@ -39,7 +39,7 @@ CUresult make_tmap_2d(CUtensorMap* map, const void* base, CUtensorMapDataType dt
 
 CUresult make_tmap_3d(CUtensorMap* map, const void* base, CUtensorMapDataType dtype, size_t elem,
                       uint64_t d0, uint64_t d1, uint64_t d2, uint64_t s1, uint64_t s2,
-                      uint32_t b0, uint32_t b1, uint32_t b2, bool swizzle128) {
+                      uint32_t b0, uint32_t b1, uint32_t b2, int swizzle_bytes) {
     std::call_once(g_encode_once, load_encode);
     if (!g_encode) return CUDA_ERROR_NOT_FOUND;
     cuuint64_t dims[3] = {d0, d1, d2};
@@ -48,7 +48,9 @@ CUresult make_tmap_3d(CUtensorMap* map, const void* base, CUtensorMapDataType dt
     cuuint32_t estr[3] = {1, 1, 1};
     return g_encode(map, dtype, 3, const_cast<void*>(base), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                    swizzle_bytes == 128  ? CU_TENSOR_MAP_SWIZZLE_128B
+                    : swizzle_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                          : CU_TENSOR_MAP_SWIZZLE_NONE,
                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
 }
 
