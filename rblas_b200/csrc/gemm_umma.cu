@@ -371,12 +371,12 @@ __global__ void __launch_bounds__(UCfg<MODE>::THREADS, 1)
 // ------------------------------------------------------------------------------
 // The BF16-split GEMM on CTA pairs: 256 x 256 tiles, M = 256 N = 256 MMAs.
 //
-// An M = 128 N = 128 MMA reads both operands from shared memory at the full
-// 128 bytes per clock, and TMA's writes of the next stage come on top, so
-// umma_gemm_kernel's tensor pipe waits for shared memory. A pair's MMA reads
-// 128 rows of A and 128 of B per SM for twice the products: 64 bytes per
-// clock, and half the TMA bytes per product. Each CTA loads its 128 rows of
-// A and its 128 of B; the even CTA's warp 1 issues for both.
+// 128 x 128 tiles take 83 bytes (3xBF16; BF16X6 62) of operands from L2 per SM
+// and clock of MMA, twice what TMA was seen to land on all SMs at once (~40),
+// so their tensor pipe waits. A pair's tile needs half of that: each CTA loads
+// its 128 rows of A and its 128 of B for 256 x 256 outputs; the even CTA's
+// warp 1 issues for both. (Shared memory itself is no limit: M = 128 N = 128
+// MMAs kept their 64 clocks beside 112 bytes per clock of other writes.)
 // 3xBF16 alternates two accumulators of 256 columns. BF16X6 keeps hi*hi apart
 // (as umma_body does), which fills TMEM with one accumulator of each kind. A
 // drain takes ~1200 clocks from the last MMA to the even CTA's knowing (the
@@ -545,7 +545,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
                         break;
                     }
                 }
-                mbar_arrive_rank(&bar->peer_full[it % PS], 0);
+                mbar_arrive_rank_relaxed(&bar->peer_full[it % PS], 0);
             }
     } else if (warp == 1 && lane == 0) {
         // ------------------------- even CTA: MMA issuer -------------------------
@@ -1091,6 +1091,8 @@ struct OzCfg {
 // kernels.
 constexpr int kOzRaster = 16;
 
+constexpr int kOzGroups = 3;  // groups of four diagonals, slices <= 12
+
 struct OzParams {
     int m, n, k;
     int tiles_m, tiles_n, num_tiles;
@@ -1117,6 +1119,10 @@ struct OzParams {
     double* ws;
     int tail_tiles;
     int un;  // tile width (256 or 128): the split tail's plane size and the reduce kernel's tiling
+    // Pair kernel's tail (see ozaki_pair_kernel): K parts of each group of
+    // four diagonals, the groups in order of an item's cost (dearest first),
+    // and the first workspace plane of each within a tile's `planes`.
+    int parts[kOzGroups], order[kOzGroups], plane0[kOzGroups], planes;
 };
 
 // 2^x for x in [-1022, 1023]
@@ -1557,6 +1563,503 @@ __global__ void __launch_bounds__(kOzThreads, 1)
     ozaki_grouped_kernel(const OzGroupEntry* __restrict__ tab, const int* __restrict__ starts, int nprob,
                          uint32_t* err) {
     ozaki_body<UN>(OzGroupSrc{tab, starts, nprob, err});
+}
+
+// ------------------------------------------------------------------------------
+// Ozaki GEMM on CTA pairs: 256 x 128 tiles, four diagonals at a time.
+//
+// ozaki_body's tensor cores wait while a unit of two diagonals drains through
+// C: 512 KiB per SM and unit through L2, on all SMs at once (11 us, 19 % of a
+// CTA's time at K = 2048), and its operands take 52 bytes per SM and clock of
+// MMA from L2. Here a unit is four diagonals {4g .. 4g+3}, whose accumulators
+// (4 x 128 columns) fill TMEM, so a tile has half as many units; each
+// epilogue thread keeps its 64 outputs of the tile in FP64 registers from the
+// first unit (beta * C0, loaded while the tensor cores run) to the last, so C
+// is read and written once and a drain touches TMEM only. Stage st of a K
+// tile brings A_{top-st} and B_st; A_{top-st} is multiplied by the B tiles of
+// this stage and of up to three before it (diagonal top - lag), 31 operand
+// bytes per SM and clock.
+// The epilogue folds the pairs of diagonals exactly as ozaki_body does, in the
+// same order, so the results are its bits: term = (S_d0 * 256 + S_d1) *
+// 2^(e + f - w), acc = fma(alpha, term, acc). Where row and column exponents
+// and alpha are moderate, alpha * 2^(e + f - w) is exact and one fma(sv,
+// alpha * 2^(..), acc) has the same rounding.
+// Tail: the tiles of the partial last wave run as items of one group over a
+// part of K each, which write the exact sums S_d0 * 256 + S_d1 to workspace
+// planes; ozaki_pair_reduce_kernel adds the parts (exactly) and folds.
+// Warps per CTA: 0 TMA producer, 1 TMEM owner and MMA issuer (even CTA; odd:
+// passes on that a stage landed), 2..9 epilogue (two per TMEM lane quarter,
+// 64 columns each).
+// ------------------------------------------------------------------------------
+constexpr int kPzN = 128;
+constexpr int kPzEpiWarps = 8;
+constexpr int kPzThreads = 64 + 32 * kPzEpiWarps;
+// Ring depths: a B tile is used for up to three stages after its own, so with
+// three more B slots than A slots both rings' next slots are free once the
+// stage kPzAS back is done, and one barrier per stage serves both.
+constexpr int kPzAS = 8, kPzBS = kPzAS + 3;
+constexpr int kPzBTile = 64 * kRowBytes;           // this CTA's half of a B tile
+constexpr int kPzCols = kPzN / 2;                  // columns per epilogue warp
+constexpr int kPzTab = kPzCols * (8 + 4);          // per epilogue warp: 2^fc and fc
+constexpr int kPzTileElems = 256 * kPzN;
+constexpr int kPzSmem = kPzAS * kATile + kPzBS * kPzBTile + 512 + kPzEpiWarps * kPzTab + 1024;
+static_assert(kPzSmem <= 232448, "the pair kernel's rings must fit one CTA's shared memory");
+
+struct PzBar {
+    uint64_t full[kPzAS], done[kPzAS];  // stage landed; its MMAs complete
+    uint64_t peer_full[kPzAS];          // even CTA: the odd CTA's stage has landed
+    uint64_t acc_full, acc_empty, drain;
+    uint32_t tmem_base;
+};
+static_assert(sizeof(PzBar) <= 512, "shared memory reserved for the pair kernel's barriers");
+
+// Diagonals 4g .. 4g + nd - 1 of group g.
+__host__ __device__ __forceinline__ int pz_nd(int slices, int g) { return slices - 4 * g < 4 ? slices - 4 * g : 4; }
+
+// A work item: units [u_lo, u_hi) of tile t over K tiles kt0.. of each chunk
+// (unit u: group groups-1 - u % groups of chunk u / groups), or, in the tail
+// (tt >= 0), one group over K tiles [kt0, kt1) into workspace planes from
+// `plane` on.
+struct PzWork {
+    const OzParams* p;
+    const CUtensorMap* ta;
+    const CUtensorMap* tb;
+    int t, u_lo, u_hi, tt, kt0, kt1, plane;
+};
+
+__host__ __device__ __forceinline__ int pz_items(const OzParams& p) {
+    const int groups = (p.slices + 3) / 4;
+    int per_tile = 0;
+    for (int g = 0; g < kOzGroups; ++g) per_tile += g < groups ? p.parts[g] : 0;
+    return p.num_tiles - p.tail_tiles + p.tail_tiles * per_tile;
+}
+
+// Tail items are ranked by cost and dealt to the G pairs in a snake, as in oz_item.
+__host__ __device__ __forceinline__ void pz_item(const OzParams& p, int G, int item, PzWork& w) {
+    const int groups = (p.slices + 3) / 4, fused = p.num_tiles - p.tail_tiles;
+    w.tt = -1;
+    w.plane = 0;
+    w.kt0 = 0;
+    w.kt1 = p.num_kt;
+    if (item < fused) {
+        w.t = item;
+        w.u_lo = 0;
+        w.u_hi = p.kchunks * groups;
+        return;
+    }
+    const int j = item - fused, total = pz_items(p) - fused;
+    const int pass = j / G, q = j - pass * G;
+    const int len = (total - pass * G < G) ? total - pass * G : G;
+    int rank = (pass & 1) ? pass * G + (len - 1 - q) : j;
+    for (int i = 0; i < groups; ++i) {
+        const int g = p.order[i], n = p.tail_tiles * p.parts[g];
+        if (rank < n) {
+            const int part = rank / p.tail_tiles;
+            w.tt = rank - part * p.tail_tiles;
+            w.t = fused + w.tt;
+            w.u_lo = groups - 1 - g;
+            w.u_hi = w.u_lo + 1;
+            w.kt0 = static_cast<int>(static_cast<long long>(p.num_kt) * part / p.parts[g]);
+            w.kt1 = static_cast<int>(static_cast<long long>(p.num_kt) * (part + 1) / p.parts[g]);
+            w.plane = p.plane0[g] + part * ((pz_nd(p.slices, g) + 1) / 2);
+            return;
+        }
+        rank -= n;
+    }
+}
+
+struct PzSingleSrc {
+    const OzParams* p;
+    const CUtensorMap* ta;
+    const CUtensorMap* tb;
+    __device__ __forceinline__ uint32_t* err() const { return p->err; }
+    __device__ __forceinline__ int items() const { return pz_items(*p); }
+    __device__ __forceinline__ PzWork get(int item) const {
+        PzWork w{p, ta, tb, 0, 0, 0, -1, 0, 0, 0};
+        pz_item(*p, gridDim.x >> 1, item, w);
+        return w;
+    }
+};
+
+// Whole tiles of many problems, as OzGroupSrc.
+struct PzGroupSrc {
+    OzGroupSrc s;
+    __device__ __forceinline__ uint32_t* err() const { return s.err(); }
+    __device__ __forceinline__ int items() const { return s.items(); }
+    __device__ __forceinline__ PzWork get(int item) const {
+        const OzWork o = s.get(item);
+        return PzWork{o.p, o.ta, o.tb, o.t, 0, o.p->kchunks * ((o.p->slices + 3) / 4), -1, 0, o.p->num_kt, 0};
+    }
+};
+
+// K tiles of unit u of an item.
+__device__ __forceinline__ void pz_kt(const PzWork& w, int u, int groups, int& kt0, int& kt1) {
+    if (w.tt >= 0) {
+        kt0 = w.kt0;
+        kt1 = w.kt1;
+    } else {
+        kt0 = (u / groups) * w.p->kt_per_chunk;
+        kt1 = min(w.p->num_kt, kt0 + w.p->kt_per_chunk);
+    }
+}
+
+// sv * 2^(er + fc - wexp) for any exponents (0 for a zero row or column).
+__device__ __noinline__ double pz_term(double sv, int er, int fc, int wexp) {
+    return (er != kExpSentinel && fc != kExpSentinel) ? scale_pow2(sv, er + fc - wexp) : 0.0;
+}
+
+template <class Src>
+__device__ __forceinline__ void ozaki_pair_body(const Src& src) {
+    constexpr int AS = kPzAS, BS = kPzBS;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    uint8_t* bring = smem + AS * kATile;
+    PzBar* bar = reinterpret_cast<PzBar*>(bring + BS * kPzBTile);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_rank();
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < AS; ++i) {
+            mbar_init(&bar->full[i], 1);
+            mbar_init(&bar->done[i], 1);
+            mbar_init(&bar->peer_full[i], 1);
+        }
+        mbar_init(&bar->acc_full, 1);
+        mbar_init(&bar->acc_empty, 2 * kPzEpiWarps);
+        mbar_init(&bar->drain, 1);
+        fence_barrier_init();
+    }
+    if (warp == 1) tmem_alloc_pair(&bar->tmem_base, 512);
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();  // the other CTA's barriers are initialised too
+    tc_fence_after();
+    const uint32_t tmem_base = bar->tmem_base;
+    const int items = src.items(), first = blockIdx.x >> 1, step = gridDim.x >> 1;
+    uint32_t* const err = src.err();
+    bool ok = true;
+
+    if (warp == 0 && lane == 0) {
+        // ------------------------------ TMA producer ------------------------------
+        uint32_t it = 0;
+        const CUtensorMap* fetched = nullptr;
+        for (int item = first; ok && item < items; item += step) {
+            const PzWork w = src.get(item);
+            const OzParams& p = *w.p;
+            if (w.ta != fetched) {
+                prefetch_tmap(w.ta);
+                prefetch_tmap(w.tb);
+                fetched = w.ta;
+            }
+            const int groups = (p.slices + 3) / 4;
+            int tm, tn;
+            raster_tile<kOzRaster / 2>(w.t, p.tiles_m, p.tiles_n, tm, tn);
+            const int m0 = tm * 256 + rank * 128, n0 = tn * kPzN + rank * 64;
+            for (int u = w.u_lo; ok && u < w.u_hi; ++u) {
+                const int g = groups - 1 - u % groups, top = 4 * g + pz_nd(p.slices, g) - 1;
+                int kt0, kt1;
+                pz_kt(w, u, groups, kt0, kt1);
+                for (int kt = kt0; ok && kt < kt1; ++kt)
+                    for (int st = 0; st <= top; ++st, ++it) {
+                        const uint32_t as = it % AS, bs = it % BS;
+                        if (it >= AS && !mbar_wait_cluster(&bar->done[as], ((it / AS) - 1) & 1, err, 0x311)) {
+                            ok = false;
+                            break;
+                        }
+                        mbar_arrive_expect_tx(&bar->full[as], kATile + kPzBTile);
+                        tma_load_3d(smem + as * kATile, w.ta, &bar->full[as], kt * 128, m0, top - st);
+                        tma_load_3d(bring + bs * kPzBTile, w.tb, &bar->full[as], kt * 128, n0, st);
+                    }
+            }
+        }
+        if (!ok) {  // this CTA's copies land before it exits
+            for (uint32_t j = it > (uint32_t)AS ? it - AS : 0; j < it; ++j)
+                mbar_wait_drain(&bar->full[j % AS], (j / AS) & 1);
+        }
+    } else if (warp == 1) {
+        // ---------- odd CTA: landed stages, told to the even one; even CTA: MMA issuer ----------
+        // (the whole warp runs the loop, one lane issues: see elect_one)
+        const bool lead = elect_one();
+        const uint64_t d0 = sw128_kmajor_desc(smem_u32(smem));  // (see umma_pair_kernel on descriptors)
+        const uint32_t a_lo = static_cast<uint32_t>(d0), b_lo = a_lo + AS * kATile / 16;
+        const uint64_t d_hi = d0 & 0xffffffff00000000ull;
+        constexpr uint32_t idesc = umma_idesc(2, 1, 256, kPzN);  // s32 <- s8 x s8
+        uint32_t uc = 0, as = 0, ph = 0, bs = 0;  // ring slots, A's phase
+        // one stage's MMAs: A (descriptor low word a) with the B tiles of NL
+        // lags (b), lag l into accumulator nd-1-l; `fresh`: the last lag's
+        // accumulator starts. Straight-line per NL: an MMA takes 64 clocks,
+        // and a test around each of them took the issuing thread longer.
+        auto stage = [&](auto nl, uint32_t a, const uint32_t (&b)[4], uint32_t d, bool fresh) {
+            constexpr int NL = decltype(nl)::value;
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+                for (int l = 0; l < NL; ++l)
+                    umma_i8_pair(d - l * kPzN, d_hi | (a + 2 * kk), d_hi | (b[l] + 2 * kk), idesc,
+                                 (kk == 0 && l == NL - 1) ? (fresh ? 0u : 1u) : 1u);
+        };
+        for (int item = first; ok && item < items; item += step) {
+            const PzWork w = src.get(item);
+            const int slices = w.p->slices, groups = (slices + 3) / 4;
+            for (int u = w.u_lo; ok && u < w.u_hi; ++u, ++uc) {
+                const int g = groups - 1 - u % groups, nd = pz_nd(slices, g), top = 4 * g + nd - 1;
+                int kt0, kt1;
+                pz_kt(w, u, groups, kt0, kt1);
+                const uint32_t d = tmem_base + (nd - 1) * kPzN;
+                if (rank == 0) {
+                    if (uc >= 1 &&
+                        !__all_sync(0xffffffffu, mbar_wait_cluster(&bar->acc_empty, (uc - 1) & 1, err, 0x313))) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                }
+                for (int kt = kt0; ok && kt < kt1; ++kt)
+                    for (int st = 0; st <= top; ++st) {
+                        if (!__all_sync(0xffffffffu, mbar_wait_cluster(&bar->full[as], ph, err, 0x314))) {
+                            ok = false;
+                            break;
+                        }
+                        if (rank == 1) {
+                            if (lead) mbar_arrive_rank_relaxed(&bar->peer_full[as], 0);
+                        } else {
+                            if (!__all_sync(0xffffffffu, mbar_wait_cluster(&bar->peer_full[as], ph, err, 0x316))) {
+                                ok = false;
+                                break;
+                            }
+                            tc_fence_after();
+                            const uint32_t a = a_lo + as * (kATile / 16);
+                            uint32_t b[4];
+#pragma unroll
+                            for (int l = 0; l < 4; ++l)
+                                b[l] = b_lo + (bs >= (uint32_t)l ? bs - l : bs + BS - l) * (kPzBTile / 16);
+                            const int nl = min(st + 1, nd);
+                            const bool fresh = kt == kt0 && st == nl - 1;
+                            if (lead) {
+                                if (nl == 4)      stage(std::integral_constant<int, 4>{}, a, b, d, fresh);
+                                else if (nl == 3) stage(std::integral_constant<int, 3>{}, a, b, d, fresh);
+                                else if (nl == 2) stage(std::integral_constant<int, 2>{}, a, b, d, fresh);
+                                else              stage(std::integral_constant<int, 1>{}, a, b, d, fresh);
+                                tc_commit_pair(&bar->done[as]);
+                            }
+                        }
+                        if (++as == AS) {
+                            as = 0;
+                            ph ^= 1;
+                        }
+                        if (++bs == BS) bs = 0;
+                    }
+                if (ok && rank == 0 && lead) tc_commit_pair(&bar->acc_full);
+            }
+        }
+        if (rank == 0 && lead) {  // nothing of ours is in flight before TMEM is released
+            tc_commit_pair(&bar->drain);
+            mbar_wait_drain(&bar->drain, 0);
+        }
+    } else if (warp >= 2) {
+        // ------------------------------ epilogue ------------------------------
+        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        const int row_in_pair = static_cast<int>(rank) * 128 + quarter * 32 + lane;
+        uint8_t* tab = reinterpret_cast<uint8_t*>(bar) + 512 + (warp - 2) * kPzTab;
+        double* col_scale = reinterpret_cast<double*>(tab);
+        int* col_e = reinterpret_cast<int*>(tab + kPzCols * sizeof(double));
+        const uint32_t tbase = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * kPzCols;
+        uint32_t uc = 0;
+        for (int item = first; ok && item < items; item += step) {
+            const PzWork w = src.get(item);
+            const OzParams& p = *w.p;
+            const int groups = (p.slices + 3) / 4;
+            int tm, tn;
+            raster_tile<kOzRaster / 2>(w.t, p.tiles_m, p.tiles_n, tm, tn);
+            const int r = tm * 256 + row_in_pair, cb = tn * kPzN + half * kPzCols;
+            const bool row_ok = r < p.m, tail = w.tt >= 0;
+            const int er = row_ok ? p.row_exp[r] : kExpSentinel;
+            // moderate exponents: alpha * 2^(er - w) * 2^fc and every product
+            // with it stay in the normal range
+            const int ea = static_cast<int>((static_cast<unsigned long long>(__double_as_longlong(p.alpha)) >> 52) & 0x7FF);
+            const bool alpha_fast = ea >= 1023 - 200 && ea <= 1023 + 200;
+            const bool row_fast = er >= -200 && er <= 200 && alpha_fast;
+            __syncwarp();  // the previous item's reads of the table are done
+            bool cols_fast = true;
+#pragma unroll
+            for (int h = 0; h < kPzCols / 32; ++h) {
+                const int j = lane + 32 * h, col = cb + j;
+                const int fc = col < p.n ? __ldg(p.col_exp + col) : kExpSentinel;
+                const bool mod = fc >= -200 && fc <= 200;
+                col_e[j] = fc;
+                col_scale[j] = mod ? pow2_normal(fc) : 0.0;
+                cols_fast = cols_fast && (mod || col >= p.n);  // a column outside C: never stored
+            }
+            __syncwarp();
+            // the whole warp takes the one-fma form, or none of it
+            const bool fast = __all_sync(0xffffffffu, cols_fast && (row_fast || !row_ok));
+            double acc[kPzCols];
+            if (!tail) {
+                const double* c0 = p.cin + (row_ok ? r : 0) + static_cast<size_t>(cb) * p.ldc;
+#pragma unroll
+                for (int j = 0; j < kPzCols; ++j)
+                    acc[j] = (row_ok && p.beta_mode != 0 && cb + j < p.n) ? c0[static_cast<size_t>(j) * p.ldc] : 0.0;
+                if (p.beta_mode == 2) {
+#pragma unroll
+                    for (int j = 0; j < kPzCols; ++j) acc[j] = p.beta * acc[j];
+                }
+            }
+            bool first_pair = true;
+            for (int u = w.u_lo; ok && u < w.u_hi; ++u, ++uc) {
+                const int g = groups - 1 - u % groups, nd = pz_nd(p.slices, g), npair = (nd + 1) / 2;
+                const bool got = mbar_wait_cluster(&bar->acc_full, uc & 1, err, 0x317);
+                if (!__all_sync(0xffffffffu, got)) {  // the whole warp goes on, or the whole warp stops
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+#pragma unroll 1
+                for (int pi = 0; pi < npair; ++pi) {
+                    const int j0 = 2 * (npair - 1 - pi);  // diagonals 4g + j0 and, in a pair, 4g + j0 + 1
+                    const bool pair = j0 + 1 < nd;
+                    const int wexp = 14 + 8 * (4 * g + j0 + (pair ? 1 : 0)) - 2;
+                    const int mul = pair ? 256 : 0;
+                    const double ars = fast && row_ok ? p.alpha * pow2_normal(er - wexp) : 0.0;
+                    double* wplane = tail ? p.ws + (static_cast<size_t>(w.tt) * p.planes + w.plane + pi) * kPzTileElems +
+                                                row_in_pair + static_cast<size_t>(half * kPzCols) * 256
+                                          : nullptr;
+                    const bool live = row_ok && (first_pair || er != kExpSentinel);
+                    // chunks of 4 columns, each requested before the one ahead
+                    // of it is used (4-column ones: 64 outputs in FP64 leave
+                    // registers for two chunks of 2 x 4)
+                    constexpr int CH = 4, NCH = kPzCols / CH;
+                    uint32_t v0[2][CH], v1[2][CH];
+                    auto request = [&](int ch) {
+                        tmem_ld4(tbase + j0 * kPzN + ch * CH, v0[ch & 1]);
+                        tmem_ld4(tbase + (pair ? j0 + 1 : j0) * kPzN + ch * CH, v1[ch & 1]);
+                    };
+                    // S_d0 * 256 + S_d1 (below 2^40) as a double: exact, by the
+                    // bits of 1.5 * 2^52 + T (alone, S_d0: mul 0 + 1 * v1)
+                    auto sum = [&](int ch, int jj) {
+                        const long long T = static_cast<long long>(static_cast<int32_t>(v0[ch & 1][jj])) * mul +
+                                            static_cast<int32_t>(v1[ch & 1][jj]);
+                        return __longlong_as_double(T + 0x4338000000000000LL) - 6755399441055744.0;
+                    };
+                    // one loop per case, so that a chunk's chains interleave
+                    request(0);
+                    if (tail) {
+#pragma unroll 2
+                        for (int ch = 0; ch < NCH; ++ch) {
+                            tmem_ld_wait();
+                            if (ch + 1 < NCH) request(ch + 1);
+#pragma unroll
+                            for (int jj = 0; jj < CH; ++jj)
+                                wplane[static_cast<size_t>(ch * CH + jj) * 256] = sum(ch, jj);
+                        }
+                    } else if (fast) {
+#pragma unroll
+                        for (int ch = 0; ch < NCH; ++ch) {
+                            tmem_ld_wait();
+                            if (ch + 1 < NCH) request(ch + 1);
+#pragma unroll
+                            for (int jj = 0; jj < CH; ++jj)
+                                acc[ch * CH + jj] = fma(sum(ch, jj), ars * col_scale[ch * CH + jj], acc[ch * CH + jj]);
+                        }
+                    } else {
+#pragma unroll
+                        for (int ch = 0; ch < NCH; ++ch) {
+                            tmem_ld_wait();
+                            if (ch + 1 < NCH) request(ch + 1);
+                            if (live) {
+#pragma unroll
+                                for (int jj = 0; jj < CH; ++jj)
+                                    acc[ch * CH + jj] = fma(p.alpha, pz_term(sum(ch, jj), er, col_e[ch * CH + jj], wexp),
+                                                            acc[ch * CH + jj]);
+                            }
+                        }
+                    }
+                    first_pair = false;
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_rank_relaxed(&bar->acc_empty, 0);
+            }
+            if (ok && row_ok && !tail) {
+                double* c = p.c + r + static_cast<size_t>(cb) * p.ldc;
+#pragma unroll
+                for (int j = 0; j < kPzCols; ++j)
+                    if (cb + j < p.n) c[static_cast<size_t>(j) * p.ldc] = acc[j];
+            }
+        }
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();  // no CTA leaves while the other may still reach its memory
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc_pair(tmem_base, 512);
+    }
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPzThreads, 1)
+    ozaki_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                      const __grid_constant__ OzParams p) {
+    ozaki_pair_body(PzSingleSrc{&p, &tmA, &tmB});
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPzThreads, 1)
+    ozaki_pair_grouped_kernel(const OzGroupEntry* __restrict__ tab, const int* __restrict__ starts, int nprob,
+                              uint32_t* err) {
+    ozaki_pair_body(PzGroupSrc{OzGroupSrc{tab, starts, nprob, err}});
+}
+
+// The pair kernel's tail: per element, beta * C0, then for each pair of
+// diagonals from the highest down the exact sum of its K parts, scaled and
+// folded as in the epilogue. Two rows per thread (planes are 256 x 128, rows
+// contiguous, so every plane read is 16 bytes).
+__global__ void __launch_bounds__(256) ozaki_pair_reduce_kernel(const OzParams p) {
+    const int fused = p.num_tiles - p.tail_tiles, groups = (p.slices + 3) / 4;
+    const size_t total = static_cast<size_t>(p.tail_tiles) * (kPzTileElems / 2);
+    for (size_t idx = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; idx < total;
+         idx += static_cast<size_t>(gridDim.x) * blockDim.x) {
+        const int tt = static_cast<int>(idx / (kPzTileElems / 2));
+        const int local = 2 * static_cast<int>(idx - static_cast<size_t>(tt) * (kPzTileElems / 2));
+        int tm, tn;
+        raster_tile<kOzRaster / 2>(fused + tt, p.tiles_m, p.tiles_n, tm, tn);
+        const int r = tm * 256 + local % 256, col = tn * kPzN + local / 256;
+        if (r >= p.m || col >= p.n) continue;
+        const bool two = r + 1 < p.m;
+        double* cp = p.c + r + static_cast<size_t>(col) * p.ldc;
+        const double* c0 = p.cin + r + static_cast<size_t>(col) * p.ldc;
+        double acc[2] = {p.beta_mode ? c0[0] : 0.0, p.beta_mode && two ? c0[1] : 0.0};
+        if (p.beta_mode == 2) {
+            acc[0] = p.beta * acc[0];
+            acc[1] = p.beta * acc[1];
+        }
+        const int er[2] = {p.row_exp[r], two ? p.row_exp[r + 1] : kExpSentinel};
+        const int fc = p.col_exp[col];
+        const double* w = p.ws + static_cast<size_t>(tt) * p.planes * kPzTileElems + local;
+        bool first_pair = true;
+        for (int g = groups - 1; g >= 0; --g) {
+            const int nd = pz_nd(p.slices, g), npair = (nd + 1) / 2;
+            for (int pi = 0; pi < npair; ++pi) {
+                const int j0 = 2 * (npair - 1 - pi);
+                const int wexp = 14 + 8 * (4 * g + j0 + (j0 + 1 < nd ? 1 : 0)) - 2;
+                double sv[2] = {0.0, 0.0};
+                for (int part = 0; part < p.parts[g]; ++part) {
+                    const double2 v = *reinterpret_cast<const double2*>(
+                        w + static_cast<size_t>(p.plane0[g] + part * npair + pi) * kPzTileElems);
+                    sv[0] += v.x;
+                    sv[1] += v.y;
+                }
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    if (first_pair || er[h] != kExpSentinel)
+                        acc[h] = fma(p.alpha,
+                                     (er[h] != kExpSentinel && fc != kExpSentinel) ? scale_pow2(sv[h], er[h] + fc - wexp)
+                                                                                   : 0.0,
+                                     acc[h]);
+                first_pair = false;
+            }
+        }
+        cp[0] = acc[0];
+        if (two) cp[1] = acc[1];
+    }
 }
 
 // Split tail: C of the tail tiles = the fused epilogue's sequence over the
@@ -2462,6 +2965,11 @@ cudaError_t ozaki_kernel_attributes() {
         if (result == cudaSuccess)
             result = cudaFuncSetAttribute(ozaki_grouped_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           OzCfg<128>::SMEM);
+        if (result == cudaSuccess)
+            result = cudaFuncSetAttribute(ozaki_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPzSmem);
+        if (result == cudaSuccess)
+            result = cudaFuncSetAttribute(ozaki_pair_grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          kPzSmem);
     });
     return result;
 }
@@ -2490,6 +2998,93 @@ int ozaki_tail_tiles(int num_tiles, int slices, int kchunks, int k, int sms, int
     return (fits && product_s * max_load + reduce_s < 0.9 * whole_tile_s) ? tail : 0;
 }
 
+// The pair kernel's tail (OzParams::tail_tiles, parts, order, plane0, planes):
+// the tiles of the partial last wave (all tiles when there are fewer than
+// pairs), cut into groups of diagonals and K parts, where that finishes
+// before a whole further wave would. Costs in products (36 per K tile of a
+// whole tile at 8 slices) over the K tiles; a product of a 256 x 128 tile and
+// one K tile takes 256 clocks, an item 3 us beside its products, the planes'
+// traffic and the second launch 10 us and their bytes at 5 TB/s. Measured
+// against whole tiles (us; parts of the dearer group): 300 x 300 x 4000 -121
+// (4), 512^3 -12 (4), 3000 x 5000 x 2048 -34 (3), 4096 x 2048 x 4096 -33 (3);
+// 1024^3 +10 and 777 x 999 x 1234 +6 (1), 1500^3 +42 (1): left whole.
+void ozaki_pair_tail(OzParams& p, int pairs) {
+    const int groups = (p.slices + 3) / 4;
+    p.tail_tiles = 0;
+    p.planes = 0;
+    int cost[kOzGroups] = {};
+    for (int g = 0; g < kOzGroups; ++g) {
+        p.parts[g] = 0;
+        p.order[g] = 0;
+        p.plane0[g] = 0;
+        if (g >= groups) continue;
+        p.parts[g] = 1;
+        for (int d = 4 * g; d < 4 * g + pz_nd(p.slices, g); ++d) cost[g] += d + 1;
+    }
+    const int tail = p.num_tiles % pairs;
+    if (p.kchunks != 1 || tail == 0) return;
+    const int all = p.slices * (p.slices + 1) / 2;
+    const double prod_us = 256 / 1.7e3;                   // one product, one K tile
+    double best = all * p.num_kt * prod_us + 4.0;         // a whole tile's wave
+    OzParams cand = p;
+    cand.tail_tiles = tail;
+    // parts of the dearest group; the others in proportion to their cost
+    for (int pd = 1; pd <= 16 && pd <= p.num_kt; pd = pd < 3 ? pd + 1 : pd + pd / 2) {
+        int dear = 0;
+        for (int g = 1; g < groups; ++g)
+            if (cost[g] > cost[dear]) dear = g;
+        int planes = 0, order[kOzGroups];
+        for (int g = 0; g < groups; ++g) {
+            cand.parts[g] = std::max(1, std::min(p.num_kt, (cost[g] * pd + cost[dear] / 2) / cost[dear]));
+            cand.plane0[g] = planes;
+            planes += cand.parts[g] * ((pz_nd(p.slices, g) + 1) / 2);
+            order[g] = g;
+        }
+        std::sort(order, order + groups, [&](int x, int y) {
+            return static_cast<double>(cost[x]) / cand.parts[x] > static_cast<double>(cost[y]) / cand.parts[y];
+        });
+        for (int g = 0; g < groups; ++g) cand.order[g] = order[g];
+        cand.planes = planes;
+        const size_t bytes = static_cast<size_t>(tail) * planes * kPzTileElems * sizeof(double);
+        if (bytes > (size_t(512) << 20)) break;
+        // the snake's fullest pair: the items' costs in rank order, one per pass
+        const int total = pz_items(cand) - (p.num_tiles - tail);
+        double load = 0;
+        for (int q = 0; q < std::min(total, pairs); ++q) {
+            double l = 0;
+            for (int j = q; j < total; j += pairs) {
+                PzWork w{};
+                pz_item(cand, pairs, p.num_tiles - tail + j, w);
+                const int g = groups - 1 - w.u_lo;
+                l += cost[g] * (w.kt1 - w.kt0) * prod_us + 3.0;
+            }
+            load = std::max(load, l);
+        }
+        const double t = load + 10.0 + (bytes + 2.0 * tail * kPzTileElems * sizeof(double)) / 5e6;
+        if (t < best) {
+            best = t;
+            p.tail_tiles = tail;
+            p.planes = planes;
+            for (int g = 0; g < kOzGroups; ++g) {
+                p.parts[g] = cand.parts[g];
+                p.order[g] = cand.order[g];
+                p.plane0[g] = cand.plane0[g];
+            }
+        }
+    }
+}
+
+// Whether an m x n product takes the pair kernel: unless one tile row of 128 is
+// all it has, or a pair's 256 rows pad so much more than 128 that the wide
+// tiles' larger cost (per 128 x 256 C of one SM 1 against 0.85 for a pair's
+// 256 x 128) is the smaller one. A width that the autotuner forces while it
+// times the other kernels wins.
+bool ozaki_pair_tiles(int m, int n) {
+    if (m <= 128 || ozaki_width_forced()) return false;
+    const double wide = static_cast<double>((m + 127) / 128) * ((n + 255) / 256);
+    return n <= 128 || 0.85 * ((m + 255) / 256) * ((n + 127) / 128) <= wide;
+}
+
 cudaError_t launch_ozaki_gemm(bool ta, bool tb, int m, int n, int k, double alpha, const double* A,
                               size_t lda, const double* B, size_t ldb, double beta, double* C,
                               size_t ldc, int slices, cudaStream_t st, CUresult* cu_err) {
@@ -2502,15 +3097,24 @@ cudaError_t launch_ozaki_gemm(bool ta, bool tb, int m, int n, int k, double alph
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int un = ozaki_tile_n(m, n, k);
-    const int num_tiles = ((m + kUM - 1) / kUM) * ((n + un - 1) / un);
+    const bool pair = sms >= 2 && ozaki_pair_tiles(m, n);
+    const int un = pair ? kPzN : ozaki_tile_n(m, n, k), um = pair ? 256 : kUM;
     const int upc = (slices + 1) / 2;
-    const long long kt_chunk = 2147483647LL / (static_cast<long long>(slices) * 128 * 128) / 128;
-    const long long ktc = std::max(kt_chunk, 1LL);
-    const int kchunks = static_cast<int>(((k + 127) / 128 + ktc - 1) / ktc);
-    const int tail_tiles = ozaki_tail_tiles(num_tiles, slices, kchunks, k, sms, un);
+    OzParams p{};
+    p.m = m; p.n = n; p.k = k;
+    p.un = un;
+    p.tiles_m = (m + um - 1) / um;
+    p.tiles_n = (n + un - 1) / un;
+    p.num_tiles = p.tiles_m * p.tiles_n;
+    p.num_kt = static_cast<int>((k + 127) / 128);
+    p.slices = slices;
+    // exact INT32: a diagonal has <= slices products of |d_t d_u| <= 128*128 per K element
+    p.kt_per_chunk = static_cast<int>(std::max(2147483647LL / (static_cast<long long>(slices) * 128 * 128) / 128, 1LL));
+    p.kchunks = (p.num_kt + p.kt_per_chunk - 1) / p.kt_per_chunk;
+    if (pair) ozaki_pair_tail(p, sms / 2);
+    else      p.tail_tiles = ozaki_tail_tiles(p.num_tiles, slices, p.kchunks, k, sms, un);
     const size_t b_bytes = round_up(slices * pb, 256);
-    const size_t w_bytes = static_cast<size_t>(tail_tiles) * upc * kUM * un * sizeof(double);
+    const size_t w_bytes = static_cast<size_t>(p.tail_tiles) * (pair ? p.planes : upc) * um * un * sizeof(double);
     cudaError_t e = scratch_alloc(&buf, exps + a_bytes + b_bytes + w_bytes, st);
     if (e != cudaSuccess) return e;
     int* ea = static_cast<int*>(buf);
@@ -2532,50 +3136,41 @@ cudaError_t launch_ozaki_gemm(bool ta, bool tb, int m, int n, int k, double alph
     count_launch(5);
     CUtensorMap tma, tmb;
     CUresult r = make_tmap_planes(&tma, sla, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, k, m, slices, kp, kUM);
-    if (r == CUDA_SUCCESS) r = make_tmap_planes(&tmb, slb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, k, n, slices, kp, un);
+    if (r == CUDA_SUCCESS)
+        r = make_tmap_planes(&tmb, slb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, k, n, slices, kp, pair ? 64 : un);
     if (r != CUDA_SUCCESS) {
         if (cu_err) *cu_err = r;
         cudaFreeAsync(buf, st);
         return cudaErrorInvalidValue;
     }
-    OzParams p{};
-    p.m = m; p.n = n; p.k = k;
-    p.un = un;
-    p.tiles_m = (m + kUM - 1) / kUM;
-    p.tiles_n = (n + un - 1) / un;
-    p.num_tiles = p.tiles_m * p.tiles_n;
-    p.num_kt = static_cast<int>((k + 127) / 128);
-    p.slices = slices;
-    // exact INT32: a diagonal has <= slices products of |d_t d_u| <= 128*128 per K element
-    const long long max_k = 2147483647LL / (static_cast<long long>(slices) * 128 * 128);
-    p.kt_per_chunk = static_cast<int>(max_k / 128);
-    if (p.kt_per_chunk < 1) p.kt_per_chunk = 1;
-    p.kchunks = (p.num_kt + p.kt_per_chunk - 1) / p.kt_per_chunk;
     p.beta_mode = (beta == 0.0) ? 0 : (beta == 1.0 ? 1 : 2);
     p.alpha = alpha; p.beta = beta;
     p.c = C; p.ldc = ldc;
     p.cin = C;
     p.row_exp = ea; p.col_exp = eb;
     p.err = device_error_word();
-    if (tail_tiles > 0) {
-        p.tail_tiles = tail_tiles;
+    if (p.tail_tiles > 0)
         p.ws = reinterpret_cast<double*>(static_cast<uint8_t*>(buf) + exps + a_bytes + b_bytes);
-    }
 
     e = ozaki_kernel_attributes();
     if (e != cudaSuccess) { cudaFreeAsync(buf, st); return e; }
-    const int items = p.num_tiles + p.tail_tiles * (p.kchunks * upc - 1);
-    const int grid = items < sms ? items : sms;
     KernelTimer tmr;
     kernel_timing_begin("umma_ozaki_i8", 2.0 * m * n * static_cast<double>(k) * slices * (slices + 1) / 2, st, &tmr);
-    if (un == 256) ozaki_gemm_kernel<256><<<grid, kOzThreads, OzCfg<256>::SMEM, st>>>(tma, tmb, p);
-    else           ozaki_gemm_kernel<128><<<grid, kOzThreads, OzCfg<128>::SMEM, st>>>(tma, tmb, p);
+    if (pair) {
+        ozaki_pair_kernel<<<2 * std::min(pz_items(p), sms / 2), kPzThreads, kPzSmem, st>>>(tma, tmb, p);
+    } else {
+        const int items = p.num_tiles + p.tail_tiles * (p.kchunks * upc - 1);
+        const int grid = items < sms ? items : sms;
+        if (un == 256) ozaki_gemm_kernel<256><<<grid, kOzThreads, OzCfg<256>::SMEM, st>>>(tma, tmb, p);
+        else           ozaki_gemm_kernel<128><<<grid, kOzThreads, OzCfg<128>::SMEM, st>>>(tma, tmb, p);
+    }
     kernel_timing_end(&tmr, st);
     count_launch();
     if (p.tail_tiles > 0) {
-        const size_t elems = static_cast<size_t>(p.tail_tiles) * kUM * un;
-        const size_t blocks = std::min<size_t>((elems + 255) / 256, static_cast<size_t>(sms) * 16);
-        ozaki_reduce_kernel<<<static_cast<unsigned>(blocks), 256, 0, st>>>(p, p.kchunks * upc);
+        const size_t work = static_cast<size_t>(p.tail_tiles) * um * un / (pair ? 2 : 1);
+        const unsigned blocks = static_cast<unsigned>(std::min<size_t>((work + 255) / 256, static_cast<size_t>(sms) * 16));
+        if (pair) ozaki_pair_reduce_kernel<<<blocks, 256, 0, st>>>(p);
+        else      ozaki_reduce_kernel<<<blocks, 256, 0, st>>>(p, p.kchunks * upc);
         count_launch();
     }
     e = cudaGetLastError();
@@ -2595,6 +3190,9 @@ int ozaki_grouped_dev(const rb_gemm_problem* probs, size_t count, const void* co
                       cudaStream_t st, int32_t* ce) {
     const int slices = rb_get_ozaki_slices();
     const long long kt_chunk = std::max(2147483647LL / (static_cast<long long>(slices) * 128 * 128) / 128, 1LL);
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     struct Job {
         bool ta, tb;
         int m, n, k;
@@ -2606,7 +3204,7 @@ int ozaki_grouped_dev(const rb_gemm_problem* probs, size_t count, const void* co
         double alpha, beta;
         size_t kp, off_exp, off_a, off_b;
         int num_kt;
-        int un;  // tile width
+        int kind;  // 0: CTA pairs; 1, 2: 256- and 128-wide tiles
     };
     std::vector<Job> jobs;
     jobs.reserve(count);
@@ -2657,7 +3255,7 @@ int ozaki_grouped_dev(const rb_gemm_problem* probs, size_t count, const void* co
         j.beta = q.beta;
         j.kp = round_up(q.k, 16);
         j.num_kt = static_cast<int>((q.k + 127) / 128);
-        j.un = ozaki_tile_n(j.m, j.n, j.k);
+        j.kind = sms >= 2 && ozaki_pair_tiles(j.m, j.n) ? 0 : ozaki_tile_n(j.m, j.n, j.k) == 256 ? 1 : 2;
         j.off_exp = exps;
         exps += m + n;
         j.off_a = planes;
@@ -2671,15 +3269,15 @@ int ozaki_grouped_dev(const rb_gemm_problem* probs, size_t count, const void* co
         return RB_ERR_CUDA;
     }
     if (jobs.empty()) return RB_OK;
-    // one launch per tile width, wide tiles first; inside each, longest tiles
-    // first: the CTAs walk the items with a stride of the grid
+    // one launch per kind of tile; inside each, longest tiles first: the CTAs
+    // walk the items with a stride of the grid
     std::stable_sort(jobs.begin(), jobs.end(), [](const Job& x, const Job& y) {
-        return x.un != y.un ? x.un > y.un : x.num_kt > y.num_kt;
+        return x.kind != y.kind ? x.kind < y.kind : x.num_kt > y.num_kt;
     });
     const int np = static_cast<int>(jobs.size());
     // device image: [entries][starts][operands] then exponents, then planes
     const size_t ent_bytes = round_up(np * sizeof(OzGroupEntry), 256);
-    const size_t starts_bytes = round_up((np + 2) * sizeof(int), 256);  // starts of each width's table
+    const size_t starts_bytes = round_up((np + 3) * sizeof(int), 256);  // each kind's starts and its end
     const size_t ops_bytes = round_up(2 * np * sizeof(OzOperand), 256);
     const size_t img_bytes = ent_bytes + starts_bytes + ops_bytes;
     const size_t exp_bytes = round_up(exps * sizeof(int), 256);
@@ -2696,8 +3294,10 @@ int ozaki_grouped_dev(const rb_gemm_problem* probs, size_t count, const void* co
     int* dexp = reinterpret_cast<int*>(mem + img_bytes);
     int8_t* dplanes = reinterpret_cast<int8_t*>(mem + img_bytes + exp_bytes);
     uint32_t* err_word = device_error_word();
-    int tiles = 0, exp_blocks = 0, slice_blocks = 0;
-    int n_wide = 0, tiles_wide = 0;  // the problems (and their tiles) of the 256-wide launch
+    int exp_blocks = 0, slice_blocks = 0;
+    int kind_first[3] = {}, kind_count[3] = {}, kind_tiles[3] = {};  // problems and tiles of each launch
+    for (const Job& j : jobs) ++kind_count[j.kind];
+    for (int q = 1; q < 3; ++q) kind_first[q] = kind_first[q - 1] + kind_count[q - 1];
     double work = 0;
     CUresult r = CUDA_SUCCESS;
     for (int i = 0; i < np && r == CUDA_SUCCESS; ++i) {
@@ -2728,12 +3328,14 @@ int ozaki_grouped_dev(const rb_gemm_problem* probs, size_t count, const void* co
         OzGroupEntry g{};  // 64-byte aligned here; copied into the image below
         r = make_tmap_planes(&g.tmA, sla, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, j.k, j.m, slices, j.kp, kUM);
         if (r == CUDA_SUCCESS)
-            r = make_tmap_planes(&g.tmB, slb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, j.k, j.n, slices, j.kp, j.un);
+            r = make_tmap_planes(&g.tmB, slb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, j.k, j.n, slices, j.kp,
+                                 j.kind == 0 ? 64 : j.kind == 1 ? 256 : 128);
         OzParams& p = g.p;
         p.m = j.m; p.n = j.n; p.k = j.k;
-        p.un = j.un;
-        p.tiles_m = (j.m + kUM - 1) / kUM;
-        p.tiles_n = (j.n + j.un - 1) / j.un;
+        const int um = j.kind == 0 ? 256 : kUM;
+        p.un = j.kind == 1 ? 256 : 128;
+        p.tiles_m = (j.m + um - 1) / um;
+        p.tiles_n = (j.n + p.un - 1) / p.un;
         p.num_tiles = p.tiles_m * p.tiles_n;
         p.num_kt = j.num_kt;
         p.slices = slices;
@@ -2746,28 +3348,18 @@ int ozaki_grouped_dev(const rb_gemm_problem* probs, size_t count, const void* co
         p.row_exp = ea; p.col_exp = eb;
         p.err = err_word;
         std::memcpy(img.data() + i * sizeof(OzGroupEntry), &g, sizeof(OzGroupEntry));
-        // the wide launch's starts at [0, n_wide], the narrow launch's at
-        // [n_wide + 1, np + 1], each counting from its own first tile
-        if (j.un == 256) {
-            starts[i] = tiles;
-            n_wide = i + 1;
-            tiles_wide = tiles + p.num_tiles;
-        } else {
-            starts[i + 1] = tiles - tiles_wide;
-        }
-        tiles += p.num_tiles;
+        // kind q's starts, counting from its own first tile, and its end at
+        // [kind_first[q] + q, kind_first[q] + kind_count[q] + q]
+        starts[i + j.kind] = kind_tiles[j.kind];
+        kind_tiles[j.kind] += p.num_tiles;
         work += 2.0 * j.m * j.n * static_cast<double>(j.k) * slices * (slices + 1) / 2;
     }
-    starts[n_wide] = tiles_wide;        // end of the wide table
-    starts[np + 1] = tiles - tiles_wide;  // end of the narrow table (at n_wide + 1 .. np + 1)
+    for (int q = 0; q < 3; ++q) starts[kind_first[q] + kind_count[q] + q] = kind_tiles[q];
     if (r != CUDA_SUCCESS) {
         if (ce) *ce = static_cast<int32_t>(r);
         cudaFreeAsync(mem, st);
         return RB_ERR_CUDA;
     }
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     e = ozaki_kernel_attributes();
     // a pageable source: the driver has staged the image when the call returns
     if (e == cudaSuccess) e = cudaMemcpyAsync(mem, img.data(), img_bytes, cudaMemcpyHostToDevice, st);
@@ -2788,27 +3380,37 @@ int ozaki_grouped_dev(const rb_gemm_problem* probs, size_t count, const void* co
         kernel_timing_begin("umma_ozaki_grouped_i8", work, st, &tmr);
         const OzGroupEntry* dtab = reinterpret_cast<const OzGroupEntry*>(mem);
         const int* dstarts = reinterpret_cast<const int*>(mem + ent_bytes);
-        const int tiles_narrow = tiles - tiles_wide;
-        // with both widths, the narrow launch goes on a forked stream: its
-        // CTAs take the SMs that the wide launch's CTAs leave as they finish
-        // (each persistent CTA holds a whole SM), instead of waiting for the
-        // wide launch's last tile
+        // with more than one kind, the first goes on st and the others on a
+        // forked stream: their CTAs take the SMs that the first launch's leave
+        // as they finish (each persistent CTA holds a whole SM), instead of
+        // waiting for its last tile
+        const int kinds = (kind_count[0] > 0) + (kind_count[1] > 0) + (kind_count[2] > 0);
         ForkedStream fk;
-        const bool fork = n_wide > 0 && np > n_wide && fork_stream(st, &fk) == cudaSuccess;
-        if (n_wide > 0)
-            ozaki_grouped_kernel<256><<<std::min(tiles_wide, sms), kOzThreads, OzCfg<256>::SMEM, st>>>(
-                dtab, dstarts, n_wide, err_word);
-        if (np > n_wide)
-            ozaki_grouped_kernel<128><<<std::min(tiles_narrow, sms), kOzThreads, OzCfg<128>::SMEM,
-                                        fork ? fk.s : st>>>(dtab + n_wide, dstarts + n_wide + 1, np - n_wide,
-                                                            err_word);
+        const bool fork = kinds > 1 && fork_stream(st, &fk) == cudaSuccess;
+        bool started = false;
+        for (int q = 0; q < 3; ++q) {
+            if (kind_count[q] == 0) continue;
+            const cudaStream_t ks = started && fork ? fk.s : st;
+            started = true;
+            const OzGroupEntry* kt = dtab + kind_first[q];
+            const int* ks0 = dstarts + kind_first[q] + q;
+            if (q == 0)
+                ozaki_pair_grouped_kernel<<<2 * std::min(kind_tiles[0], sms / 2), kPzThreads, kPzSmem, ks>>>(
+                    kt, ks0, kind_count[0], err_word);
+            else if (q == 1)
+                ozaki_grouped_kernel<256><<<std::min(kind_tiles[1], sms), kOzThreads, OzCfg<256>::SMEM, ks>>>(
+                    kt, ks0, kind_count[1], err_word);
+            else
+                ozaki_grouped_kernel<128><<<std::min(kind_tiles[2], sms), kOzThreads, OzCfg<128>::SMEM, ks>>>(
+                    kt, ks0, kind_count[2], err_word);
+        }
         e = cudaGetLastError();
         if (fork) {
             const cudaError_t je = join_stream(st, &fk);
             if (e == cudaSuccess) e = je;
         }
         kernel_timing_end(&tmr, st);
-        count_launch(3 + (n_wide > 0) + (np > n_wide));
+        count_launch(3 + kinds);
         if (e == cudaSuccess) e = cudaGetLastError();
     }
     cudaFreeAsync(mem, st);

@@ -116,6 +116,19 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
+// One lane of a converged warp. A warp whose loop all lanes run, with only the
+// tcgen05 instructions under this predicate, keeps their operands in uniform
+// registers; a loop run by one lane moves each operand there per instruction,
+// ~60 clocks an MMA.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(p));
+    return p != 0;
+}
 // Arrive once on CTA `rank`'s copy of `bar` (same offset in both CTAs).
 __device__ __forceinline__ void mbar_arrive_rank(uint64_t* bar, uint32_t rank) {
     asm volatile(
@@ -125,10 +138,11 @@ __device__ __forceinline__ void mbar_arrive_rank(uint64_t* bar, uint32_t rank) {
         "r"(rank)
         : "memory");
 }
-// The same without the release: for an arrival that hands over TMEM columns
-// after tcgen05.wait::ld, with no memory write to publish. (A cluster-scope
-// release first waits for the thread's outstanding stores: ~2000 clocks after
-// a tile's C stores or a spill.)
+// The same without the release, for an arrival with no memory write of this
+// thread to publish: TMEM columns handed over after tcgen05.wait::ld, or the
+// word that a TMA stage (written by the async proxy before its barrier's phase
+// completed) has landed. (A cluster-scope release first waits for outstanding
+// stores, ~1000 clocks and more beside an epilogue's.)
 __device__ __forceinline__ void mbar_arrive_rank_relaxed(uint64_t* bar, uint32_t rank) {
     asm volatile(
         "{\n\t.reg .b32 ra;\n\t"
@@ -350,6 +364,12 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
                    "=r"(r[7])
+                 : "r"(taddr));
+}
+// 32 lanes x 4 consecutive 32-bit columns.
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_ld_wait() {

@@ -211,6 +211,7 @@ constexpr int kGroupedMaxSplit = 16;
 int ozaki_tile_n(size_t m, size_t n, size_t k);
 void set_tuned_ozaki_widths(std::shared_ptr<const std::map<uint32_t, int>> table);
 void force_ozaki_width(int w);
+bool ozaki_width_forced();
 
 // rblas's argument checks for one table entry (dtype, layout, transposes,
 // leading dimensions) plus the 32-bit tile-index limit; an rb_status value.
