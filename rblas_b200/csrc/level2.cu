@@ -7,24 +7,25 @@
 // through its column-major view (R x C, leading dimension ld): a row-major
 // A is the column-major view of its transpose, which swaps the two gemv
 // kernels and the roles of x and y in the rank-1 update.
-//   * "column sweep" gemv (y_r = sum_c A[r,c] x_c): one thread per row of
-//     the view, consecutive threads on consecutive rows (coalesced), the
-//     columns split into S ranges when there are too few rows to fill the
-//     GPU; each range's partial sums go to a workspace.
-//   * "column dot" gemv (y_c = sum_r A[r,c] x_r): one CTA per (column, row
-//     range), 256 threads striding down the column, a fixed-order block
-//     reduction.
-//   * a finalize pass applies rblas's beta pass and alpha: partial sums are
-//     added in range order, so results do not depend on timing.
+//   * "column sweep" gemv (y_r = sum_c A[r,c] x_c): a CTA per (row tile, range
+//     of columns), its warps on every eighth column; few columns: one thread
+//     per row.
+//   * "column dot" gemv (y_c = sum_r A[r,c] x_r): four columns at a time per
+//     CTA (per warp, for short ones) and row range, a fixed-order reduction.
+//   * the ranges (S of them, only when there are too few tiles to fill the
+//     GPU) go through a workspace and a finalize pass in range order; a single
+//     range applies rblas's beta pass and alpha itself. Results do not depend
+//     on timing.
 // Within one range the terms are added in rblas's order (fma(a, x, acc) for
-// real, acc + a*x with rblas's complex multiply for complex), so a call that
-// needs a single range reproduces rblas's gemv for NoTrans column-major
+// real, acc + a*x with rblas's complex multiply for complex), so a NoTrans
+// column-major call of fewer than kSweepSplit columns reproduces rblas's gemv
 // exactly; other shapes differ from rblas's order within rounding.
 // The rank-1 update computes each element as rblas does (alpha*x_i rounded,
 // then fma / complex multiply-add), so it matches rblas bit for bit.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstring>
 
 #include "../../include/rblas_b200.h"
 #include "rb_internal.h"
@@ -92,7 +93,61 @@ __device__ __forceinline__ C2<T> shfl_el(C2<T> v, int o) {
 
 constexpr int kL2Threads = 256;
 
-// y_r partial over columns [c0, c1) of range s: ws[s * R + r]. A CTA covers
+// V consecutive elements: one 16-byte load (VEC) or V element loads.
+template <typename E, int V> struct Pack { E e[V]; };
+template <bool VEC, int V, typename E>
+__device__ __forceinline__ Pack<E, V> ld_pack(const E* p) {
+    Pack<E, V> r;
+    if constexpr (VEC) {
+        static_assert(sizeof(Pack<E, V>) == 16, "a vector is 16 bytes");
+        const uint4 t = __ldg(reinterpret_cast<const uint4*>(p));
+        memcpy(&r, &t, 16);
+    } else {
+#pragma unroll
+        for (int i = 0; i < V; ++i) r.e[i] = ld_el(p + i);
+    }
+    return r;
+}
+template <typename E> constexpr int kVecLen = 16 / static_cast<int>(sizeof(E));
+
+template <typename E>
+__device__ __forceinline__ E warp_sum(E acc) {  // a fixed tree; lane 0 has the sum
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc = add_el(acc, shfl_el(acc, o));
+    return acc;
+}
+
+// The last step on y_i given the sum (have) or an empty one (see gemv_finalize).
+template <typename T>
+__device__ __forceinline__ void finish_y(T* yp, T acc, T alpha, T beta) {
+    T yi = *yp;
+    if (beta != T(1)) yi = (beta == T(0)) ? T(0) : mul_rn(beta, yi);
+    *yp = fma(alpha, acc, yi);
+}
+template <typename T>
+__device__ __forceinline__ void finish_y(C2<T>* yp, C2<T> acc, C2<T> alpha, C2<T> beta) {
+    C2<T> yi = *yp;
+    const bool beta_zero = beta.re == T(0) && beta.im == T(0);
+    yi = beta_zero ? C2<T>{T(0), T(0)} : cmul(beta, yi);
+    *yp = cadd(yi, cmul(alpha, acc));
+}
+
+// Where a sum goes: y itself (one range) or the range's row of the workspace.
+template <typename E>
+struct GemvOut {
+    E* y;
+    long long incy;
+    E alpha, beta;
+    E* ws;  // null: finish y
+    int len;
+};
+template <typename E>
+__device__ __forceinline__ void put(const GemvOut<E>& o, int i, int s, E acc) {
+    if (o.ws) o.ws[static_cast<size_t>(s) * o.len + i] = acc;
+    else      finish_y(o.y + static_cast<long long>(i) * o.incy, acc, o.alpha, o.beta);
+}
+
+// y_r over few columns, in column order. A CTA covers
 // kSweepRows consecutive rows (each thread kRowsPerThread of them, 256 apart,
 // so every warp load stays one contiguous 256-byte run and the CTA reads
 // 8 KB contiguous per f64 column); the accumulators are independent.
@@ -102,10 +157,8 @@ constexpr int kSweepRows = kL2Threads * kRowsPerThread;
 template <typename E>
 __global__ void __launch_bounds__(kL2Threads)
     gemv_sweep_kernel(const E* __restrict__ A, size_t ld, int R, int C, const E* __restrict__ x, long long incx,
-                      int conj, int cchunk, E* __restrict__ ws) {
+                      int conj, GemvOut<E> o) {
     const int rbase = blockIdx.x * kSweepRows + threadIdx.x;
-    const int s = blockIdx.y;
-    const int c0 = s * cchunk, c1 = min(C, c0 + cchunk);
     E acc[kRowsPerThread];
     bool live[kRowsPerThread];
 #pragma unroll
@@ -114,7 +167,7 @@ __global__ void __launch_bounds__(kL2Threads)
         live[q] = rbase + q * kL2Threads < R;
     }
 #pragma unroll 4
-    for (int c = c0; c < c1; ++c) {
+    for (int c = 0; c < C; ++c) {
         const E xc = ld_el(x + static_cast<long long>(c) * incx);
         const E* col = A + static_cast<size_t>(c) * ld + rbase;
 #pragma unroll
@@ -128,37 +181,138 @@ __global__ void __launch_bounds__(kL2Threads)
     }
 #pragma unroll
     for (int q = 0; q < kRowsPerThread; ++q)
-        if (live[q]) ws[static_cast<size_t>(s) * R + rbase + q * kL2Threads] = acc[q];
+        if (live[q]) put(o, rbase + q * kL2Threads, 0, acc[q]);
 }
 
-// y_c partial over rows [r0, r1) of range s: ws[s * C + c]
-template <typename E>
+// Column dot: y_c over rows [r0, r1) of range s. The CTA takes two columns at
+// once, so that a value of x is read once for both and two 16-byte loads of A
+// are in flight per step (one column with 8-byte loads: 4.3 TB/s at 6000 x
+// 4000 f64; two: 6.2, four: 5.6). Short columns (at most kShortRows) of which
+// there are enough take a warp each (256 x 16384 f32: 18.2 -> 6.3 us).
+// VA / VX: 16-byte loads of A / x.
+constexpr int kDotCols = 2;
+constexpr int kShortRows = 1024;
+
+// W warps (the CTA's 8, or 1) per group of COLS columns.
+template <typename E, int W, int COLS, bool VA, bool VX>
 __global__ void __launch_bounds__(kL2Threads)
     gemv_dot_kernel(const E* __restrict__ A, size_t ld, int R, int C, const E* __restrict__ x, long long incx,
-                    int conj, int rchunk, E* __restrict__ ws) {
-    __shared__ E part[kL2Threads / 32];
-    const int c = blockIdx.x, s = blockIdx.y;
-    const int r0 = s * rchunk, r1 = min(R, r0 + rchunk);
-    const E* a = A + static_cast<size_t>(c) * ld;
-    E acc = zero_el(static_cast<E*>(nullptr));
-#pragma unroll 8
-    for (int r = r0 + threadIdx.x; r < r1; r += kL2Threads) {
-        E v = ld_el(a + r);
-        if (conj) v = conj_el(v);
-        acc = mac(acc, v, ld_el(x + static_cast<long long>(r) * incx));
-    }
-    // fixed-order reduction: warp tree, then the warps' sums in warp order
+                    int conj, int rchunk, GemvOut<E> o) {
+    constexpr int V = kVecLen<E>, LANES = W * 32;
+    const int t = threadIdx.x % LANES, s = blockIdx.y;
+    const int c0 = (blockIdx.x * (kL2Threads / LANES) + threadIdx.x / LANES) * COLS;
+    const int r0 = s * rchunk, r1 = min(R, r0 + rchunk);  // rchunk: a multiple of V
+    const E* a[COLS];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc = add_el(acc, shfl_el(acc, o));
+    for (int q = 0; q < COLS; ++q) a[q] = A + static_cast<size_t>(min(c0 + q, C - 1)) * ld;
+    E acc[COLS][V];
+#pragma unroll
+    for (int q = 0; q < COLS; ++q)
+#pragma unroll
+        for (int i = 0; i < V; ++i) acc[q][i] = zero_el(static_cast<E*>(nullptr));
+    if (c0 < C) {
+#pragma unroll 2
+        for (int r = r0 + t * V; r + V <= r1; r += LANES * V) {
+            Pack<E, V> v[COLS], xv;
+#pragma unroll
+            for (int q = 0; q < COLS; ++q) v[q] = ld_pack<VA, V>(a[q] + r);
+            if constexpr (VX) {
+                xv = ld_pack<true, V>(x + r);
+            } else {
+#pragma unroll
+                for (int i = 0; i < V; ++i) xv.e[i] = ld_el(x + (static_cast<long long>(r) + i) * incx);
+            }
+#pragma unroll
+            for (int q = 0; q < COLS; ++q)
+#pragma unroll
+                for (int i = 0; i < V; ++i)
+                    acc[q][i] = mac(acc[q][i], conj ? conj_el(v[q].e[i]) : v[q].e[i], xv.e[i]);
+        }
+        const int rl = r0 + (r1 - r0) / V * V + t;  // fewer than V rows are left
+        if (t < V && rl < r1) {
+            const E xv = ld_el(x + static_cast<long long>(rl) * incx);
+#pragma unroll
+            for (int q = 0; q < COLS; ++q) {
+                const E v = ld_el(a[q] + rl);
+                acc[q][0] = mac(acc[q][0], conj ? conj_el(v) : v, xv);
+            }
+        }
+    }
+    // fixed-order reduction: a thread's V sums, the warp tree, the warps in order
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0) part[warp] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        E t = part[0];
+    __shared__ E part[COLS][kL2Threads / 32];
 #pragma unroll
-        for (int w = 1; w < kL2Threads / 32; ++w) t = add_el(t, part[w]);
-        ws[static_cast<size_t>(s) * C + c] = t;
+    for (int q = 0; q < COLS; ++q) {
+#pragma unroll
+        for (int w = V / 2; w > 0; w >>= 1)
+#pragma unroll
+            for (int i = 0; i < w; ++i) acc[q][i] = add_el(acc[q][i], acc[q][i + w]);
+        const E sum = warp_sum(acc[q][0]);
+        if constexpr (W == 1) {
+            if (lane == 0 && c0 + q < C) put(o, c0 + q, s, sum);
+        } else {
+            if (lane == 0) part[q][warp] = sum;
+        }
     }
+    if constexpr (W > 1) {
+        __syncthreads();
+        if (threadIdx.x < COLS && c0 + static_cast<int>(threadIdx.x) < C) {
+            E sum = part[threadIdx.x][0];
+#pragma unroll
+            for (int w = 1; w < kL2Threads / 32; ++w) sum = add_el(sum, part[threadIdx.x][w]);
+            put(o, c0 + threadIdx.x, s, sum);
+        }
+    }
+}
+
+// Column sweep of at least kSweepSplit columns: y_r over columns [c0, c1) of
+// range s. A CTA takes 64 rows; its eight warps take every eighth column of
+// the range and their sums are added in warp order, so few ranges fill the
+// GPU: with one thread per row and up to 198 ranges, the finalize pass's
+// serial sum of the ranges was most of the time. Element loads: 16-byte ones
+// of 64 to 256 rows were slower (6000 x 4000 f64: 33 us; 44-52 with them, 56
+// before; 256 x 16384: 98 -> 15).
+constexpr int kSweepPack = 2;
+constexpr int kSweepSplit = 32;  // fewer columns: gemv_sweep_kernel in one range, rblas's own order
+constexpr int kSplitRows = 32 * kSweepPack;
+
+template <typename E>
+__global__ void __launch_bounds__(kL2Threads)
+    gemv_split_kernel(const E* __restrict__ A, size_t ld, int R, int C, const E* __restrict__ x, long long incx,
+                      int conj, int cchunk, GemvOut<E> o) {
+    constexpr int WARPS = kL2Threads / 32;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, s = blockIdx.y;
+    const int rb = blockIdx.x * kSplitRows + lane;
+    const int c0 = s * cchunk, c1 = min(C, c0 + cchunk);
+    E acc[kSweepPack];
+    bool live[kSweepPack];
+#pragma unroll
+    for (int q = 0; q < kSweepPack; ++q) {
+        acc[q] = zero_el(static_cast<E*>(nullptr));
+        live[q] = rb + q * 32 < R;
+    }
+#pragma unroll 4
+    for (int c = c0 + warp; c < c1; c += WARPS) {
+        const E* col = A + static_cast<size_t>(c) * ld + rb;
+        const E xc = ld_el(x + static_cast<long long>(c) * incx);
+#pragma unroll
+        for (int q = 0; q < kSweepPack; ++q)
+            if (live[q]) {
+                E v = ld_el(col + q * 32);
+                if (conj) v = conj_el(v);
+                acc[q] = mac(acc[q], v, xc);
+            }
+    }
+    __shared__ E part[WARPS][kSplitRows];
+#pragma unroll
+    for (int q = 0; q < kSweepPack; ++q) part[warp][q * 32 + lane] = acc[q];
+    __syncthreads();
+    const int r = blockIdx.x * kSplitRows + threadIdx.x;
+    if (threadIdx.x >= kSplitRows || r >= R) return;
+    E sum = part[0][threadIdx.x];
+#pragma unroll
+    for (int w = 1; w < WARPS; ++w) sum = add_el(sum, part[w][threadIdx.x]);
+    put(o, r, s, sum);
 }
 
 // rblas's beta pass, then y += alpha * (sum of the S partials in range order).
@@ -167,45 +321,53 @@ __global__ void __launch_bounds__(kL2Threads)
 // the beta pass always runs (beta == 0 writes 0, else beta*y with the
 // complex multiply); then y = y + alpha*acc. alpha == 0 stops after the
 // beta pass.
-// alpha_mode: 0 no alpha step; 1 add alpha * (sum of the S partials);
-// 2 add alpha * 0 (rblas still runs the step on an empty sum).
+// alpha_mode: 0 no alpha step; 2 add alpha * 0 (rblas still runs the step on
+// an empty sum). A non-empty sum ends in finish_y.
 template <typename T>
-__global__ void gemv_finalize_real(T* y, long long incy, int len, const T* __restrict__ ws, int S, T alpha, T beta,
-                                   int alpha_mode) {
+__global__ void gemv_beta_real(T* y, long long incy, int len, T alpha, T beta, int alpha_mode) {
     const int i = blockIdx.x * kL2Threads + threadIdx.x;
     if (i >= len) return;
     T* yp = y + static_cast<long long>(i) * incy;
     T yi = *yp;
     if (beta != T(1)) yi = (beta == T(0)) ? T(0) : mul_rn(beta, yi);
-    if (alpha_mode != 0) {
-        T acc = T(0);
-        if (alpha_mode == 1) {
-            acc = ws[i];
-            for (int s = 1; s < S; ++s) acc = add_rn(acc, ws[static_cast<size_t>(s) * len + i]);
-        }
-        yi = fma(alpha, acc, yi);
-    }
+    if (alpha_mode != 0) yi = fma(alpha, T(0), yi);
     *yp = yi;
 }
 
 template <typename T>
-__global__ void gemv_finalize_cplx(C2<T>* y, long long incy, int len, const C2<T>* __restrict__ ws, int S,
-                                   C2<T> alpha, C2<T> beta, int alpha_mode) {
+__global__ void gemv_beta_cplx(C2<T>* y, long long incy, int len, C2<T> alpha, C2<T> beta, int alpha_mode) {
     const int i = blockIdx.x * kL2Threads + threadIdx.x;
     if (i >= len) return;
     C2<T>* yp = y + static_cast<long long>(i) * incy;
     C2<T> yi = *yp;
     const bool beta_zero = beta.re == T(0) && beta.im == T(0);
     yi = beta_zero ? C2<T>{T(0), T(0)} : cmul(beta, yi);
-    if (alpha_mode != 0) {
-        C2<T> acc{T(0), T(0)};
-        if (alpha_mode == 1) {
-            acc = ws[i];
-            for (int s = 1; s < S; ++s) acc = cadd(acc, ws[static_cast<size_t>(s) * len + i]);
-        }
-        yi = cadd(yi, cmul(alpha, acc));
-    }
+    if (alpha_mode != 0) yi = cadd(yi, cmul(alpha, C2<T>{T(0), T(0)}));
     *yp = yi;
+}
+
+// Sum of the S ranges' partials, then finish_y. A CTA takes 32 elements; its
+// eight warps sum an eighth of the ranges each, in order, and the eighths are
+// added in order.
+template <typename E>
+__global__ void __launch_bounds__(kL2Threads) gemv_finalize(GemvOut<E> o, int S) {
+    constexpr int WARPS = kL2Threads / 32;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = blockIdx.x * 32 + lane;
+    const int per = (S + WARPS - 1) / WARPS, s0 = warp * per, s1 = min(S, s0 + per);
+    __shared__ E part[WARPS][32];
+    E acc = zero_el(static_cast<E*>(nullptr));
+    if (i < o.len && s0 < s1) {
+        acc = o.ws[static_cast<size_t>(s0) * o.len + i];
+#pragma unroll 8
+        for (int s = s0 + 1; s < s1; ++s) acc = add_el(acc, o.ws[static_cast<size_t>(s) * o.len + i]);
+    }
+    part[warp][lane] = acc;
+    __syncthreads();
+    if (warp != 0 || i >= o.len) return;
+#pragma unroll
+    for (int w = 1; w < WARPS; ++w)
+        if (w * per < S) acc = add_el(acc, part[w][lane]);
+    finish_y(o.y + static_cast<long long>(i) * o.incy, acc, o.alpha, o.beta);
 }
 
 // A[r, c] (column-major view) += alpha*x (.) y: the x index is the view's
@@ -303,45 +465,80 @@ int gemv_dev(int layout, int trans, size_t m, size_t n, T ar, T ai, const T* A, 
     const bool sweep = (col && !tr) || (!col && tr);
     const int conj = (CX && trans == RB_CONJ_TRANS) ? 1 : 0;
     const int len = static_cast<int>(leny);
+    const bool have_work = !alpha_zero && R > 0 && Cc > 0;
+    E ea, eb;
+    if constexpr (CX) {
+        ea = E{ar, ai};
+        eb = E{br, bi};
+    } else {
+        ea = ar;
+        eb = br;
+    }
+    E* yv = reinterpret_cast<E*>(y);
+    if (!have_work) {
+        // rblas runs the alpha step on an empty sum too, except for the real
+        // Trans loop, which has no step when m == 0 (src/level2.rs:41-60,
+        // src/complex2.rs:55-76)
+        const int alpha_mode = alpha_zero ? 0 : ((!CX && tr) ? 0 : 2);
+        if constexpr (CX) gemv_beta_cplx<T><<<blocks_for(len), kL2Threads, 0, st>>>(yv, incy, len, ea, eb, alpha_mode);
+        else              gemv_beta_real<T><<<blocks_for(len), kL2Threads, 0, st>>>(yv, incy, len, ea, eb, alpha_mode);
+        count_launch();
+        const cudaError_t e0 = cudaGetLastError();
+        return e0 == cudaSuccess ? RB_OK : fail(e0, ce);
+    }
+    const E* Av = reinterpret_cast<const E*>(A);
+    const E* xv = reinterpret_cast<const E*>(x);
+    constexpr int V = kVecLen<E>;
+    const bool va = reinterpret_cast<uintptr_t>(A) % 16 == 0 && (lda * sizeof(E)) % 16 == 0;
+    const bool vx = incx == 1 && reinterpret_cast<uintptr_t>(x) % 16 == 0;
+    // ranges (S) so that the grid fills the GPU, each with enough work
     int S = 1, chunk = 0;
-    const int target = 148 * 8;  // CTAs for a full GPU at 8 resident CTAs per SM
-    bool have_work = !alpha_zero && R > 0 && Cc > 0;
-    if (have_work) {
-        if (sweep) {
-            const int rb = (R + kSweepRows - 1) / kSweepRows;
-            S = std::max(1, std::min((target + rb - 1) / rb, std::max(1, Cc / 16)));
-            chunk = (Cc + S - 1) / S;
-            S = (Cc + chunk - 1) / chunk;
-        } else {
-            S = std::max(1, std::min((target + Cc - 1) / Cc, std::max(1, R / 1024)));
-            chunk = (R + S - 1) / S;
-            S = (R + chunk - 1) / chunk;
-        }
+    dim3 grid;
+    const bool split = sweep && Cc >= kSweepSplit;
+    const bool short_cols = !sweep && R <= kShortRows && Cc >= 148 * 4 * (kL2Threads / 32);
+    if (split) {
+        const int rb = (R + kSplitRows - 1) / kSplitRows;
+        S = std::max(1, std::min(148 * 8 / rb, Cc / 32));
+        chunk = (Cc + S - 1) / S;
+        S = (Cc + chunk - 1) / chunk;
+        grid = dim3(rb, S);
+    } else if (sweep) {
+        grid = dim3((R + kSweepRows - 1) / kSweepRows);
+    } else {
+        const int cols = short_cols ? kL2Threads / 32 : kDotCols, cb = (Cc + cols - 1) / cols;
+        if (!short_cols) S = std::max(1, std::min((148 * 4 + cb - 1) / cb, R / 1024));
+        chunk = ((R + S - 1) / S + V - 1) / V * V;
+        S = (R + chunk - 1) / chunk;
+        grid = dim3(cb, S);
     }
     E* ws = nullptr;
     cudaError_t e;
-    if (have_work) {
-        if ((e = scratch_alloc(&ws, static_cast<size_t>(S) * len * sizeof(E), st)) != cudaSuccess) return fail(e, ce);
-        const E* Av = reinterpret_cast<const E*>(A);
-        const E* xv = reinterpret_cast<const E*>(x);
-        if (sweep)
-            gemv_sweep_kernel<E><<<dim3((R + kSweepRows - 1) / kSweepRows, S), kL2Threads, 0, st>>>(
-                Av, lda, R, Cc, xv, incx, conj, chunk, ws);
-        else
-            gemv_dot_kernel<E><<<dim3(Cc, S), kL2Threads, 0, st>>>(Av, lda, R, Cc, xv, incx, conj, chunk, ws);
+    if (S > 1 && (e = scratch_alloc(&ws, static_cast<size_t>(S) * len * sizeof(E), st)) != cudaSuccess)
+        return fail(e, ce);
+    const GemvOut<E> o{yv, incy, ea, eb, ws, len};
+    if (split) {
+        gemv_split_kernel<E><<<grid, kL2Threads, 0, st>>>(Av, lda, R, Cc, xv, incx, conj, chunk, o);
+    } else if (sweep) {
+        gemv_sweep_kernel<E><<<grid, kL2Threads, 0, st>>>(Av, lda, R, Cc, xv, incx, conj, o);
+    } else {
+#define RB_DOT(W, COLS, VA, VX) \
+    gemv_dot_kernel<E, W, COLS, VA, VX><<<grid, kL2Threads, 0, st>>>(Av, lda, R, Cc, xv, incx, conj, chunk, o)
+        if (short_cols) {
+            if (va && vx)      RB_DOT(1, 1, true, true);
+            else if (va)       RB_DOT(1, 1, true, false);
+            else               RB_DOT(1, 1, false, false);
+        } else {
+            if (va && vx)      RB_DOT(8, kDotCols, true, true);
+            else if (va)       RB_DOT(8, kDotCols, true, false);
+            else               RB_DOT(8, kDotCols, false, false);
+        }
+#undef RB_DOT
+    }
+    count_launch();
+    if (S > 1) {
+        gemv_finalize<E><<<(len + 31) / 32, kL2Threads, 0, st>>>(o, S);
         count_launch();
     }
-    // rblas runs the alpha step on an empty sum too, except for the real
-    // Trans loop, which has no step when m == 0 (src/level2.rs:41-60,
-    // src/complex2.rs:55-76)
-    const int alpha_mode = alpha_zero ? 0 : (have_work ? 1 : ((!CX && tr) ? 0 : 2));
-    if constexpr (CX)
-        gemv_finalize_cplx<T><<<blocks_for(len), kL2Threads, 0, st>>>(
-            reinterpret_cast<C2<T>*>(y), incy, len, reinterpret_cast<const C2<T>*>(ws), S, C2<T>{ar, ai},
-            C2<T>{br, bi}, alpha_mode);
-    else
-        gemv_finalize_real<T><<<blocks_for(len), kL2Threads, 0, st>>>(y, incy, len, ws, S, ar, br, alpha_mode);
-    count_launch();
     e = cudaGetLastError();
     if (ws) cudaFreeAsync(ws, st);
     return e == cudaSuccess ? RB_OK : fail(e, ce);
