@@ -276,6 +276,8 @@ constexpr size_t kTbSmemMax = 227 * 1024;
 //      Y_trailing -= L[trailing, b] * X_b. Both products read A and W as
 //      DMMA fragments straight from global memory (L2: each member's A is
 //      shared by its nrhs/RB CTAs) and Y from shared memory.
+//      trsm_dmma_wide_kernel (32-wide slices, left-looking) does the same for
+//      batches that fill the GPU.
 // Rounding differs from rblas's substitution (src/level3.rs:440-512: the
 // blocks' inverses replace the divisions inside each block); the result
 // stays within the normwise backward-error bound the tests state.
@@ -630,6 +632,244 @@ __global__ void __launch_bounds__(kTbThreads, 2)
     }
 }
 
+// 32 right-hand sides per CTA, left-looking, one CTA per SM. What bounds
+// trsm_dmma_kernel is its A fragments (16 bytes per lane for two DMMAs, from
+// L1 / L2; a left-looking form with one DMMA per fragment took 1581 us against
+// 1281 at 1024 members of 512 x 64): here a fragment meets four n-blocks.
+// Block row b takes Z = Y_b - L[b, 0:b] * X[0:b] with the sums in registers
+// over the whole K -- warp (xm, ks): 16 rows x 32 columns, half ks of each
+// 64-column tile -- and then X_b = W_b * Z, warp (xm, ks) the column half ks.
+// All warps have the same work in both, and Y is read and written once per
+// block. A half's fragments are requested while the DMMAs of the half before
+// it run, across the barriers too. 1024 x (512, 64): 1281 -> 1002 us (of which
+// the inversion 171); a CTA's 104K clocks: products 64K (57K at the pipe's
+// rate), Z 21K, X 7K, B in and out 12K.
+constexpr int kTwRB = 32, kTwYS = 36;
+
+__global__ void __launch_bounds__(kTbThreads, 1)
+    trsm_dmma_wide_kernel(const double* __restrict__ A0, double* __restrict__ B0, double alpha, TbParams p,
+                          const double* __restrict__ W, int nblocks) {
+    constexpr int YS = kTwYS, RB = kTwRB;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double* Y = reinterpret_cast<double*>(smem_raw);
+    double* Z = Y + static_cast<size_t>(p.q) * YS;  // 64 x 32
+    double* P = Z + kInvNB * YS;                    // partial sums, 64 x 32
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int g = lane >> 2, t = lane & 3;
+    // the two warps of a scheduler take row blocks s and 3 - s: W_b is lower
+    // triangular, so row block xm of the X step has 2 (xm + 1) k-steps
+    const int ks = warp >> 2, xm = ks ? 3 - (warp & 3) : warp & 3;
+    const int member = blockIdx.y;
+    const double* A = A0 + static_cast<size_t>(member) * p.stride_a;
+    double* B = B0 + static_cast<size_t>(member) * p.stride_b;
+    const double* Wm = W + static_cast<size_t>(member) * nblocks * (kInvNB * kInvNB);
+    const int c0 = blockIdx.x * RB;
+    const int ncols = min(RB, p.nrhs - c0);
+    const int nn = (ncols + 7) / 8;  // n-blocks in use
+    const int q = p.q;
+
+    // four k-steps from column k0 of rows r0.. of A (past q: zero), or of W_b
+    auto load_a = [&](int b, int kb, double (&f)[4][4]) {
+        const int ra = b * kInvNB + 16 * xm + 2 * g, rb = ra + 1, k0 = kb * kInvNB + 32 * ks + t;
+        if (p.vec_a && b * kInvNB + 16 * xm + 16 <= q) {
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) {
+                const double2 lo = __ldg(reinterpret_cast<const double2*>(a_ptr(A, p, ra, k0 + 8 * kk)));
+                const double2 hi = __ldg(reinterpret_cast<const double2*>(a_ptr(A, p, ra, k0 + 8 * kk + 4)));
+                f[kk][0] = lo.x;
+                f[kk][1] = lo.y;
+                f[kk][2] = hi.x;
+                f[kk][3] = hi.y;
+            }
+        } else {
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) {
+                const int k = k0 + 8 * kk;
+                f[kk][0] = (ra < q) ? __ldg(a_ptr(A, p, ra, k)) : 0.0;
+                f[kk][1] = (rb < q) ? __ldg(a_ptr(A, p, rb, k)) : 0.0;
+                f[kk][2] = (ra < q) ? __ldg(a_ptr(A, p, ra, k + 4)) : 0.0;
+                f[kk][3] = (rb < q) ? __ldg(a_ptr(A, p, rb, k + 4)) : 0.0;
+            }
+        }
+    };
+    auto load_w = [&](int b, int h, double (&f)[4][4]) {
+        const double* Wb = Wm + static_cast<size_t>(b) * (kInvNB * kInvNB) + 16 * xm + 2 * g;
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+            const int k = 8 * (4 * h + kk) + t;
+            const double2 lo = __ldg(reinterpret_cast<const double2*>(Wb + 64 * k));
+            const double2 hi = __ldg(reinterpret_cast<const double2*>(Wb + 64 * (k + 4)));
+            f[kk][0] = lo.x;
+            f[kk][1] = lo.y;
+            f[kk][2] = hi.x;
+            f[kk][3] = hi.y;
+        }
+    };
+    double fa[4][4], fb[4][4];  // the current half, the next one
+    load_w(0, 0, fa);
+
+    // Y = alpha * B slice (rows reversed when rev), one rounding per element
+    // as rblas's B := alpha*B (src/level3.rs:403-409), 16 loads in flight
+    const bool rows_fast = p.ldb_rs == 1;
+    constexpr int kYU = 16;
+    if (rows_fast) {
+        for (int i = tid; i < q; i += kTbThreads) {
+            double* Yr = Y + (p.rev ? q - 1 - i : i) * YS;
+            const double* Br = B + i + static_cast<size_t>(c0) * p.ldb_cs;
+#pragma unroll
+            for (int j0 = 0; j0 < RB; j0 += kYU) {
+                double v[kYU];
+#pragma unroll
+                for (int u = 0; u < kYU; ++u)
+                    v[u] = j0 + u < ncols ? Br[static_cast<size_t>(j0 + u) * p.ldb_cs] : 0.0;
+#pragma unroll
+                for (int u = 0; u < kYU; ++u) Yr[j0 + u] = alpha != 1.0 ? alpha * v[u] : v[u];
+            }
+        }
+    } else {
+        const int j = tid % RB;
+        for (int i0 = tid / RB; i0 < q; i0 += kTbThreads / RB * kYU) {
+            double v[kYU];
+#pragma unroll
+            for (int u = 0; u < kYU; ++u) {
+                const int i = i0 + u * (kTbThreads / RB);
+                v[u] = (i < q && j < ncols)
+                           ? B[static_cast<size_t>(i) * p.ldb_rs + static_cast<size_t>(c0 + j) * p.ldb_cs] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < kYU; ++u) {
+                const int i = i0 + u * (kTbThreads / RB);
+                if (i < q) Y[(p.rev ? q - 1 - i : i) * YS + j] = alpha != 1.0 ? alpha * v[u] : v[u];
+            }
+        }
+    }
+    __syncthreads();
+
+    for (int b = 0; b < nblocks; ++b) {
+        const int o = b * kInvNB, nb = min(kInvNB, q - o);
+        const int r = 16 * xm + 2 * g;  // this lane's rows r, r + 1 of the block
+        double c[4][4];
+#pragma unroll
+        for (int n = 0; n < 4; ++n) c[n][0] = c[n][1] = c[n][2] = c[n][3] = 0.0;
+        for (int kb = 0; kb < b; ++kb) {  // fa: this warp's half of tile (b, kb)
+            if (kb + 1 < b) load_a(b, kb + 1, fb);
+            else            load_w(b, 0, fb);
+            const double* Ys = Y + (kb * kInvNB + 32 * ks + t) * YS + g;
+            if (nn == 4) {
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+                    for (int n = 0; n < 4; ++n) {
+                        const double bf[2] = {Ys[8 * kk * YS + 8 * n], Ys[(8 * kk + 4) * YS + 8 * n]};
+                        dmma_16x8x8(c[n], fa[kk], bf);
+                    }
+            } else {
+#pragma unroll
+                for (int n = 0; n < 3; ++n)
+                    if (n < nn) {
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk) {
+                            const double bf[2] = {Ys[8 * kk * YS + 8 * n], Ys[(8 * kk + 4) * YS + 8 * n]};
+                            dmma_16x8x8(c[n], fa[kk], bf);
+                        }
+                    }
+            }
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) fa[kk][i] = fb[kk][i];
+        }
+        load_w(b, 1, fb);
+        // each warp hands the other half of K's sums over: the column half
+        // 1 - ks to P, and finishes Z's column half ks
+        if (b > 0) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int n = 2 * (1 - ks) + h;
+                double* Ps = P + r * YS + 8 * n + 2 * t;
+                Ps[0] = ks ? c[h][0] : c[2 + h][0];
+                Ps[1] = ks ? c[h][1] : c[2 + h][1];
+                Ps[YS] = ks ? c[h][2] : c[2 + h][2];
+                Ps[YS + 1] = ks ? c[h][3] : c[2 + h][3];
+            }
+            __syncthreads();
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {  // Z (rows past nb: zero, as W's columns there)
+            const int cc = 8 * (2 * ks + h) + 2 * t;
+            const double* Yb = Y + (o + r) * YS + cc;
+            const double* Ps = P + r * YS + cc;
+            double* Zb = Z + r * YS + cc;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                double s0 = ks ? c[2 + h][i] : c[h][i], s1 = ks ? c[2 + h][2 + i] : c[h][2 + i];
+                if (b > 0) {
+                    s0 += Ps[i];
+                    s1 += Ps[YS + i];
+                }
+                Zb[i] = r < nb ? Yb[i] - s0 : 0.0;
+                Zb[YS + i] = r + 1 < nb ? Yb[YS + i] - s1 : 0.0;
+            }
+        }
+        __syncthreads();
+        // X_b = W_b * Z: fa and fb are W_b's halves
+        double x[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
+        const double* Zs = Z + t * YS + 16 * ks + g;
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+            if (kk < 2 * (xm + 1)) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const double bf[2] = {Zs[8 * kk * YS + 8 * h], Zs[(8 * kk + 4) * YS + 8 * h]};
+                    dmma_16x8x8(x[h], fa[kk], bf);
+                }
+            }
+        if (b + 1 < nblocks) load_a(b + 1, 0, fa);
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+            if (4 + kk < 2 * (xm + 1)) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const double bf[2] = {Zs[(32 + 8 * kk) * YS + 8 * h], Zs[(36 + 8 * kk) * YS + 8 * h]};
+                    dmma_16x8x8(x[h], fb[kk], bf);
+                }
+            }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            double* Yb = Y + (o + r) * YS + 8 * (2 * ks + h) + 2 * t;
+            if (r < nb) {
+                Yb[0] = x[h][0];
+                Yb[1] = x[h][1];
+            }
+            if (r + 1 < nb) {
+                Yb[YS] = x[h][2];
+                Yb[YS + 1] = x[h][3];
+            }
+        }
+        __syncthreads();  // X_b is there; Z and P may be rewritten
+    }
+
+    if (rows_fast) {
+        for (int i = tid; i < q; i += kTbThreads) {
+            const double* Yr = Y + (p.rev ? q - 1 - i : i) * YS;
+            double* Br = B + i + static_cast<size_t>(c0) * p.ldb_cs;
+#pragma unroll 8
+            for (int j = 0; j < RB; ++j)
+                if (j < ncols) Br[static_cast<size_t>(j) * p.ldb_cs] = Yr[j];
+        }
+    } else {
+        const int j = tid % RB;
+        for (int i = tid / RB; i < q; i += kTbThreads / RB)
+            if (j < ncols)
+                B[static_cast<size_t>(i) * p.ldb_rs + static_cast<size_t>(c0 + j) * p.ldb_cs] =
+                    Y[(p.rev ? q - 1 - i : i) * YS + j];
+    }
+}
+
+size_t tw_smem(int q) {
+    return (static_cast<size_t>(q) + 2 * kInvNB) * kTwYS * sizeof(double);
+}
+
 template <int RB>
 size_t td_smem(int q) {
     return static_cast<size_t>(q) * TdCfg<RB>::YS * sizeof(double);
@@ -641,9 +881,12 @@ constexpr size_t kTdWorkspace = size_t(256) << 20;
 template <int RB>
 cudaError_t td_launch(const double* A, double* B, double alpha, const TbParams& p, size_t batch, cudaStream_t st,
                       bool* alloc_failed) {
-    const size_t smem = td_smem<RB>(p.q);
-    cudaError_t e = cudaFuncSetAttribute(trsm_dmma_kernel<RB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
+    const size_t smem = RB == kTwRB ? tw_smem(p.q) : td_smem<RB == kTwRB ? 16 : RB>(p.q);
+    auto kern = [] {
+        if constexpr (RB == kTwRB) return trsm_dmma_wide_kernel;
+        else                       return trsm_dmma_kernel<RB>;
+    }();
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(trsm_inv_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kInvSmem);
     if (e != cudaSuccess) return e;
@@ -665,7 +908,7 @@ cudaError_t td_launch(const double* A, double* B, double alpha, const TbParams& 
         double* Bc = B + b0 * p.stride_b;
         trsm_inv_diag_kernel<<<dim3(nblocks, static_cast<unsigned>(nm)), kInvThreads, kInvSmem, st>>>(Ac, p, W,
                                                                                               nblocks);
-        trsm_dmma_kernel<RB><<<dim3((p.nrhs + RB - 1) / RB, static_cast<unsigned>(nm)), kTbThreads, smem, st>>>(
+        kern<<<dim3((p.nrhs + RB - 1) / RB, static_cast<unsigned>(nm)), kTbThreads, smem, st>>>(
             Ac, Bc, alpha, p, W, nblocks);
         count_launch(2);
         e = cudaGetLastError();
@@ -731,11 +974,21 @@ int trsm_batched_dev(int side, int uplo, int trans, int diag, size_t m, size_t n
     int td_rb = 0;  // f64: slice width of the tensor-core path (0: not used)
     if constexpr (sizeof(T) == 8) {
         // 16-wide slices while two CTAs fit an SM, then 8-wide, then one CTA per SM
-        if (td_smem<16>(p.q) <= kTbSmemMax / 2) td_rb = 16;
+        // 32-wide ones where 16-wide ones would put a second CTA on some SM
+        // (one 16-wide CTA per SM finishes first: 512 x 512, us: 59 against
+        // 70; 512 x 4096 of a 1024 system: 274 against 227)
+        int dev = 0, sms = 148;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        const size_t slices16 = static_cast<size_t>((p.nrhs + 15) / 16) * batch;
+        if (p.nrhs > 16 && slices16 > static_cast<size_t>(sms) && tw_smem(p.q) <= kTbSmemMax) td_rb = 32;
+        else if (td_smem<16>(p.q) <= kTbSmemMax / 2) td_rb = 16;
         else if (td_smem<8>(p.q) <= kTbSmemMax / 2) td_rb = 8;
         else if (td_smem<16>(p.q) <= kTbSmemMax) td_rb = 16;
         else if (td_smem<8>(p.q) <= kTbSmemMax) td_rb = 8;
-        if (td_rb == 16) e = td_launch<16>(reinterpret_cast<const double*>(A), reinterpret_cast<double*>(B), alpha, p,
+        if (td_rb == 32) e = td_launch<32>(reinterpret_cast<const double*>(A), reinterpret_cast<double*>(B), alpha, p,
+                                           batch, st, &alloc_failed);
+        else if (td_rb == 16) e = td_launch<16>(reinterpret_cast<const double*>(A), reinterpret_cast<double*>(B), alpha, p,
                                            batch, st, &alloc_failed);
         else if (td_rb == 8) e = td_launch<8>(reinterpret_cast<const double*>(A), reinterpret_cast<double*>(B), alpha,
                                               p, batch, st, &alloc_failed);
