@@ -411,9 +411,11 @@ size_t grouped_ws_slots(const rb_gemm_problem& q) {
 
 size_t grouped_slot_bytes() { return kSlotBytes; }
 
-int grouped_splits(const rb_gemm_problem& q) {
+int grouped_splits(const rb_gemm_problem& q, int* k_per_split) {
     if (validate_problem(q) != RB_OK) return 0;
-    return plan_problem(q, tuned_snapshot().get()).splits;
+    const Plan pl = plan_problem(q, tuned_snapshot().get());
+    if (k_per_split) *k_per_split = pl.kt_per_split * (q.dtype == 1 ? SimtCfg<double>::BK : SimtCfg<float>::BK);
+    return pl.splits;
 }
 
 namespace {

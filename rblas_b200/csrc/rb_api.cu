@@ -322,10 +322,11 @@ struct ColProblem {
     bool split_ok = true;  // the plain form may take the grouped kernel's split-K
 };
 
-// The plain problem as one grouped-kernel entry; true when the grouped
-// kernel's shape rule splits its K (fewer C tiles than SMs and a long K).
+// The plain problem as one grouped-kernel entry; the factor by which the
+// grouped kernel's shape rule splits its K (more than 1 with fewer C tiles
+// than SMs and a long K), and the k of a range.
 template <typename T>
-bool plain_split(const ColProblem<T>& p, rb_gemm_problem* q) {
+int plain_splits(const ColProblem<T>& p, rb_gemm_problem* q, int* k_range) {
     *q = rb_gemm_problem{};
     q->dtype = sizeof(T) == 8 ? 1 : 0;
     q->layout = RB_COL_MAJOR;
@@ -338,8 +339,25 @@ bool plain_split(const ColProblem<T>& p, rb_gemm_problem* q) {
     q->b = p.b; q->ldb = p.ldb;
     q->c = p.c; q->ldc = p.ldc;
     // an f32 problem the narrow tile fills the GPU with runs unsplit
-    if (sizeof(T) == 4 && simt_narrow_f32(p.m, p.n)) return false;
-    return !p.tri && grouped_splits(*q) > 1;
+    *k_range = 0;
+    if (p.tri || (sizeof(T) == 4 && simt_narrow_f32(p.m, p.n))) return 1;
+    return std::max(1, grouped_splits(*q, k_range));
+}
+
+// The small tile a plain problem runs on (small_gemm_cfg), or 0; splits as
+// plain_splits.
+template <typename T>
+int plain_small(const ColProblem<T>& p, int splits) {
+    static std::atomic<int> sms{0};
+    int n = sms.load(std::memory_order_relaxed);
+    if (!n) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
+            return 0;
+        sms.store(n, std::memory_order_relaxed);
+    }
+    return small_gemm_cfg<T>(p.m, p.n, p.k, splits, n);
 }
 
 template <typename T>
@@ -413,11 +431,19 @@ rb_status run_dev(const ColProblem<T>& p, rb_precision prec, cudaStream_t st, rb
         }
         return run_precision_form(p, prec, st, err);
     }
-    // Fewer C tiles than SMs and a long K (the 1024^3 SGEMM: 64 tiles): the
-    // grouped kernel's deterministic split-K fills the GPU. The factor
-    // depends on the shape alone, so a call's bits repeat from call to call.
+    // Few C tiles of 128: small tiles, or with a long K the grouped kernel's
+    // deterministic split-K, fill the GPU. Either depends on the shape alone,
+    // and the small tiles sum K in the ranges that the other would split it
+    // into, so a call's bits repeat from call to call.
     rb_gemm_problem gq;
-    if (p.split_ok && plain_split(p, &gq)) {
+    int k_range = 0;
+    const int splits = p.split_ok ? plain_splits(p, &gq, &k_range) : 1;
+    if (const int cfg = p.split_ok ? plain_small(p, splits) : 0) {
+        e = launch_small_gemm<T>(cfg, p.ta, !p.tb, (int)p.m, (int)p.n, (int)p.k, p.alpha, p.a, p.lda, p.b, p.ldb,
+                                 p.beta, p.c, p.ldc, st, p.tri, splits > 1 ? k_range : 0);
+        return e == cudaSuccess ? RB_OK : cuda_fail(err, e);
+    }
+    if (splits > 1) {
         int32_t ce = 0;
         const int rc = grouped_gemm_dev(&gq, 1, nullptr, nullptr, st, &ce, nullptr);
         if (rc != RB_OK) set_err(err, rc, 0, 0, 0, ce);
@@ -542,12 +568,13 @@ rb_status host_gemm(rb_layout layout, rb_transpose transa, rb_transpose transb, 
     const size_t el = sizeof(T);
     const size_t total_bytes = (need_ab ? (a_rows * a_cols + b_rows * b_cols) * el : 0) +
                                p.m * p.n * el * (read_c ? 2 : 1);
-    // a plain call whose whole shape takes split-K runs whole (a panel's
-    // split could differ, and with it the summation order), and so does one
-    // whose C the narrow f32 tile spreads over the SMs (its panels would not)
+    // a plain call whose whole shape takes split-K runs whole (a panel's split
+    // could differ, and with it the summation order), and so does one whose C
+    // the narrow f32 tile spreads over the SMs (its panels would not)
     rb_gemm_problem whole;
-    const bool whole_call = prec == RB_PREC_PLAIN &&
-                            (plain_split(p, &whole) || (sizeof(T) == 4 && simt_narrow_f32(p.m, p.n)));
+    int whole_range = 0;
+    const bool whole_call = prec == RB_PREC_PLAIN && (plain_splits(p, &whole, &whole_range) > 1 ||
+                                                      (sizeof(T) == 4 && simt_narrow_f32(p.m, p.n)));
     if (total_bytes >= (size_t(64) << 20) && p.n >= 2 * 256 && !whole_call) {
         size_t lens[kHostPanels];
         const int np = panel_plan(p.n, lens);

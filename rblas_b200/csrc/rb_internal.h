@@ -116,6 +116,15 @@ cudaError_t launch_simt_gemm(bool a_kmajor, bool b_kmajor, int m, int n, int k, 
                              size_t ldc, cudaStream_t st, CUresult* cu_err, int tri = 0,
                              const T* Cin = nullptr, size_t ldcin = 0);
 bool simt_narrow_f32(size_t m, size_t n);
+// The plain GEMM on small tiles (gemm_small.cu); any alignment. small_gemm_cfg: the tile (1, 2) a shape runs on, 0: the
+// 128-wide tiles (with the grouped kernel's K split `splits`). k_range: where
+// the grouped kernel splits K, the k of its ranges (0: unsplit), whose sums
+// are then formed apart and added in order, as there.
+template <typename T>
+int small_gemm_cfg(size_t m, size_t n, size_t k, int splits, int sms);
+template <typename T>
+cudaError_t launch_small_gemm(int cfg, bool a_kmajor, bool b_kmajor, int m, int n, int k, T alpha, const T* A, size_t lda,
+                              const T* B, size_t ldb, T beta, T* C, size_t ldc, cudaStream_t st, int tri, int k_range);
 
 // C := beta*C over an m x n column-major block (beta == 0 writes zeros
 // without reading; beta == 1 is a no-op and launches nothing); tri as above.
@@ -196,7 +205,8 @@ size_t grouped_table_bytes(size_t count, size_t sems);
 // Split-K workspace slots (grouped_slot_bytes() each) one problem needs.
 size_t grouped_ws_slots(const rb_gemm_problem& q);
 size_t grouped_slot_bytes();
-int grouped_splits(const rb_gemm_problem& q);
+// The factor by which one problem's K is split (0: invalid), and the k of a range.
+int grouped_splits(const rb_gemm_problem& q, int* k_per_split = nullptr);
 // Split-K autotuning: bucket key of a (column-major) shape, the installed
 // table of tuned factors (nullptr: the built-in rule), and a per-thread
 // forced factor for timing candidates (0: off).

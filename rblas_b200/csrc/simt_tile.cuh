@@ -246,6 +246,8 @@ __device__ __forceinline__ void fma_f32x2(f32x2& c, f32x2 a, f32x2 b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
 }
 
+__device__ __forceinline__ void add_f32x2(f32x2& s, f32x2 v) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(s) : "l"(v)); }
+
 template <bool PACKED> struct PairAcc { using type = f32x2; };
 template <> struct PairAcc<false> { using type = float; };
 
