@@ -712,304 +712,362 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 
 // ------------------------------------------------------------------------------
 // The BF16-split forms with A split inside the GEMM (A rows contiguous:
-// NoTrans).
+// NoTrans), on CTA pairs: 256 x 128 tiles.
 //
 // Two passes read A, write its planes and read the planes again: about three
 // times A's bytes, which is most of the time of a tall-skinny product
-// (65536 x 128 x 8192: A is 2.1 GB, the GEMM itself ~0.3 ms of tensor work in
-// 3xBF16). Here TMA brings 128 x 64 f32 tiles of A (128 contiguous rows per K
-// column) into shared memory, and the epilogue warps split them, between
-// their accumulator promotions, into the planes (hi, lo for 3xBF16; hi, mid,
-// lo for BF16X6) in the 128-byte-swizzled K-major layout the UMMA
-// descriptors read: row r's 16-byte chunk c at r * 128 + ((c ^ (r & 7)) *
-// 16), the layout a TMA load of the planes produces. The split is the split
+// (65536 x 128 x 8192: A is 2.1 GB). Here TMA brings 128 x 64 f32 tiles of A
+// (128 contiguous rows per K column) into shared memory, and the epilogue
+// warps split them, between their accumulator promotions, into the planes
+// (hi, lo for 3xBF16; hi, mid, lo for BF16X6): for 3xBF16 into TMEM, as the
+// MMA's A operand (row = lane, two K values per column), beside the
+// accumulators' 256 columns; for BF16X6, whose accumulators fill TMEM, into the
+// 128-byte-swizzled K-major tiles that a TMA load of planes gives (row r's
+// 16-byte chunk c at r * 128 + ((c ^ (r & 7)) * 16)). The split is the split
 // pass's (hi = rn(x), then each next plane rn of what is left) and the
 // products, their order, the accumulators and the promotions are
 // umma_gemm_kernel<MODE>'s, so the results are the two-pass form's bit for
-// bit. B's planes come from the split pass (B is small). Rings: A's f32
-// tiles (released as soon as the splitters hold them in registers), A's
-// planes (released by the MMAs), B's planes. BF16X6's three-plane stages
-// leave room for one f32 stage only; its refill overlaps the conversion and
-// the wait for a free plane stage.
-// Warps: 0 TMA producer, 1 TMEM owner / MMA issuer, 2..9 splitter and
-// epilogue: tile row quarter * 32 + lane (quarter = warp % 4, the TMEM lane
-// quarter the warp may read) in both roles, and one half of the tile -- K
-// chunks 4h..4h+3 of each 64-column K tile to split, columns 64h..64h+63 to
-// promote and write -- for h = (warp - 2) / 4. Two such warps per scheduler
-// hide each other's latencies, and 64 running sums per thread leave
-// registers for the split.
+// bit. B's planes come from the split pass (B is small), half of a tile's
+// columns to each CTA.
+// Rings: A's f32 tiles (released as soon as the splitters hold them in
+// registers); stages of A's planes and B's planes, released together by the
+// MMAs' one commit.
+// Warps: 0 producer of A's tiles; 1 TMEM owner and, in the even CTA, MMA issuer
+// for both (the odd one's tells it of full stages); 2 producer of B's planes;
+// 3..18 splitter and epilogue: tile row quarter * 32 + lane (quarter = warp % 4,
+// the TMEM lanes the warp may use) in both roles; K values 32 half .. + 31 of
+// every second K tile to split (so that one tile's loads overlap the other's
+// stores), columns 32 part .. + 31 of the tile to promote and write.
+// Bound: A's bytes from memory. 65536 x 128 x 8192 back to back, 3xBF16: 430 us
+// (A at 5.1 TB/s, its four waves 86 % full), BF16X6 693 (24 MMAs of 64 clocks a
+// K tile); on single CTAs with planes in shared memory, one splitter group and
+// one issuing lane, 634 and 900: the issuing lane took ~110 clocks an MMA.
+// Splitting with 16 warps a tile instead of two groups of 8: 523 and 768. Tiles
+// of 112 rows, which fill the fourth wave, took longer (471): their columns
+// start inside 128-byte lines.
 // ------------------------------------------------------------------------------
 template <int MODE> struct FzCfg;
-template <> struct FzCfg<kModeBf16x3> { static constexpr int FS = 3, PS = 2, BS = 2; };
-template <> struct FzCfg<kModeBf16x6> { static constexpr int FS = 1, PS = 2, BS = 2; };
-constexpr int kFzMaxStages = 3;
-constexpr int kFzThreads = 320;
-constexpr int kFzEpiWarps = 8;
+template <> struct FzCfg<kModeBf16x3> { static constexpr int FS = 4, RS = 4; static constexpr bool A_TMEM = true; };
+template <> struct FzCfg<kModeBf16x6> { static constexpr int FS = 2, RS = 2; static constexpr bool A_TMEM = false; };
+constexpr int kFzEpiWarps = 16;
+constexpr int kFzThreads = 96 + 32 * kFzEpiWarps;
+constexpr int kFzN = 128;                 // tile columns
 constexpr int kFzF32Tile = kUM * 64 * 4;  // 64 K columns of 128 f32 rows: 32 KiB
+constexpr int kFzBTile = kFzN / 2 * kRowBytes;
+constexpr int kFzUnit = 2;  // K tiles to a promotion (kt_per_chunk): one per splitter group
 template <int MODE>
 constexpr int fz_smem_bytes() {
     using F = FzCfg<MODE>;
-    // f32 stages, then A's and B's plane stages (NA planes of one 128 x 64 tile each)
-    return F::FS * kFzF32Tile + (F::PS + F::BS) * UCfg<MODE>::NA * kATile + 256 + 1024;
+    return F::FS * kFzF32Tile + F::RS * UCfg<MODE>::NA * (kFzBTile + (F::A_TMEM ? 0 : kATile)) + 256 + 1024;
 }
 static_assert(fz_smem_bytes<kModeBf16x3>() <= 232448 && fz_smem_bytes<kModeBf16x6>() <= 232448,
               "the fused kernels' rings must fit one CTA's shared memory");
 
 struct FzBar {
-    uint64_t f_full[kFzMaxStages], f_empty[kFzMaxStages];
-    uint64_t a_full[kFzMaxStages], a_empty[kFzMaxStages];
-    uint64_t b_full[kFzMaxStages], b_empty[kFzMaxStages];
+    uint64_t f_full[4], f_empty[4];  // A's f32 tiles
+    uint64_t full[4];                // plane stages: A's split here and B's landed
+    uint64_t peer_full[4];           // (even CTA) the same of the odd one's
+    uint64_t empty[4];               // the pair's MMAs have read them
     uint64_t acc_full[2], acc_empty[2], drain;
     uint32_t tmem_base;
 };
 static_assert(sizeof(FzBar) <= 256, "the fused kernels reserve 256 bytes of shared memory for their barriers");
 
 template <int MODE>
-__global__ void __launch_bounds__(kFzThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFzThreads, 1)
     umma_split_fused_kernel(const __grid_constant__ CUtensorMap tmA32, const __grid_constant__ CUtensorMap tmB,
                             const __grid_constant__ UParams p) {
     using Cfg = UCfg<MODE>;
-    constexpr int UN = Cfg::UN, NP = Cfg::NA;
-    constexpr int FS = FzCfg<MODE>::FS, PS = FzCfg<MODE>::PS, BS = FzCfg<MODE>::BS;
-    static_assert(FS <= kFzMaxStages && PS <= kFzMaxStages && BS <= kFzMaxStages, "FzBar holds the rings");
-    static_assert(Cfg::NB == NP, "A and B have the same planes");
-    constexpr int PLANES = NP * kATile;  // one plane stage: NP planes of a 128 x 64 tile
+    constexpr int NP = Cfg::NA, FS = FzCfg<MODE>::FS, RS = FzCfg<MODE>::RS;
+    constexpr bool A_TMEM = FzCfg<MODE>::A_TMEM;
+    static_assert(FS <= 4 && RS <= 4 && Cfg::NB == NP, "FzBar holds the rings; A and B have the same planes");
+    // a slot's tiles then are all one splitter group's, whose waits on it see
+    // every phase (copies may land out of order)
+    static_assert(FS % 2 == 0 && RS % 2 == 0, "even rings");
     constexpr int KSTEPS = 4;
-    constexpr uint32_t IDESC = umma_idesc(1, 1, kUM, UN);  // f32 <- bf16
+    constexpr uint32_t IDESC = umma_idesc(1, 1, 256, kFzN);  // f32 <- bf16
     // BF16X6 keeps hi*hi in an accumulator of its own, as umma_body does
     constexpr bool SPLIT_ACC = (MODE == kModeBf16x6);
-    constexpr uint32_t ACC_COLS = SPLIT_ACC ? 2 * UN : UN;  // per accumulator buffer
-    constexpr uint32_t TMEM_COLS = 2 * ACC_COLS;
-    static_assert(TMEM_COLS <= 512, "two buffers must fit the SM's TMEM");
-    static_assert(UN * kRowBytes == kATile, "B plane tiles are as large as A's");
+    constexpr uint32_t ACC_COLS = SPLIT_ACC ? 2 * kFzN : kFzN;  // per accumulator buffer
+    constexpr uint32_t A_COL = 2 * ACC_COLS;                    // TMEM columns of A's planes, 32 each
+    static_assert(A_COL + (A_TMEM ? RS * NP * 32 : 0) <= 512, "accumulators and planes fit TMEM");
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    uint8_t* f32s = smem;                        // FS x 32 KiB, [k][row] f32
-    uint8_t* aps = f32s + FS * kFzF32Tile;       // PS x NP planes, swizzled K-major
-    uint8_t* bps = aps + PS * PLANES;            // BS x NP planes, by TMA
-    FzBar* bar = reinterpret_cast<FzBar*>(bps + BS * PLANES);
+    uint8_t* f32s = smem;                           // FS x 32 KiB, [k][row] f32
+    uint8_t* bps = f32s + FS * kFzF32Tile;          // RS x NP planes, by TMA
+    uint8_t* aps = bps + RS * NP * kFzBTile;        // RS x NP planes, swizzled K-major (BF16X6)
+    FzBar* bar = reinterpret_cast<FzBar*>(aps + (A_TMEM ? 0 : RS * NP * kATile));
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_rank();
     if (threadIdx.x == 0) {
         for (int s = 0; s < FS; ++s) {
             mbar_init(&bar->f_full[s], 1);
-            mbar_init(&bar->f_empty[s], kFzEpiWarps);
+            mbar_init(&bar->f_empty[s], kFzEpiWarps / 2);
         }
-        for (int s = 0; s < PS; ++s) {
-            mbar_init(&bar->a_full[s], kFzEpiWarps);
-            mbar_init(&bar->a_empty[s], 1);
-        }
-        for (int s = 0; s < BS; ++s) {
-            mbar_init(&bar->b_full[s], 1);
-            mbar_init(&bar->b_empty[s], 1);
+        for (int s = 0; s < RS; ++s) {
+            mbar_init(&bar->full[s], 1 + kFzEpiWarps / 2);
+            mbar_init(&bar->peer_full[s], 1);
+            mbar_init(&bar->empty[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&bar->acc_full[b], 1);
-            mbar_init(&bar->acc_empty[b], kFzEpiWarps);
+            mbar_init(&bar->acc_empty[b], 2 * kFzEpiWarps);
         }
         mbar_init(&bar->drain, 1);
         fence_barrier_init();
     }
-    if (warp == 1) {
-        tmem_alloc(&bar->tmem_base, TMEM_COLS);
-        tmem_relinquish();
-    }
+    if (warp == 1) tmem_alloc_pair(&bar->tmem_base, 512);
     tc_fence_before();
     __syncthreads();
+    cluster_sync();  // the other CTA's barriers are initialised too
     tc_fence_after();
     const uint32_t tmem_base = bar->tmem_base;
-    const int items = p.num_tiles;
+    const int items = p.num_tiles, first = blockIdx.x >> 1, step = gridDim.x >> 1;
     uint32_t* const err = p.err;
     bool ok = true;
 
     if (warp == 0 && lane == 0) {
         // ------------------------------ TMA producer ------------------------------
         prefetch_tmap(&tmA32);
-        prefetch_tmap(&tmB);
-        uint32_t nf = 0, nb = 0;  // f32 tiles and B plane tiles issued
-        for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
+        uint32_t it = 0, fs = 0, ph = 1;  // tiles issued, ring slot, the phase to wait for
+        for (int item = first; ok && item < items; item += step) {
             int tm, tn;
             raster_tile(item, p.tiles_m, p.tiles_n, tm, tn);
-            const int m0 = tm * kUM, n0 = tn * UN;
-            for (int kt = 0; kt < p.num_kt; ++kt) {
-                const int fs = nf % FS;
-                if (nf >= FS && !mbar_wait(&bar->f_empty[fs], ((nf / FS) - 1) & 1, err, 0x211)) {
+            const int m0 = tm * 256 + rank * 128;
+            for (int kt = 0; kt < p.num_kt; ++kt, ++it) {
+                if (!mbar_wait(&bar->f_empty[fs], ph, err, 0x211)) {  // (a fresh slot's wait passes)
                     ok = false;
                     break;
                 }
                 mbar_arrive_expect_tx(&bar->f_full[fs], kFzF32Tile);
                 tma_load_2d(f32s + fs * kFzF32Tile, &tmA32, &bar->f_full[fs], m0, kt * 64);
-                ++nf;
-                const int bs = nb % BS;
-                if (nb >= BS && !mbar_wait(&bar->b_empty[bs], ((nb / BS) - 1) & 1, err, 0x212)) {
-                    ok = false;
-                    break;
+                if (++fs == FS) {
+                    fs = 0;
+                    ph ^= 1;
                 }
-                mbar_arrive_expect_tx(&bar->b_full[bs], PLANES);
-#pragma unroll
-                for (int q = 0; q < NP; ++q)
-                    tma_load_3d(bps + bs * PLANES + q * kATile, &tmB, &bar->b_full[bs], kt * 64, n0, q);
-                ++nb;
             }
         }
         if (!ok) {  // this CTA's copies land before it exits
-            for (uint32_t j = nf > (uint32_t)FS ? nf - FS : 0; j < nf; ++j)
+            for (uint32_t j = it > (uint32_t)FS ? it - FS : 0; j < it; ++j)
                 mbar_wait_drain(&bar->f_full[j % FS], (j / FS) & 1);
-            for (uint32_t j = nb > (uint32_t)BS ? nb - BS : 0; j < nb; ++j)
-                mbar_wait_drain(&bar->b_full[j % BS], (j / BS) & 1);
         }
-    } else if (warp == 1 && lane == 0) {
-        // ------------------------------ MMA issuer ------------------------------
-        uint32_t it = 0, uc = 0;
-        for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
-            for (int u = 0; ok && u < p.kchunks; ++u, ++uc) {
-                const int kt0 = u * p.kt_per_chunk, kt1 = min(p.num_kt, kt0 + p.kt_per_chunk);
-                const uint32_t b = uc & 1;
-                if (uc >= 2 && !mbar_wait(&bar->acc_empty[b], ((uc >> 1) - 1) & 1, err, 0x213)) {
+    } else if (warp == 2 && lane == 0) {
+        prefetch_tmap(&tmB);
+        uint32_t it = 0, rs = 0, ph = 1;
+        for (int item = first; ok && item < items; item += step) {
+            int tm, tn;
+            raster_tile(item, p.tiles_m, p.tiles_n, tm, tn);
+            const int n0 = tn * kFzN + rank * (kFzN / 2);
+            for (int kt = 0; kt < p.num_kt; ++kt, ++it) {
+                if (!mbar_wait_cluster(&bar->empty[rs], ph, err, 0x212)) {
                     ok = false;
                     break;
                 }
-                tc_fence_after();
-                const uint32_t d_tmem = tmem_base + b * ACC_COLS;        // the products (all, or all but hi*hi)
-                const uint32_t d_big = SPLIT_ACC ? d_tmem + UN : d_tmem;  // hi*hi
-                uint32_t accumulate = 0;
-                for (int kt = kt0; kt < kt1; ++kt, ++it) {
-                    const int ps = it % PS, bs = it % BS;
-                    if (!mbar_wait(&bar->a_full[ps], (it / PS) & 1, err, 0x214) ||
-                        !mbar_wait(&bar->b_full[bs], (it / BS) & 1, err, 0x215)) {
+                mbar_arrive_expect_tx(&bar->full[rs], NP * kFzBTile);
+#pragma unroll
+                for (int q = 0; q < NP; ++q)
+                    tma_load_3d(bps + (rs * NP + q) * kFzBTile, &tmB, &bar->full[rs], kt * 64, n0, q);
+                if (++rs == RS) {
+                    rs = 0;
+                    ph ^= 1;
+                }
+            }
+        }
+        // this CTA's copies land before it exits (a stage whose split of A does
+        // not come ends the wait by its time limit)
+        if (!ok) {
+            for (uint32_t j = it > (uint32_t)RS ? it - RS : 0; j < it; ++j)
+                if (!mbar_wait_drain(&bar->full[j % RS], (j / RS) & 1)) break;
+        }
+    } else if (warp == 1) {
+        // ---------- odd CTA: full stages, told to the even one; even CTA: MMA issuer ----------
+        // (the whole warp runs the loop, one lane issues: see elect_one)
+        const bool lead = elect_one();
+        const uint64_t d0 = sw128_kmajor_desc(smem_u32(bps));  // (see umma_pair_kernel on descriptors)
+        const uint32_t b_lo = static_cast<uint32_t>(d0), a_lo = b_lo + RS * NP * kFzBTile / 16;
+        const uint64_t d_hi = d0 & 0xffffffff00000000ull;
+        uint32_t uc = 0, rs = 0, ph = 0;  // ring slot and its phase
+        for (int item = first; ok && item < items; item += step) {
+            for (int u = 0; ok && u < p.kchunks; ++u, ++uc) {
+                const int kt0 = u * kFzUnit, kt1 = min(p.num_kt, kt0 + kFzUnit);
+                const uint32_t b = uc & 1;
+                if (rank == 0) {
+                    if (uc >= 2) ok = mbar_wait_cluster(&bar->acc_empty[b], ((uc >> 1) - 1) & 1, err, 0x213);
+                    if (!__all_sync(0xffffffffu, ok)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t sa = smem_u32(aps + ps * PLANES);
-                    const uint32_t sb = smem_u32(bps + bs * PLANES);
-#pragma unroll
-                    for (int kk = 0; kk < KSTEPS; ++kk) {
-#pragma unroll
-                        for (int q = 0; q < Cfg::NPROD; ++q) {
-                            const bool big = SPLIT_ACC && q == Cfg::NPROD - 1;
-                            umma_f16(big ? d_big : d_tmem, sw128_kmajor_desc(sa + Cfg::pa(q) * kATile) + 2 * kk,
-                                     sw128_kmajor_desc(sb + Cfg::pb(q) * kATile) + 2 * kk, IDESC,
-                                     (q == 0 || big) ? accumulate : 1u);
-                        }
-                        accumulate = 1;
-                    }
-                    tc_commit(&bar->a_empty[ps]);  // plane stages free once these MMAs complete
-                    tc_commit(&bar->b_empty[bs]);
                 }
-                if (ok) tc_commit(&bar->acc_full[b]);
+                const uint32_t d_tmem = tmem_base + b * ACC_COLS;         // the products (all, or all but hi*hi)
+                const uint32_t d_big = SPLIT_ACC ? d_tmem + kFzN : d_tmem;  // hi*hi
+                for (int kt = kt0; kt < kt1; ++kt) {
+                    ok = mbar_wait_inline(&bar->full[rs], ph, err, 0x214);
+                    if (rank == 0 && ok) ok = mbar_wait_cluster(&bar->peer_full[rs], ph, err, 0x215);
+                    if (!__all_sync(0xffffffffu, ok)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    if (rank != 0) {
+                        tc_fence_before();
+                        if (lead) mbar_arrive_rank_relaxed(&bar->peer_full[rs], 0);
+                    } else {
+                        const uint32_t sb = b_lo + rs * (NP * kFzBTile / 16), sa = a_lo + rs * (NP * kATile / 16);
+                        const uint32_t ta = tmem_base + A_COL + rs * (NP * 32);
+#pragma unroll
+                        for (int kk = 0; kk < KSTEPS; ++kk)
+#pragma unroll
+                            for (int q = 0; q < Cfg::NPROD; ++q) {
+                                const bool big = SPLIT_ACC && q == Cfg::NPROD - 1;
+                                const uint32_t d = big ? d_big : d_tmem;
+                                const uint32_t acc = (kk == 0 && (q == 0 || big)) ? (kt != kt0) : 1u;
+                                const uint64_t db = d_hi | (sb + Cfg::pb(q) * (kFzBTile / 16) + 2 * kk);
+                                if constexpr (A_TMEM) {
+                                    if (lead) umma_f16_pair_ts(d, ta + Cfg::pa(q) * 32 + kk * 8, db, IDESC, acc);
+                                } else {
+                                    if (lead)
+                                        umma_f16_pair(d, d_hi | (sa + Cfg::pa(q) * (kATile / 16) + 2 * kk), db, IDESC, acc);
+                                }
+                            }
+                        if (lead) tc_commit_pair(&bar->empty[rs]);  // free, in both CTAs, once these MMAs complete
+                    }
+                    if (++rs == RS) {
+                        rs = 0;
+                        ph ^= 1;
+                    }
+                }
+                if (ok && rank == 0 && lead) tc_commit_pair(&bar->acc_full[b]);
             }
         }
-        tc_commit(&bar->drain);
-        mbar_wait_drain(&bar->drain, 0);
-    } else if (warp >= 2) {
+        // nothing of ours is in flight before TMEM is released (arrives on the
+        // odd CTA's copy too, which nobody waits on)
+        if (rank == 0) {
+            if (lead) tc_commit_pair(&bar->drain);
+            mbar_wait_drain(&bar->drain, 0);
+        }
+    } else if (warp >= 3) {
         // ------------------------- splitter and epilogue -------------------------
-        constexpr int HC = UN / 2;  // columns per warp
-        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        constexpr int HC = kFzN / 4;  // columns per warp
+        const int quarter = warp & 3, part = (warp - 3) >> 2, half = part >> 1;
         const int row = quarter * 32 + lane;  // tile row: TMEM lane and split row
-        uint32_t it = 0, uc = 0;
-        for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
+        const uint32_t tlane = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+        uint32_t uc = 0, it = 0;  // units promoted, K tiles before this item
+        for (int item = first; ok && item < items; item += step) {
             int tm, tn;
             raster_tile(item, p.tiles_m, p.tiles_n, tm, tn);
-            const int m0 = tm * kUM, n0 = tn * UN + half * HC;
-            const int r = m0 + row;
-            const bool row_ok = r < p.m;
-            float sum[HC];
+            const int n0 = tn * kFzN + part * HC;
+            const int r = tm * 256 + static_cast<int>(rank) * 128 + row;
+            f32pair sum[HC / 2];
 #pragma unroll
-            for (int j = 0; j < HC; ++j) sum[j] = 0.f;
+            for (int j = 0; j < HC / 2; ++j) sum[j] = 0ull;
             int promoted = 0;
             // add unit `promoted`'s FP32 partial (TMEM) into sum, as umma_body does
             auto promote = [&]() -> bool {
                 const uint32_t b = uc & 1;
-                if (!mbar_wait(&bar->acc_full[b], (uc >> 1) & 1, err, 0x216)) return false;
+                const bool got = mbar_wait_inline(&bar->acc_full[b], (uc >> 1) & 1, err, 0x216);
+                if (!__all_sync(0xffffffffu, got)) return false;
                 tc_fence_after();
-                const uint32_t taddr =
-                    tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + b * ACC_COLS + half * HC;
                 // the smaller products first, then hi*hi (SPLIT_ACC)
 #pragma unroll
-                for (int part = 0; part < (SPLIT_ACC ? 2 : 1); ++part) {
+                for (int ch = 0; ch < (SPLIT_ACC ? 2 : 1); ++ch) {
+                    uint32_t v[HC];
+                    tmem_ld32(tlane + b * ACC_COLS + ch * kFzN + part * HC, v);
+                    tmem_ld_wait();
 #pragma unroll
-                    for (int ch = 0; ch < HC / 32; ++ch) {
-                        uint32_t v[32];
-                        tmem_ld32(taddr + part * UN + ch * 32, v);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) sum[ch * 32 + j] += __uint_as_float(v[j]);
-                    }
+                    for (int j = 0; j < HC / 2; ++j) add_f32pair(sum[j], v[2 * j], v[2 * j + 1]);
                 }
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&bar->acc_empty[b]);
+                if (lane == 0) mbar_arrive_rank_relaxed(&bar->acc_empty[b], 0);
                 ++uc;
                 ++promoted;
                 return true;
             };
-            for (int kt = 0; kt < p.num_kt; ++kt, ++it) {
-                const int fs = it % FS, ps = it % PS;
-                if (!mbar_wait(&bar->f_full[fs], (it / FS) & 1, err, 0x218)) {
+            // this group's K tiles: every second one over all items
+            for (int kt = (it ^ part) & 1; kt < p.num_kt; kt += 2) {
+                const uint32_t i = it + kt, fs = i % FS, rs = i % RS;
+                bool got = mbar_wait_inline(&bar->f_full[fs], (i / FS) & 1, err, 0x218);
+                if (!__all_sync(0xffffffffu, got)) {
                     ok = false;
                     break;
                 }
-                // this warp's half of the row's 64 K values, split into NP
-                // planes of packed bf16 pairs: pl[q][c4][j] holds plane q of K
-                // values 8 c4 + 2 j (low half) and 8 c4 + 2 j + 1 (high half)
-                uint32_t pl[NP][4][4];
+                // this warp's half of the row's 64 K values
+                float v[32];
                 {
-                    const float* F = reinterpret_cast<const float*>(f32s + fs * kFzF32Tile);  // F[k * 128 + row]
-                    float v[32];
+                    // F[k * 128 + row]
+                    const float* F = reinterpret_cast<const float*>(f32s + fs * kFzF32Tile) + half * 32 * kUM + row;
 #pragma unroll
-                    for (int e = 0; e < 32; ++e) v[e] = F[(half * 32 + e) * kUM + row];
-#pragma unroll
-                    for (int c4 = 0; c4 < 4; ++c4)
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            float v0 = v[c4 * 8 + 2 * j], v1 = v[c4 * 8 + 2 * j + 1];
-#pragma unroll
-                            for (int q = 0; q < NP; ++q) {
-                                const __nv_bfloat162 hb = __floats2bfloat162_rn(v0, v1);  // rn(v0) low, rn(v1) high
-                                pl[q][c4][j] = *reinterpret_cast<const uint32_t*>(&hb);
-                                if (q + 1 < NP) {
-                                    v0 -= __low2float(hb);
-                                    v1 -= __high2float(hb);
-                                }
-                            }
-                        }
+                    for (int e = 0; e < 32; ++e) v[e] = F[e * kUM];
                 }
-                // the f32 stage is free once every lane's reads have been used
-                __threadfence_block();
+                // the f32 stage is free: every lane's reads are done
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&bar->f_empty[fs]);
-                if (it >= PS && !mbar_wait(&bar->a_empty[ps], ((it / PS) - 1) & 1, err, 0x217)) {
+                got = mbar_wait_inline(&bar->empty[rs], (i / RS + 1) & 1, err, 0x217);  // (a fresh slot's wait passes)
+                if (!__all_sync(0xffffffffu, got)) {
                     ok = false;
                     break;
                 }
-                uint8_t* dst = aps + ps * PLANES;
+                if constexpr (A_TMEM) tc_fence_after();
+                uint8_t* const dst = aps + rs * NP * kATile + row * kRowBytes;
+                // split 8 (16) values at a time into NP planes of packed
+                // bf16 pairs: pl[q][j] holds plane q of K values 2 j (low
+                // half) and 2 j + 1 (high half)
+                constexpr int G = A_TMEM ? 16 : 8;
 #pragma unroll
-                for (int c4 = 0; c4 < 4; ++c4) {
-                    const int c = half * 4 + c4;
-                    const uint32_t off = static_cast<uint32_t>(row) * kRowBytes + ((c ^ (row & 7)) << 4);
+                for (int g = 0; g < 32 / G; ++g) {
+                    uint32_t pl[NP][G / 2];
 #pragma unroll
-                    for (int q = 0; q < NP; ++q)
-                        *reinterpret_cast<uint4*>(dst + q * kATile + off) =
-                            make_uint4(pl[q][c4][0], pl[q][c4][1], pl[q][c4][2], pl[q][c4][3]);
-                }
-                fence_proxy_async_smem();  // the planes' generic stores, visible to the tensor cores
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bar->a_full[ps]);
-                // once unit u's last tile is split, unit u - 1 is promoted: the
-                // MMAs of unit u + 1 wait for that buffer, and the split of
-                // unit u + 1's tiles waits for unit u's MMAs
-                if ((kt + 1) % p.kt_per_chunk == 0 || kt + 1 == p.num_kt) {
-                    if (kt / p.kt_per_chunk >= 1 && !promote()) {
-                        ok = false;
-                        break;
+                    for (int j = 0; j < G / 2; ++j) {
+                        float v0 = v[g * G + 2 * j], v1 = v[g * G + 2 * j + 1];
+#pragma unroll
+                        for (int q = 0; q < NP; ++q) {
+                            asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(pl[q][j]) : "f"(v1), "f"(v0));
+                            if (q + 1 < NP)
+                                asm("{\n\t.reg .b64 v, b, n;\n\t"
+                                    "mov.b64 v, {%0, %1};\n\t"
+                                    "mov.b64 b, {%2, %3};\n\t"
+                                    "mov.b64 n, 0xbf800000bf800000;\n\t"  // -1, -1
+                                    "fma.rn.f32x2 v, b, n, v;\n\t"
+                                    "mov.b64 {%0, %1}, v;\n\t}"
+                                    : "+f"(v0), "+f"(v1)
+                                    : "r"(pl[q][j] << 16), "r"(pl[q][j] & 0xffff0000u));
+                        }
+                    }
+                    if constexpr (A_TMEM) {
+#pragma unroll
+                        for (int q = 0; q < NP; ++q)
+                            tmem_st8(tlane + A_COL + (rs * NP + q) * 32 + half * 16 + g * 8, pl[q]);
+                    } else {
+                        const uint32_t off = ((half * 4 + g) ^ (row & 7)) << 4;
+#pragma unroll
+                        for (int q = 0; q < NP; ++q)
+                            *reinterpret_cast<uint4*>(dst + q * kATile + off) =
+                                make_uint4(pl[q][0], pl[q][1], pl[q][2], pl[q][3]);
                     }
                 }
+                if constexpr (A_TMEM) {
+                    tmem_st_wait();
+                    tc_fence_before();
+                } else {
+                    fence_proxy_async_smem();  // the planes' generic stores, visible to the tensor cores
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bar->full[rs]);
+                // once this group's part of unit u is split, unit u - 1 is promoted:
+                // the MMAs of unit u + 1 wait for that buffer
+                if (kt >= kFzUnit && !promote()) {
+                    ok = false;
+                    break;
+                }
             }
+            it += p.num_kt;
             while (ok && promoted < p.kchunks)
                 if (!promote()) ok = false;
-            if (ok && row_ok) {
+            if (ok && r < p.m) {
+                // C0 read 16 values at a time, all requested before use
 #pragma unroll
                 for (int g = 0; g < HC / 16; ++g) {
                     float cv[16];
@@ -1022,8 +1080,10 @@ __global__ void __launch_bounds__(kFzThreads, 1)
                     for (int jj = 0; jj < 16; ++jj) {
                         const int col = n0 + g * 16 + jj;
                         if (col < p.n) {
+                            float lo, hi;
+                            asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(sum[g * 8 + jj / 2]));
                             const float tb = (p.beta_mode == 2) ? p.beta_f * cv[jj] : cv[jj];
-                            p.c[r + static_cast<size_t>(col) * p.ldc] = fmaf(p.alpha_f, sum[g * 16 + jj], tb);
+                            p.c[r + static_cast<size_t>(col) * p.ldc] = fmaf(p.alpha_f, (jj & 1) ? hi : lo, tb);
                         }
                     }
                 }
@@ -1033,9 +1093,10 @@ __global__ void __launch_bounds__(kFzThreads, 1)
 
     tc_fence_before();
     __syncthreads();
+    cluster_sync();  // no CTA leaves while the other may still reach its memory
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, TMEM_COLS);
+        tmem_dealloc_pair(tmem_base, 512);
     }
 }
 
@@ -2656,7 +2717,8 @@ bool bf16_pair_tiles(int planes, int m, int n, int sms) {
 }
 
 template <int MODE>
-cudaError_t launch_bf16_fused(const CUtensorMap& ta32, const CUtensorMap& tb, const UParams& p, cudaStream_t st) {
+cudaError_t launch_bf16_fused(const CUtensorMap& ta32, const CUtensorMap& tb, const UParams& p, int sms,
+                              cudaStream_t st) {
     auto kern = umma_split_fused_kernel<MODE>;
     constexpr int smem = fz_smem_bytes<MODE>();
     static bool attr = false;
@@ -2665,10 +2727,7 @@ cudaError_t launch_bf16_fused(const CUtensorMap& ta32, const CUtensorMap& tb, co
         if (e != cudaSuccess) return e;
         attr = true;
     }
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int grid = p.num_tiles < sms ? p.num_tiles : sms;
+    const int grid = 2 * std::min(p.num_tiles, sms / 2);
     const char* name = (MODE == kModeBf16x3) ? "umma_bf16x3" : "umma_bf16x6";
     KernelTimer tm;
     kernel_timing_begin(name, 2.0 * p.m * p.n * static_cast<double>(p.k) * UCfg<MODE>::NPROD, st, &tm);
@@ -2686,7 +2745,7 @@ cudaError_t launch_bf16_split_gemm(int planes, bool ta, bool tb, int m, int n, i
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const bool fused = bf16_fused_a(ta, n, A, lda);
     const bool pair = !fused && bf16_pair_tiles(planes, m, n, sms);
-    const int UM = pair ? 256 : kUM, UN = pair ? kPairN : 128;
+    const int UM = pair || fused ? 256 : kUM, UN = pair ? kPairN : 128;
     const size_t kp = round_up(static_cast<size_t>(k), 8);  // 16-byte rows of bf16
     const size_t pa = fused ? 0 : static_cast<size_t>(m) * kp, pb = static_cast<size_t>(n) * kp;
     void* buf = nullptr;
@@ -2712,7 +2771,8 @@ cudaError_t launch_bf16_split_gemm(int planes, bool ta, bool tb, int m, int n, i
     CUresult r = fused ? make_tmap_2d(&tma, A, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, sizeof(float), m, k, lda, kUM, 64,
                                       false)
                        : make_tmap_planes(&tma, sa, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, k, m, planes, kp, 128, rb);
-    if (r == CUDA_SUCCESS) r = make_tmap_planes(&tmb, sb, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, k, n, planes, kp, 128, rb);
+    if (r == CUDA_SUCCESS)
+        r = make_tmap_planes(&tmb, sb, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, k, n, planes, kp, fused ? kFzN / 2 : 128, rb);
     if (r != CUDA_SUCCESS) {
         if (cu_err) *cu_err = r;
         cudaFreeAsync(buf, st);
@@ -2735,8 +2795,8 @@ cudaError_t launch_bf16_split_gemm(int planes, bool ta, bool tb, int m, int n, i
         e = (planes == 2) ? launch_umma_pair<kModeBf16x3>(tma, tmb, p, sms, st)
                           : launch_umma_pair<kModeBf16x6>(tma, tmb, p, sms, st);
     else if (fused)
-        e = (planes == 2) ? launch_bf16_fused<kModeBf16x3>(tma, tmb, p, st)
-                          : launch_bf16_fused<kModeBf16x6>(tma, tmb, p, st);
+        e = (planes == 2) ? launch_bf16_fused<kModeBf16x3>(tma, tmb, p, sms, st)
+                          : launch_bf16_fused<kModeBf16x6>(tma, tmb, p, sms, st);
     else
         e = (planes == 2) ? launch_umma<kModeBf16x3>(tma, tmb, p, st) : launch_umma<kModeBf16x6>(tma, tmb, p, st);
     cudaFreeAsync(buf, st);

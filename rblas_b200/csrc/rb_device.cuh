@@ -95,6 +95,22 @@ static __device__ __noinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, ui
     }
 }
 
+// The same, inline: around a call a caller saves the registers it keeps.
+static __device__ __forceinline__ bool mbar_wait_inline(uint64_t* bar, uint32_t parity, uint32_t* err, uint32_t site) {
+    if (mbar_try_wait(bar, parity)) return true;
+    const uint64_t t0 = globaltimer();
+    for (uint32_t it = 1;; ++it) {
+        if (mbar_try_wait(bar, parity)) return true;
+        if ((it & 31u) == 0u) {
+            if (dev_aborted(err)) return false;
+            if (globaltimer() - t0 > RB_WAIT_LIMIT_NS) {
+                dev_raise(err, RB_DEVERR_TIMEOUT | site);
+                return false;
+            }
+        }
+    }
+}
+
 // Wait used only on the error path to let this CTA's own copies land before
 // it exits: ignores the abort flag, bounded by time alone.
 static __device__ __noinline__ bool mbar_wait_drain(uint64_t* bar, uint32_t parity) {
@@ -271,6 +287,17 @@ __device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t adesc, u
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// The same with A in TMEM (row = lane, K values 2 j and 2 j + 1 in column j):
+// each CTA's own rows, at the same columns in both.
+__device__ __forceinline__ void umma_f16_pair_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
+                                                 uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
 __device__ __forceinline__ void umma_i8_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                              uint32_t accumulate) {
     asm volatile(
@@ -372,6 +399,13 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"(taddr));
 }
+// One register per column, 8 columns of the warp's 32 lanes, into TMEM.
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]),
+                 "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld_wait() {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
