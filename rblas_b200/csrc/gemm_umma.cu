@@ -1634,7 +1634,7 @@ __global__ void __launch_bounds__(kOzThreads, 1)
 // CTA's time at K = 2048), and its operands take 52 bytes per SM and clock of
 // MMA from L2. Here a unit is four diagonals {4g .. 4g+3}, whose accumulators
 // (4 x 128 columns) fill TMEM, so a tile has half as many units; each
-// epilogue thread keeps its 64 outputs of the tile in FP64 registers from the
+// epilogue thread keeps its outputs of the tile in FP64 registers from the
 // first unit (beta * C0, loaded while the tensor cores run) to the last, so C
 // is read and written once and a drain touches TMEM only. Stage st of a K
 // tile brings A_{top-st} and B_st; A_{top-st} is multiplied by the B tiles of
@@ -1649,21 +1649,25 @@ __global__ void __launch_bounds__(kOzThreads, 1)
 // part of K each, which write the exact sums S_d0 * 256 + S_d1 to workspace
 // planes; ozaki_pair_reduce_kernel adds the parts (exactly) and folds.
 // Warps per CTA: 0 TMA producer, 1 TMEM owner and MMA issuer (even CTA; odd:
-// passes on that a stage landed), 2..9 epilogue (two per TMEM lane quarter,
-// 64 columns each).
+// passes on that a stage landed), 2.. epilogue (two or four per TMEM lane
+// quarter).
 // ------------------------------------------------------------------------------
 constexpr int kPzN = 128;
-constexpr int kPzEpiWarps = 8;
-constexpr int kPzThreads = 64 + 32 * kPzEpiWarps;
+// Epilogue warps EW: 8 (64 columns each) for one problem, 16 (32 columns) in
+// the grouped kernel. At large sizes the power cap holds both, and 8 warps run
+// fewer instructions (8192^3: 12.1 against 12.5 ms); the grouped sets end in few
+// tiles, whose drains' latency 16 warps halve (eleven f64 requests of 32 .. 4096
+// a side: 1587 -> 1421 us; seven: 875 -> 865).
+constexpr int kPzEpiWarps = 8, kPzGroupEpiWarps = 16;
+constexpr int pz_threads(int ew) { return 64 + 32 * ew; }
 // Ring depths: a B tile is used for up to three stages after its own, so with
 // three more B slots than A slots both rings' next slots are free once the
 // stage kPzAS back is done, and one barrier per stage serves both.
 constexpr int kPzAS = 8, kPzBS = kPzAS + 3;
 constexpr int kPzBTile = 64 * kRowBytes;           // this CTA's half of a B tile
-constexpr int kPzCols = kPzN / 2;                  // columns per epilogue warp
-constexpr int kPzTab = kPzCols * (8 + 4);          // per epilogue warp: 2^fc and fc
+constexpr int kPzTabs = 4 * kPzN * 2 * 4;          // the epilogue warps' tables: fc << 20 and fc of their columns
 constexpr int kPzTileElems = 256 * kPzN;
-constexpr int kPzSmem = kPzAS * kATile + kPzBS * kPzBTile + 512 + kPzEpiWarps * kPzTab + 1024;
+constexpr int kPzSmem = kPzAS * kATile + kPzBS * kPzBTile + 512 + kPzTabs + 1024;
 static_assert(kPzSmem <= 232448, "the pair kernel's rings must fit one CTA's shared memory");
 
 struct PzBar {
@@ -1769,8 +1773,10 @@ __device__ __noinline__ double pz_term(double sv, int er, int fc, int wexp) {
     return (er != kExpSentinel && fc != kExpSentinel) ? scale_pow2(sv, er + fc - wexp) : 0.0;
 }
 
-template <class Src>
+template <int EW, class Src>
 __device__ __forceinline__ void ozaki_pair_body(const Src& src) {
+    constexpr int COLS = kPzN / (EW / 4);  // columns per epilogue warp
+    static_assert(COLS % 32 == 0, "a warp fills its table 32 columns at a time");
     constexpr int AS = kPzAS, BS = kPzBS;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -1785,7 +1791,7 @@ __device__ __forceinline__ void ozaki_pair_body(const Src& src) {
             mbar_init(&bar->peer_full[i], 1);
         }
         mbar_init(&bar->acc_full, 1);
-        mbar_init(&bar->acc_empty, 2 * kPzEpiWarps);
+        mbar_init(&bar->acc_empty, 2 * EW);
         mbar_init(&bar->drain, 1);
         fence_barrier_init();
     }
@@ -1918,12 +1924,12 @@ __device__ __forceinline__ void ozaki_pair_body(const Src& src) {
         }
     } else if (warp >= 2) {
         // ------------------------------ epilogue ------------------------------
-        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        const int quarter = warp & 3, part = (warp - 2) >> 2;
         const int row_in_pair = static_cast<int>(rank) * 128 + quarter * 32 + lane;
-        uint8_t* tab = reinterpret_cast<uint8_t*>(bar) + 512 + (warp - 2) * kPzTab;
-        double* col_scale = reinterpret_cast<double*>(tab);
-        int* col_e = reinterpret_cast<int*>(tab + kPzCols * sizeof(double));
-        const uint32_t tbase = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * kPzCols;
+        uint8_t* tab = reinterpret_cast<uint8_t*>(bar) + 512 + (warp - 2) * (kPzTabs / EW);
+        int* col_hi = reinterpret_cast<int*>(tab);  // what 2^fc adds to a double's high word
+        int* col_e = col_hi + COLS;
+        const uint32_t tbase = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + part * COLS;
         uint32_t uc = 0;
         for (int item = first; ok && item < items; item += step) {
             const PzWork w = src.get(item);
@@ -1931,7 +1937,7 @@ __device__ __forceinline__ void ozaki_pair_body(const Src& src) {
             const int groups = (p.slices + 3) / 4;
             int tm, tn;
             raster_tile<kOzRaster / 2>(w.t, p.tiles_m, p.tiles_n, tm, tn);
-            const int r = tm * 256 + row_in_pair, cb = tn * kPzN + half * kPzCols;
+            const int r = tm * 256 + row_in_pair, cb = tn * kPzN + part * COLS;
             const bool row_ok = r < p.m, tail = w.tt >= 0;
             const int er = row_ok ? p.row_exp[r] : kExpSentinel;
             // moderate exponents: alpha * 2^(er - w) * 2^fc and every product
@@ -1942,26 +1948,26 @@ __device__ __forceinline__ void ozaki_pair_body(const Src& src) {
             __syncwarp();  // the previous item's reads of the table are done
             bool cols_fast = true;
 #pragma unroll
-            for (int h = 0; h < kPzCols / 32; ++h) {
+            for (int h = 0; h < COLS / 32; ++h) {
                 const int j = lane + 32 * h, col = cb + j;
                 const int fc = col < p.n ? __ldg(p.col_exp + col) : kExpSentinel;
                 const bool mod = fc >= -200 && fc <= 200;
                 col_e[j] = fc;
-                col_scale[j] = mod ? pow2_normal(fc) : 0.0;
+                col_hi[j] = mod ? fc * (1 << 20) : 0;
                 cols_fast = cols_fast && (mod || col >= p.n);  // a column outside C: never stored
             }
             __syncwarp();
             // the whole warp takes the one-fma form, or none of it
             const bool fast = __all_sync(0xffffffffu, cols_fast && (row_fast || !row_ok));
-            double acc[kPzCols];
+            double acc[COLS];
             if (!tail) {
                 const double* c0 = p.cin + (row_ok ? r : 0) + static_cast<size_t>(cb) * p.ldc;
 #pragma unroll
-                for (int j = 0; j < kPzCols; ++j)
+                for (int j = 0; j < COLS; ++j)
                     acc[j] = (row_ok && p.beta_mode != 0 && cb + j < p.n) ? c0[static_cast<size_t>(j) * p.ldc] : 0.0;
                 if (p.beta_mode == 2) {
 #pragma unroll
-                    for (int j = 0; j < kPzCols; ++j) acc[j] = p.beta * acc[j];
+                    for (int j = 0; j < COLS; ++j) acc[j] = p.beta * acc[j];
                 }
             }
             bool first_pair = true;
@@ -1981,24 +1987,29 @@ __device__ __forceinline__ void ozaki_pair_body(const Src& src) {
                     const int mul = pair ? 256 : 0;
                     const double ars = fast && row_ok ? p.alpha * pow2_normal(er - wexp) : 0.0;
                     double* wplane = tail ? p.ws + (static_cast<size_t>(w.tt) * p.planes + w.plane + pi) * kPzTileElems +
-                                                row_in_pair + static_cast<size_t>(half * kPzCols) * 256
+                                                row_in_pair + static_cast<size_t>(part * COLS) * 256
                                           : nullptr;
                     const bool live = row_ok && (first_pair || er != kExpSentinel);
                     // chunks of 4 columns, each requested before the one ahead
                     // of it is used (4-column ones: 64 outputs in FP64 leave
                     // registers for two chunks of 2 x 4)
-                    constexpr int CH = 4, NCH = kPzCols / CH;
+                    constexpr int CH = 4, NCH = COLS / CH;
                     uint32_t v0[2][CH], v1[2][CH];
                     auto request = [&](int ch) {
                         tmem_ld4(tbase + j0 * kPzN + ch * CH, v0[ch & 1]);
                         tmem_ld4(tbase + (pair ? j0 + 1 : j0) * kPzN + ch * CH, v1[ch & 1]);
                     };
-                    // S_d0 * 256 + S_d1 (below 2^40) as a double: exact, by the
-                    // bits of 1.5 * 2^52 + T (alone, S_d0: mul 0 + 1 * v1)
+                    // T = S_d0 * 256 + S_d1 (below 2^40) as a double: exact, by the
+                    // bits of 1.5 * 2^52 + 2^31 + T, where S_d1 + 2^31 is a low
+                    // word (alone, S_d0: mul 0 + 1 * v1)
                     auto sum = [&](int ch, int jj) {
-                        const long long T = static_cast<long long>(static_cast<int32_t>(v0[ch & 1][jj])) * mul +
-                                            static_cast<int32_t>(v1[ch & 1][jj]);
-                        return __longlong_as_double(T + 0x4338000000000000LL) - 6755399441055744.0;
+                        const long long biased = 0x4338000000000000LL | (v1[ch & 1][jj] ^ 0x80000000u);
+                        const long long T = static_cast<long long>(static_cast<int32_t>(v0[ch & 1][jj])) * mul + biased;
+                        return __longlong_as_double(T) - 6755401588539392.0;
+                    };
+                    // ars * 2^fc, in the normal range (fast)
+                    auto scale = [&](int j) {
+                        return __hiloint2double(__double2hiint(ars) + col_hi[j], __double2loint(ars));
                     };
                     // one loop per case, so that a chunk's chains interleave
                     request(0);
@@ -2018,7 +2029,7 @@ __device__ __forceinline__ void ozaki_pair_body(const Src& src) {
                             if (ch + 1 < NCH) request(ch + 1);
 #pragma unroll
                             for (int jj = 0; jj < CH; ++jj)
-                                acc[ch * CH + jj] = fma(sum(ch, jj), ars * col_scale[ch * CH + jj], acc[ch * CH + jj]);
+                                acc[ch * CH + jj] = fma(sum(ch, jj), scale(ch * CH + jj), acc[ch * CH + jj]);
                         }
                     } else {
 #pragma unroll
@@ -2042,7 +2053,7 @@ __device__ __forceinline__ void ozaki_pair_body(const Src& src) {
             if (ok && row_ok && !tail) {
                 double* c = p.c + r + static_cast<size_t>(cb) * p.ldc;
 #pragma unroll
-                for (int j = 0; j < kPzCols; ++j)
+                for (int j = 0; j < COLS; ++j)
                     if (cb + j < p.n) c[static_cast<size_t>(j) * p.ldc] = acc[j];
             }
         }
@@ -2057,16 +2068,16 @@ __device__ __forceinline__ void ozaki_pair_body(const Src& src) {
     }
 }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPzThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pz_threads(kPzEpiWarps), 1)
     ozaki_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const __grid_constant__ OzParams p) {
-    ozaki_pair_body(PzSingleSrc{&p, &tmA, &tmB});
+    ozaki_pair_body<kPzEpiWarps>(PzSingleSrc{&p, &tmA, &tmB});
 }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPzThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pz_threads(kPzGroupEpiWarps), 1)
     ozaki_pair_grouped_kernel(const OzGroupEntry* __restrict__ tab, const int* __restrict__ starts, int nprob,
                               uint32_t* err) {
-    ozaki_pair_body(PzGroupSrc{OzGroupSrc{tab, starts, nprob, err}});
+    ozaki_pair_body<kPzGroupEpiWarps>(PzGroupSrc{OzGroupSrc{tab, starts, nprob, err}});
 }
 
 // The pair kernel's tail: per element, beta * C0, then for each pair of
@@ -3217,7 +3228,7 @@ cudaError_t launch_ozaki_gemm(bool ta, bool tb, int m, int n, int k, double alph
     KernelTimer tmr;
     kernel_timing_begin("umma_ozaki_i8", 2.0 * m * n * static_cast<double>(k) * slices * (slices + 1) / 2, st, &tmr);
     if (pair) {
-        ozaki_pair_kernel<<<2 * std::min(pz_items(p), sms / 2), kPzThreads, kPzSmem, st>>>(tma, tmb, p);
+        ozaki_pair_kernel<<<2 * std::min(pz_items(p), sms / 2), pz_threads(kPzEpiWarps), kPzSmem, st>>>(tma, tmb, p);
     } else {
         const int items = p.num_tiles + p.tail_tiles * (p.kchunks * upc - 1);
         const int grid = items < sms ? items : sms;
@@ -3455,7 +3466,7 @@ int ozaki_grouped_dev(const rb_gemm_problem* probs, size_t count, const void* co
             const OzGroupEntry* kt = dtab + kind_first[q];
             const int* ks0 = dstarts + kind_first[q] + q;
             if (q == 0)
-                ozaki_pair_grouped_kernel<<<2 * std::min(kind_tiles[0], sms / 2), kPzThreads, kPzSmem, ks>>>(
+                ozaki_pair_grouped_kernel<<<2 * std::min(kind_tiles[0], sms / 2), pz_threads(kPzGroupEpiWarps), kPzSmem, ks>>>(
                     kt, ks0, kind_count[0], err_word);
             else if (q == 1)
                 ozaki_grouped_kernel<256><<<std::min(kind_tiles[1], sms), kOzThreads, OzCfg<256>::SMEM, ks>>>(
