@@ -289,9 +289,13 @@ constexpr int kInvNB = 64;
 // columns g, g and t < 4) then touch distinct banks.
 constexpr int kInvLD = 68;
 constexpr int kInvThreads = 128;
-// L block and W (its inverse); the temporaries live in L's upper triangle,
-// which is zero and never read (three CTAs per SM)
-constexpr int kInvSmem = 2 * kInvNB * kInvLD * static_cast<int>(sizeof(double));
+// L block, which W (its inverse) replaces part by part: a part of L is read for
+// the last time when the product with it is formed. The temporaries live in
+// the upper triangle. A CTA is a chain of latencies (the load, 16 divisions, the
+// products), so the kernel's time goes with how many share an SM: six, with W in
+// a tile of its own three (1024 members of 512: 115 us against 171).
+constexpr int kInvSmem = kInvNB * kInvLD * static_cast<int>(sizeof(double));
+constexpr int kInvCtas = 6;
 
 // C(16 x 16) += A(16 x K) * B(K x 16), A and B column-major in shared memory
 // with column stride kInvLD; c[nb] holds columns 8 nb .. 8 nb + 7 in the DMMA
@@ -323,12 +327,11 @@ __device__ __forceinline__ void inv_store16(double* Ds, const double (&c)[2][4],
     }
 }
 
-__global__ void __launch_bounds__(kInvThreads) trsm_inv_diag_kernel(const double* __restrict__ A0, TbParams p,
+__global__ void __launch_bounds__(kInvThreads, kInvCtas) trsm_inv_diag_kernel(const double* __restrict__ A0, TbParams p,
                                                                      double* __restrict__ W, int nblocks) {
     extern __shared__ __align__(16) unsigned char inv_smem[];
     // element (r, c) of a tile at [c * kInvLD + r]
-    double* Ls = reinterpret_cast<double*>(inv_smem);  // L block (lower part read)
-    double* Ws = Ls + kInvNB * kInvLD;                  // its inverse
+    double* Ls = reinterpret_cast<double*>(inv_smem);  // L block, then its inverse
     const int b = blockIdx.x, member = blockIdx.y;
     const double* A = A0 + static_cast<size_t>(member) * p.stride_a;
     const int o = b * kInvNB, nb = min(kInvNB, p.q - o);
@@ -336,21 +339,22 @@ __global__ void __launch_bounds__(kInvThreads) trsm_inv_diag_kernel(const double
     const int g = lane >> 2, t = lane & 3;
 
     // L (lower part of the block; Unit puts 1 on the diagonal; rows and
-    // columns past nb are the identity), W zero. Thread tid & 63 loads row r
-    // of columns c = tid >> 6, +2, ...: 32 loads in flight.
+    // columns past nb are the identity). Thread tid & 63 loads row r of columns
+    // c = tid >> 6, +2, ...: 16 loads in flight.
     {
-        const int r = tid & 63, c0 = tid >> 6;
-        double v[kInvNB / 2];
+        const int r = tid & 63;
 #pragma unroll
-        for (int i = 0; i < kInvNB / 2; ++i) {
-            const int c = c0 + 2 * i;
-            const bool in = r < nb && (c < r || (c == r && !p.unit));
-            v[i] = in ? __ldg(a_ptr(A, p, o + r, o + c)) : (c == r ? 1.0 : 0.0);
-        }
+        for (int h = 0; h < 2; ++h) {
+            const int c0 = (tid >> 6) + kInvNB / 2 * h;
+            double v[kInvNB / 4];
 #pragma unroll
-        for (int i = 0; i < kInvNB / 2; ++i) {
-            Ls[(c0 + 2 * i) * kInvLD + r] = v[i];
-            Ws[(c0 + 2 * i) * kInvLD + r] = 0.0;
+            for (int i = 0; i < kInvNB / 4; ++i) {
+                const int c = c0 + 2 * i;
+                const bool in = r < nb && (c < r || (c == r && !p.unit));
+                v[i] = in ? __ldg(a_ptr(A, p, o + r, o + c)) : (c == r ? 1.0 : 0.0);
+            }
+#pragma unroll
+            for (int i = 0; i < kInvNB / 4; ++i) Ls[(c0 + 2 * i) * kInvLD + r] = v[i];
         }
     }
     __syncthreads();
@@ -367,8 +371,9 @@ __global__ void __launch_bounds__(kInvThreads) trsm_inv_diag_kernel(const double
             const double v = ((r == c) ? 1.0 : 0.0) - (acc[0] + acc[1]);
             w[r] = (r < c) ? 0.0 : v / Ls[(d + r) * kInvLD + d + r];
         }
+        __syncwarp();  // the warp's two blocks have been read
 #pragma unroll
-        for (int r = 0; r < 16; ++r) Ws[(d + c) * kInvLD + d + r] = w[r];
+        for (int r = 0; r < 16; ++r) Ls[(d + c) * kInvLD + d + r] = w[r];
     }
     __syncthreads();
     // 16 -> 32: warp h (0, 1) forms W[hi][lo] of the 32 x 32 diagonal block h
@@ -378,12 +383,15 @@ __global__ void __launch_bounds__(kInvThreads) trsm_inv_diag_kernel(const double
         const int lo = 32 * warp, hi = lo + 16;
         double* Tw = Ls + hi * kInvLD + lo;  // L[lo][hi]: upper, unused
         double c[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
-        inv_mm16<16>(Ls + lo * kInvLD + hi, Ws + lo * kInvLD + lo, c, g, t);
+        inv_mm16<16>(Ls + lo * kInvLD + hi, Ls + lo * kInvLD + lo, c, g, t);
         inv_store16(Tw, c, 1.0, g, t);
         __syncwarp();
         double e[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
-        inv_mm16<16>(Ws + hi * kInvLD + hi, Tw, e, g, t);
-        inv_store16(Ws + lo * kInvLD + hi, e, -1.0, g, t);
+        inv_mm16<16>(Ls + hi * kInvLD + hi, Tw, e, g, t);
+        inv_store16(Ls + lo * kInvLD + hi, e, -1.0, g, t);
+        __syncwarp();
+        const double zero[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
+        inv_store16(Tw, zero, 1.0, g, t);  // the 32 x 32 inverses are read whole below
     }
     __syncthreads();
     // 32 -> 64: T = L[32:64][0:32] * W[0:32][0:32], then
@@ -393,19 +401,20 @@ __global__ void __launch_bounds__(kInvThreads) trsm_inv_diag_kernel(const double
         const int mi = warp >> 1, ni = warp & 1;
         double c[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
         double* Ts = Ls + 32 * kInvLD;  // L[0:32][32:64]: upper, unused
-        inv_mm16<32>(Ls + 32 + 16 * mi, Ws + 16 * ni * kInvLD, c, g, t);
+        inv_mm16<32>(Ls + 32 + 16 * mi, Ls + 16 * ni * kInvLD, c, g, t);
         inv_store16(Ts + 16 * ni * kInvLD + 16 * mi, c, 1.0, g, t);
         __syncthreads();
         double e[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
-        inv_mm16<32>(Ws + 32 * kInvLD + 32 + 16 * mi, Ts + 16 * ni * kInvLD, e, g, t);
-        inv_store16(Ws + 16 * ni * kInvLD + 32 + 16 * mi, e, -1.0, g, t);
+        inv_mm16<32>(Ls + 32 * kInvLD + 32 + 16 * mi, Ts + 16 * ni * kInvLD, e, g, t);
+        inv_store16(Ls + 16 * ni * kInvLD + 32 + 16 * mi, e, -1.0, g, t);
     }
     __syncthreads();
-    // W_b column-major, zero outside the block's nb x nb (coalesced stores)
+    // W_b column-major, zero above its diagonal 16 x 16 blocks and outside the
+    // block's nb x nb (coalesced stores)
     double* Wb = W + (static_cast<size_t>(member) * nblocks + b) * (kInvNB * kInvNB);
     for (int idx = tid; idx < kInvNB * kInvNB; idx += kInvThreads) {
         const int r = idx % kInvNB, c = idx / kInvNB;
-        Wb[idx] = (r < nb && c < nb) ? Ws[c * kInvLD + r] : 0.0;
+        Wb[idx] = (r < nb && c < nb && (r >> 4) >= (c >> 4)) ? Ls[c * kInvLD + r] : 0.0;
     }
 }
 
@@ -641,8 +650,8 @@ __global__ void __launch_bounds__(kTbThreads, 2)
 // 64-column tile -- and then X_b = W_b * Z, warp (xm, ks) the column half ks.
 // All warps have the same work in both, and Y is read and written once per
 // block. A half's fragments are requested while the DMMAs of the half before
-// it run, across the barriers too. 1024 x (512, 64): 1281 -> 1002 us (of which
-// the inversion 171); a CTA's 104K clocks: products 64K (57K at the pipe's
+// it run, across the barriers too. 1024 x (512, 64): 1281 -> 1002 us (171 of
+// either the inversion, 115 now); a CTA's 104K clocks: products 64K (57K at the pipe's
 // rate), Z 21K, X 7K, B in and out 12K.
 constexpr int kTwRB = 32, kTwYS = 36;
 
