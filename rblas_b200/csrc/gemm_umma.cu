@@ -19,13 +19,14 @@
 // (src/kernel/gemm.rs:185-429) for the precision forms that rblas does not
 // have; the plain forms live in gemm_simt.cu.
 //
-// Kernel structure (persistent, one CTA per SM, 6 warps):
+// Large products run on CTA pairs (umma_pair_kernel, ozaki_pair_kernel; tall
+// ones with A split inside: umma_split_fused_kernel). Single-CTA structure of
+// the others (persistent, one CTA per SM, 6 warps; Ozaki's 18):
 //   warp 0 lane 0  TMA producer: K-major operand tiles (128-byte rows, 128-byte
 //                  swizzle) into a STAGES-deep shared-memory ring.
-//   warp 1         allocates 512 TMEM columns; lane 0 issues tcgen05.mma
-//                  (M=128, N=256) into one of two 256-column accumulators and
-//                  commits each stage back to the producer.
-//   warps 2..5     epilogue: tcgen05.ld the accumulator (warp w reads TMEM
+//   warp 1         allocates TMEM; lane 0 issues tcgen05.mma into one of two
+//                  accumulators and commits each stage back to the producer.
+//   warps 2..      epilogue: tcgen05.ld the accumulator (warp w reads TMEM
 //                  lanes 32*(w%4)..+31 = tile rows), apply the form's
 //                  scaling and alpha/beta, store C coalesced; release the
 //                  accumulator so the next unit's MMAs overlap this drain.
@@ -2215,6 +2216,38 @@ __device__ __forceinline__ void row_exp_rcontig(const double* __restrict__ x, si
     for (int q = p0; q < p1; ++q) best = max(best, abs_bits(x[r + static_cast<size_t>(q) * ps]));
     if (best != 0) atomicMax(e + r, frexp_exp(__longlong_as_double(best)));
 }
+// The same for the real form of a complex operand (cx: see load_tile_complex), whose
+// rows 2 i and 2 i + 1 hold row i's parts and their negatives: R and K are the
+// complex sizes here.
+__global__ void row_exp_complex_kernel(const double* __restrict__ x, size_t ld, int cx, int R, int K,
+                                       int* __restrict__ e) {
+    long long best = 0;
+    int r;
+    if (cx == 1) {  // rows contiguous: a thread per row, 32 columns
+        r = blockIdx.x * blockDim.x + threadIdx.x;
+        if (r >= R) return;
+        const int p0 = blockIdx.y * 32, p1 = min(K, p0 + 32);
+#pragma unroll 8
+        for (int q = p0; q < p1; ++q) {
+            const double* v = x + 2 * (r + static_cast<size_t>(q) * ld);
+            best = max(best, max(abs_bits(v[0]), abs_bits(v[1])));
+        }
+    } else {  // K contiguous: a warp per row, 1024 columns
+        r = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+        if (r >= R) return;
+        const double* v = x + 2 * static_cast<size_t>(r) * ld;
+        const int p1 = 2 * min(K, static_cast<int>(blockIdx.y + 1) * 1024);
+#pragma unroll 8
+        for (int q = blockIdx.y * 2048 + (threadIdx.x & 31); q < p1; q += 32) best = max(best, abs_bits(v[q]));
+        for (int o = 16; o; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
+        if ((threadIdx.x & 31) != 0) return;
+    }
+    if (best != 0) {
+        const int ex = frexp_exp(__longlong_as_double(best));
+        atomicMax(e + 2 * r, ex);
+        atomicMax(e + 2 * r + 1, ex);
+    }
+}
 __global__ void row_exp_kcontig_kernel(const double* __restrict__ x, size_t rs, int R, int K,
                                        int* __restrict__ e) {
     row_exp_kcontig(x, rs, R, K, e, blockIdx.x, blockIdx.y);
@@ -2317,15 +2350,47 @@ __device__ __forceinline__ void load_tile_sliced(const double* __restrict__ x, s
     }
 }
 
+// The tile of the real form [[Re, -Im], [Im, Re]] (by element: rows 2 i, 2 i + 1,
+// columns 2 p, 2 p + 1) of op(A), A complex column-major with leading dimension
+// ld: cx 1 A, 2 A^T, 3 A^H. r0, p0, R, K in the real form.
+__device__ __forceinline__ void load_tile_complex(const double* __restrict__ x, size_t ld, int cx, int R, int K,
+                                                  int r0, int p0, double (*tile)[kSliceLD]) {
+    constexpr int CT = kTile / 2, PER = CT * CT / kTileThreads;
+    double re[PER], im[PER];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int idx = threadIdx.x + i * kTileThreads;
+        const int a = idx % CT, b = idx / CT;  // along the columns of A, across them
+        const int r = r0 / 2 + (cx == 1 ? a : b), q = p0 / 2 + (cx == 1 ? b : a);
+        const double* v = x + 2 * (cx == 1 ? r + static_cast<size_t>(q) * ld : q + static_cast<size_t>(r) * ld);
+        const bool in = r < R / 2 && q < K / 2;
+        re[i] = in ? v[0] : 0.0;
+        im[i] = in ? v[1] : 0.0;
+    }
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int idx = threadIdx.x + i * kTileThreads;
+        const int a = idx % CT, b = idx / CT;
+        const int r = 2 * (cx == 1 ? a : b), q = 2 * (cx == 1 ? b : a);
+        const double v = cx == 3 ? 0.0 - im[i] : im[i];
+        tile[r][slice_col(q)] = re[i];
+        tile[r + 1][slice_col(q)] = v;
+        tile[r][slice_col(q + 1)] = 0.0 - v;
+        tile[r + 1][slice_col(q + 1)] = re[i];
+    }
+}
+
+// cx != 0: x is a complex operand with leading dimension rs (load_tile_complex).
 template <int S>
-__device__ __forceinline__ void ozaki_slice_tile(const double* __restrict__ x, size_t rs, size_t ps, int R, int K,
-                                                 const int* __restrict__ e, int8_t* __restrict__ out, size_t kp,
-                                                 size_t plane, int bx, int by) {
+__device__ __forceinline__ void ozaki_slice_tile(const double* __restrict__ x, size_t rs, size_t ps, int cx, int R,
+                                                 int K, const int* __restrict__ e, int8_t* __restrict__ out,
+                                                 size_t kp, size_t plane, int bx, int by) {
     using Int = typename std::conditional<(S <= 8), long long, __int128>::type;
     constexpr int slices = S;
     __shared__ double tile[kTile][kSliceLD];
     const int r0 = by * kTile, p0 = bx * kTile;
-    load_tile_sliced(x, rs, ps, R, K, r0, p0, tile);
+    if (cx) load_tile_complex(x, rs, cx, R, K, r0, p0, tile);
+    else    load_tile_sliced(x, rs, ps, R, K, r0, p0, tile);
     __syncthreads();
     const int r = threadIdx.x >> 2, c = threadIdx.x & 3;  // 64 rows x 4 chunks of 16
     if (r0 + r >= R) return;
@@ -2392,10 +2457,10 @@ __device__ __forceinline__ void ozaki_slice_tile(const double* __restrict__ x, s
 }
 
 template <int S>
-__global__ void __launch_bounds__(256) ozaki_slice_kernel(const double* __restrict__ x, size_t rs, size_t ps,
+__global__ void __launch_bounds__(256) ozaki_slice_kernel(const double* __restrict__ x, size_t rs, size_t ps, int cx,
                                                           int R, int K, const int* __restrict__ e,
                                                           int8_t* __restrict__ out, size_t kp, size_t plane) {
-    ozaki_slice_tile<S>(x, rs, ps, R, K, e, out, kp, plane, blockIdx.x, blockIdx.y);
+    ozaki_slice_tile<S>(x, rs, ps, cx, R, K, e, out, kp, plane, blockIdx.x, blockIdx.y);
 }
 
 // ---- grouped pre-pass: one launch per pass over every operand of a batch ------
@@ -2440,15 +2505,15 @@ template <int S>
 __global__ void __launch_bounds__(256) ozaki_slice_grouped_kernel(const OzOperand* __restrict__ ops, int nops) {
     const OzOperand& o = ops[oz_find_operand(ops, nops, blockIdx.x, true)];
     const int b = blockIdx.x - o.slice_start;
-    ozaki_slice_tile<S>(o.x, o.rs, o.ps, o.R, o.K, o.e, o.out, o.kp, o.plane, b % o.slice_gx, b / o.slice_gx);
+    ozaki_slice_tile<S>(o.x, o.rs, o.ps, 0, o.R, o.K, o.e, o.out, o.kp, o.plane, b % o.slice_gx, b / o.slice_gx);
 }
 
 // Host dispatch on the slice count (2 .. 12).
-void launch_ozaki_slices(dim3 grid, cudaStream_t st, const double* x, size_t rs, size_t ps, int R, int K,
+void launch_ozaki_slices(dim3 grid, cudaStream_t st, const double* x, size_t rs, size_t ps, int cx, int R, int K,
                          const int* e, int slices, int8_t* out, size_t kp, size_t plane) {
     switch (slices) {
 #define RB_SLICES(S) \
-    case S: ozaki_slice_kernel<S><<<grid, 256, 0, st>>>(x, rs, ps, R, K, e, out, kp, plane); break;
+    case S: ozaki_slice_kernel<S><<<grid, 256, 0, st>>>(x, rs, ps, cx, R, K, e, out, kp, plane); break;
         RB_SLICES(2) RB_SLICES(3) RB_SLICES(4) RB_SLICES(5) RB_SLICES(6) RB_SLICES(7) RB_SLICES(8)
         RB_SLICES(9) RB_SLICES(10) RB_SLICES(11) RB_SLICES(12)
 #undef RB_SLICES
@@ -3158,7 +3223,7 @@ bool ozaki_pair_tiles(int m, int n) {
 
 cudaError_t launch_ozaki_gemm(bool ta, bool tb, int m, int n, int k, double alpha, const double* A,
                               size_t lda, const double* B, size_t ldb, double beta, double* C,
-                              size_t ldc, int slices, cudaStream_t st, CUresult* cu_err) {
+                              size_t ldc, int slices, cudaStream_t st, CUresult* cu_err, int a_cx) {
     const size_t kp = round_up(static_cast<size_t>(k), 16);
     const size_t pa = static_cast<size_t>(m) * kp, pb = static_cast<size_t>(n) * kp;
     void* buf = nullptr;
@@ -3196,14 +3261,19 @@ cudaError_t launch_ozaki_gemm(bool ta, bool tb, int m, int n, int k, double alph
     operand_views(ta, tb, lda, ldb, ars, aps, brs, bps);
     fill_int_kernel<<<64, 256, 0, st>>>(ea, m + n, kExpSentinel);
     const int kb = (k + 1023) / 1024, k32 = (k + 31) / 32;
-    if (aps == 1) row_exp_kcontig_kernel<<<dim3((m + 7) / 8, kb), 256, 0, st>>>(A, ars, m, k, ea);
+    if (a_cx) {
+        ars = lda;
+        const int mc = m / 2, kc = k / 2;
+        const dim3 g = a_cx == 1 ? dim3((mc + 255) / 256, (kc + 31) / 32) : dim3((mc + 7) / 8, (kc + 1023) / 1024);
+        row_exp_complex_kernel<<<g, 256, 0, st>>>(A, lda, a_cx, mc, kc, ea);
+    } else if (aps == 1) row_exp_kcontig_kernel<<<dim3((m + 7) / 8, kb), 256, 0, st>>>(A, ars, m, k, ea);
     else          row_exp_rcontig_kernel<<<dim3((m + 255) / 256, k32), 256, 0, st>>>(A, aps, m, k, ea);
     if (bps == 1) row_exp_kcontig_kernel<<<dim3((n + 7) / 8, kb), 256, 0, st>>>(B, brs, n, k, eb);
     else          row_exp_rcontig_kernel<<<dim3((n + 255) / 256, k32), 256, 0, st>>>(B, bps, n, k, eb);
     const dim3 ga((kp + kTile - 1) / kTile, (m + kTile - 1) / kTile);
     const dim3 gb((kp + kTile - 1) / kTile, (n + kTile - 1) / kTile);
-    launch_ozaki_slices(ga, st, A, ars, aps, m, k, ea, slices, sla, kp, pa);
-    launch_ozaki_slices(gb, st, B, brs, bps, n, k, eb, slices, slb, kp, pb);
+    launch_ozaki_slices(ga, st, A, ars, aps, a_cx, m, k, ea, slices, sla, kp, pa);
+    launch_ozaki_slices(gb, st, B, brs, bps, 0, n, k, eb, slices, slb, kp, pb);
     count_launch(5);
     CUtensorMap tma, tmb;
     CUresult r = make_tmap_planes(&tma, sla, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, k, m, slices, kp, kUM);
@@ -3635,8 +3705,8 @@ extern "C" rb_status rb_dgemm_ozaki_noalloc(rb_layout layout, rb_transpose trans
         else          row_exp_rcontig_kernel<<<dim3((N + 255) / 256, k32), 256, 0, st>>>(cb, bps, N, K, eb);
         const dim3 ga((kp + kTile - 1) / kTile, (M + kTile - 1) / kTile);
         const dim3 gb((kp + kTile - 1) / kTile, (N + kTile - 1) / kTile);
-        launch_ozaki_slices(ga, st, ca, ars, aps, M, K, ea, slices, sla, kp, pa);
-        launch_ozaki_slices(gb, st, cb, brs, bps, N, K, eb, slices, slb, kp, pb);
+        launch_ozaki_slices(ga, st, ca, ars, aps, 0, M, K, ea, slices, sla, kp, pa);
+        launch_ozaki_slices(gb, st, cb, brs, bps, 0, N, K, eb, slices, slb, kp, pb);
         count_launch(5);
         CUtensorMap tma, tmb;
         CUresult r = make_tmap_planes(&tma, sla, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, K, M, slices, kp, kUM);

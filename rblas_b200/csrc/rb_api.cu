@@ -320,6 +320,7 @@ struct ColProblem {
     T* c; size_t ldc;
     int tri = 0;  // syrk: restrict C to one triangle
     bool split_ok = true;  // the plain form may take the grouped kernel's split-K
+    int a_cx = 0;          // Ozaki form: A complex (launch_ozaki_gemm)
 };
 
 // The plain problem as one grouped-kernel entry; the factor by which the
@@ -400,7 +401,7 @@ rb_status run_precision_form(const ColProblem<T>& p, rb_precision prec, cudaStre
             return RB_ERR_UNSUPPORTED;
         }
         e = launch_ozaki_gemm(p.ta, p.tb, (int)p.m, (int)p.n, (int)p.k, p.alpha, p.a, p.lda, p.b, p.ldb,
-                              p.beta, p.c, p.ldc, ozaki_slices(), st, &cu);
+                              p.beta, p.c, p.ldc, ozaki_slices(), st, &cu, p.a_cx);
     }
     if (cu != CUDA_SUCCESS) {
         set_err(err, RB_ERR_CUDA, 0, 0, 0, static_cast<int32_t>(cu));
@@ -849,8 +850,9 @@ rb_status invalid(rb_error* err) {
 template <typename T>
 int gemm_colmajor_dev(bool ta, bool tb, size_t m, size_t n, size_t k, T alpha, const T* A,
                       size_t lda, const T* B, size_t ldb, T beta, T* C, size_t ldc, int prec,
-                      cudaStream_t st, int tri, int32_t* cuda_err) {
+                      cudaStream_t st, int tri, int32_t* cuda_err, int a_cx) {
     ColProblem<T> p{ta, tb, m, n, k, alpha, beta, A, lda, B, ldb, C, ldc, tri};
+    p.a_cx = a_cx;
     rb_error e{};
     const rb_status s = run_dev<T>(p, static_cast<rb_precision>(prec), st, &e);
     if (cuda_err) *cuda_err = e.cuda_error;
@@ -858,10 +860,10 @@ int gemm_colmajor_dev(bool ta, bool tb, size_t m, size_t n, size_t k, T alpha, c
 }
 template int gemm_colmajor_dev<float>(bool, bool, size_t, size_t, size_t, float, const float*, size_t,
                                       const float*, size_t, float, float*, size_t, int, cudaStream_t,
-                                      int, int32_t*);
+                                      int, int32_t*, int);
 template int gemm_colmajor_dev<double>(bool, bool, size_t, size_t, size_t, double, const double*,
                                        size_t, const double*, size_t, double, double*, size_t, int,
-                                       cudaStream_t, int, int32_t*);
+                                       cudaStream_t, int, int32_t*, int);
 
 uint32_t* device_error_word() {
     cudaError_t e;

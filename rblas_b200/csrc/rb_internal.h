@@ -138,7 +138,7 @@ cudaError_t launch_scale_c(int m, int n, T beta, T* C, size_t ldc, cudaStream_t 
 template <typename T>
 int gemm_colmajor_dev(bool ta, bool tb, size_t m, size_t n, size_t k, T alpha, const T* A,
                       size_t lda, const T* B, size_t ldb, T beta, T* C, size_t ldc, int prec,
-                      cudaStream_t st, int tri, int32_t* cuda_err);
+                      cudaStream_t st, int tri, int32_t* cuda_err, int a_cx = 0);
 
 // BF16-split SGEMM on tcgen05 (kind::f16): planes == 2 is 3xBF16
 // (hi*hi + hi*lo + lo*hi), planes == 3 is the 6-product form over hi/mid/lo.
@@ -149,10 +149,12 @@ cudaError_t launch_bf16_split_gemm(int planes, bool ta, bool tb, int m, int n, i
                                    float* C, size_t ldc, cudaStream_t st, CUresult* cu_err);
 
 // Ozaki INT8-slice DGEMM on tcgen05 (kind::i8, exact INT32 in TMEM, FP64
-// summation and alpha/beta epilogue).
+// summation and alpha/beta epilogue). a_cx != 0: A is complex, lda in complex
+// elements, and its real form (m x k, [[Re, -Im], [Im, Re]] by element) is the
+// operand: 1 of A, 2 of A^T, 3 of A^H.
 cudaError_t launch_ozaki_gemm(bool ta, bool tb, int m, int n, int k, double alpha, const double* A,
                               size_t lda, const double* B, size_t ldb, double beta, double* C,
-                              size_t ldc, int slices, cudaStream_t st, CUresult* cu_err);
+                              size_t ldc, int slices, cudaStream_t st, CUresult* cu_err, int a_cx = 0);
 
 // Many f64 problems in the Ozaki form in one grouped launch (plus one
 // exponent and one slice pass over all operands). cin / ldcin (optional)
