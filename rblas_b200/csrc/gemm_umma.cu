@@ -2219,26 +2219,26 @@ __device__ __forceinline__ void row_exp_rcontig(const double* __restrict__ x, si
 // The same for the real form of a complex operand (cx: see load_tile_complex), whose
 // rows 2 i and 2 i + 1 hold row i's parts and their negatives: R and K are the
 // complex sizes here.
-__global__ void row_exp_complex_kernel(const double* __restrict__ x, size_t ld, int cx, int R, int K,
-                                       int* __restrict__ e) {
+__device__ __forceinline__ void row_exp_complex(const double* __restrict__ x, size_t ld, int cx, int R, int K,
+                                                int* __restrict__ e, int bx, int by) {
     long long best = 0;
     int r;
     if (cx == 1) {  // rows contiguous: a thread per row, 32 columns
-        r = blockIdx.x * blockDim.x + threadIdx.x;
+        r = bx * blockDim.x + threadIdx.x;
         if (r >= R) return;
-        const int p0 = blockIdx.y * 32, p1 = min(K, p0 + 32);
+        const int p0 = by * 32, p1 = min(K, p0 + 32);
 #pragma unroll 8
         for (int q = p0; q < p1; ++q) {
             const double* v = x + 2 * (r + static_cast<size_t>(q) * ld);
             best = max(best, max(abs_bits(v[0]), abs_bits(v[1])));
         }
     } else {  // K contiguous: a warp per row, 1024 columns
-        r = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+        r = bx * (blockDim.x / 32) + (threadIdx.x >> 5);
         if (r >= R) return;
         const double* v = x + 2 * static_cast<size_t>(r) * ld;
-        const int p1 = 2 * min(K, static_cast<int>(blockIdx.y + 1) * 1024);
+        const int p1 = 2 * min(K, (by + 1) * 1024);
 #pragma unroll 8
-        for (int q = blockIdx.y * 2048 + (threadIdx.x & 31); q < p1; q += 32) best = max(best, abs_bits(v[q]));
+        for (int q = by * 2048 + (threadIdx.x & 31); q < p1; q += 32) best = max(best, abs_bits(v[q]));
         for (int o = 16; o; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
         if ((threadIdx.x & 31) != 0) return;
     }
@@ -2248,15 +2248,6 @@ __global__ void row_exp_complex_kernel(const double* __restrict__ x, size_t ld, 
         atomicMax(e + 2 * r + 1, ex);
     }
 }
-__global__ void row_exp_kcontig_kernel(const double* __restrict__ x, size_t rs, int R, int K,
-                                       int* __restrict__ e) {
-    row_exp_kcontig(x, rs, R, K, e, blockIdx.x, blockIdx.y);
-}
-__global__ void row_exp_rcontig_kernel(const double* __restrict__ x, size_t ps, int R, int K,
-                                       int* __restrict__ e) {
-    row_exp_rcontig(x, ps, R, K, e, blockIdx.x, blockIdx.y);
-}
-
 constexpr int kTile = 64;
 
 // Load a 64 x 64 tile of the R x K view into shared memory (coalesced along
@@ -2456,22 +2447,16 @@ __device__ __forceinline__ void ozaki_slice_tile(const double* __restrict__ x, s
         *reinterpret_cast<uint4*>(out + t * plane + off) = make_uint4(w[t][0], w[t][1], w[t][2], w[t][3]);
 }
 
-template <int S>
-__global__ void __launch_bounds__(256) ozaki_slice_kernel(const double* __restrict__ x, size_t rs, size_t ps, int cx,
-                                                          int R, int K, const int* __restrict__ e,
-                                                          int8_t* __restrict__ out, size_t kp, size_t plane) {
-    ozaki_slice_tile<S>(x, rs, ps, cx, R, K, e, out, kp, plane, blockIdx.x, blockIdx.y);
-}
+// ---- pre-pass: one launch per pass over both operands, or every one of a batch ------
 
-// ---- grouped pre-pass: one launch per pass over every operand of a batch ------
-
-// One operand of a grouped Ozaki launch, viewed as R x K (element (r, p) at
+// One operand, viewed as R x K (element (r, p) at
 // x[r*rs + p*ps]): its exponents e[R] and digit planes out[slices][R][kp].
 // exp_blocks / slice_blocks: the blocks it takes in each pass (the grid's
 // blocks are dealt to operands by the prefix sums exp_start / slice_start).
 struct OzOperand {
     const double* x;
     size_t rs, ps;
+    int cx;  // != 0: complex, leading dimension rs (load_tile_complex)
     int R, K;
     int* e;
     int8_t* out;
@@ -2490,35 +2475,74 @@ __device__ __forceinline__ int oz_find_operand(const OzOperand* ops, int nops, i
     return lo;
 }
 
-// The exponent pass of every operand (grid = total exponent blocks; e
-// pre-filled with the zero-row sentinel).
-__global__ void __launch_bounds__(256) ozaki_exp_grouped_kernel(const OzOperand* __restrict__ ops, int nops) {
-    const OzOperand& o = ops[oz_find_operand(ops, nops, blockIdx.x, false)];
-    const int b = blockIdx.x - o.exp_start;
+// Block b of an operand's exponent pass (e pre-filled with the zero-row
+// sentinel), of its slice pass. CX: operands may be complex (a test of o.cx cost
+// the grouped passes 4 % of a call).
+template <bool CX>
+__device__ __forceinline__ void oz_exp_block(const OzOperand& o, int b) {
     const int bx = b % o.exp_gx, by = b / o.exp_gx;
-    if (o.ps == 1) row_exp_kcontig(o.x, o.rs, o.R, o.K, o.e, bx, by);
-    else           row_exp_rcontig(o.x, o.ps, o.R, o.K, o.e, bx, by);
+    if (CX && o.cx)     row_exp_complex(o.x, o.rs, o.cx, o.R / 2, o.K / 2, o.e, bx, by);
+    else if (o.ps == 1) row_exp_kcontig(o.x, o.rs, o.R, o.K, o.e, bx, by);
+    else                row_exp_rcontig(o.x, o.ps, o.R, o.K, o.e, bx, by);
+}
+template <int S, bool CX>
+__device__ __forceinline__ void oz_slice_block(const OzOperand& o, int b) {
+    ozaki_slice_tile<S>(o.x, o.rs, o.ps, CX ? o.cx : 0, o.R, o.K, o.e, o.out, o.kp, o.plane, b % o.slice_gx, b / o.slice_gx);
+}
+// Sets o's blocks along R and K and the first block after those before it
+// (exp, slice: blocks so far, advanced).
+void oz_operand_blocks(OzOperand* o, int* exp, int* slice) {
+    const int R = o->cx ? o->R / 2 : o->R, K = o->cx ? o->K / 2 : o->K;
+    const bool kcontig = o->cx ? o->cx != 1 : o->ps == 1;
+    o->exp_gx = kcontig ? (R + 7) / 8 : (R + 255) / 256;
+    o->exp_start = *exp;
+    *exp += o->exp_gx * (kcontig ? (K + 1023) / 1024 : (K + 31) / 32);
+    o->slice_gx = static_cast<int>((o->kp + kTile - 1) / kTile);
+    o->slice_start = *slice;
+    *slice += o->slice_gx * ((o->R + kTile - 1) / kTile);
 }
 
-// The slice pass of every operand (grid = total slice tiles).
+__global__ void __launch_bounds__(256) ozaki_exp_grouped_kernel(const OzOperand* __restrict__ ops, int nops) {
+    const OzOperand& o = ops[oz_find_operand(ops, nops, blockIdx.x, false)];
+    oz_exp_block<false>(o, blockIdx.x - o.exp_start);
+}
 template <int S>
 __global__ void __launch_bounds__(256) ozaki_slice_grouped_kernel(const OzOperand* __restrict__ ops, int nops) {
     const OzOperand& o = ops[oz_find_operand(ops, nops, blockIdx.x, true)];
-    const int b = blockIdx.x - o.slice_start;
-    ozaki_slice_tile<S>(o.x, o.rs, o.ps, 0, o.R, o.K, o.e, o.out, o.kp, o.plane, b % o.slice_gx, b / o.slice_gx);
+    oz_slice_block<S, false>(o, blockIdx.x - o.slice_start);
 }
 
-// Host dispatch on the slice count (2 .. 12).
-void launch_ozaki_slices(dim3 grid, cudaStream_t st, const double* x, size_t rs, size_t ps, int cx, int R, int K,
-                         const int* e, int slices, int8_t* out, size_t kp, size_t plane) {
+// One problem: its operands as kernel parameters, A's blocks then B's, so the
+// two share a launch's tail (five launches before: 1024^3 91 -> 81 us).
+struct OzPair {
+    OzOperand op[2];
+};
+__global__ void __launch_bounds__(256) ozaki_exp_kernel(const __grid_constant__ OzPair p) {
+    const int b = blockIdx.x, i = b >= p.op[1].exp_start;
+    oz_exp_block<true>(p.op[i], b - p.op[i].exp_start);
+}
+template <int S>
+__global__ void __launch_bounds__(256) ozaki_slice_kernel(const __grid_constant__ OzPair p) {
+    const int b = blockIdx.x, i = b >= p.op[1].slice_start;
+    oz_slice_block<S, true>(p.op[i], b - p.op[i].slice_start);
+}
+
+// Exponents (op[0].e, op[1].e adjacent) and digit planes of both operands;
+// slices 2 .. 12.
+void launch_ozaki_prepass(OzPair p, int slices, cudaStream_t st) {
+    int exp = 0, slice = 0;
+    for (OzOperand& o : p.op) oz_operand_blocks(&o, &exp, &slice);
+    fill_int_kernel<<<64, 256, 0, st>>>(p.op[0].e, p.op[0].R + p.op[1].R, kExpSentinel);
+    ozaki_exp_kernel<<<exp, 256, 0, st>>>(p);
     switch (slices) {
 #define RB_SLICES(S) \
-    case S: ozaki_slice_kernel<S><<<grid, 256, 0, st>>>(x, rs, ps, cx, R, K, e, out, kp, plane); break;
+    case S: ozaki_slice_kernel<S><<<slice, 256, 0, st>>>(p); break;
         RB_SLICES(2) RB_SLICES(3) RB_SLICES(4) RB_SLICES(5) RB_SLICES(6) RB_SLICES(7) RB_SLICES(8)
         RB_SLICES(9) RB_SLICES(10) RB_SLICES(11) RB_SLICES(12)
 #undef RB_SLICES
         default: break;
     }
+    count_launch(3);
 }
 
 // BF16 split into `planes` (2 or 3) planes: out[0] = bf16(x),
@@ -3259,22 +3283,10 @@ cudaError_t launch_ozaki_gemm(bool ta, bool tb, int m, int n, int k, double alph
     int8_t* slb = sla + a_bytes;
     size_t ars, aps, brs, bps;
     operand_views(ta, tb, lda, ldb, ars, aps, brs, bps);
-    fill_int_kernel<<<64, 256, 0, st>>>(ea, m + n, kExpSentinel);
-    const int kb = (k + 1023) / 1024, k32 = (k + 31) / 32;
-    if (a_cx) {
-        ars = lda;
-        const int mc = m / 2, kc = k / 2;
-        const dim3 g = a_cx == 1 ? dim3((mc + 255) / 256, (kc + 31) / 32) : dim3((mc + 7) / 8, (kc + 1023) / 1024);
-        row_exp_complex_kernel<<<g, 256, 0, st>>>(A, lda, a_cx, mc, kc, ea);
-    } else if (aps == 1) row_exp_kcontig_kernel<<<dim3((m + 7) / 8, kb), 256, 0, st>>>(A, ars, m, k, ea);
-    else          row_exp_rcontig_kernel<<<dim3((m + 255) / 256, k32), 256, 0, st>>>(A, aps, m, k, ea);
-    if (bps == 1) row_exp_kcontig_kernel<<<dim3((n + 7) / 8, kb), 256, 0, st>>>(B, brs, n, k, eb);
-    else          row_exp_rcontig_kernel<<<dim3((n + 255) / 256, k32), 256, 0, st>>>(B, bps, n, k, eb);
-    const dim3 ga((kp + kTile - 1) / kTile, (m + kTile - 1) / kTile);
-    const dim3 gb((kp + kTile - 1) / kTile, (n + kTile - 1) / kTile);
-    launch_ozaki_slices(ga, st, A, ars, aps, a_cx, m, k, ea, slices, sla, kp, pa);
-    launch_ozaki_slices(gb, st, B, brs, bps, 0, n, k, eb, slices, slb, kp, pb);
-    count_launch(5);
+    if (a_cx) ars = lda;
+    launch_ozaki_prepass(OzPair{{{A, ars, aps, a_cx, m, k, ea, sla, kp, pa, 0, 0, 0, 0},
+                                 {B, brs, bps, 0, n, k, eb, slb, kp, pb, 0, 0, 0, 0}}},
+                         slices, st);
     CUtensorMap tma, tmb;
     CUresult r = make_tmap_planes(&tma, sla, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, k, m, slices, kp, kUM);
     if (r == CUDA_SUCCESS)
@@ -3449,23 +3461,9 @@ int ozaki_grouped_dev(const rb_gemm_problem* probs, size_t count, const void* co
         int8_t* slb = dplanes + j.off_b;
         size_t ars, aps, brs, bps;
         operand_views(j.ta, j.tb, j.lda, j.ldb, ars, aps, brs, bps);
-        const int kb = (j.k + 1023) / 1024, k32 = (j.k + 31) / 32;
-        const int skb = static_cast<int>((j.kp + kTile - 1) / kTile);
-        const struct { const double* x; size_t rs, ps; int R; int* e; int8_t* out; } od[2] = {
-            {j.a, ars, aps, j.m, ea, sla}, {j.b, brs, bps, j.n, eb, slb}};
-        for (int h = 0; h < 2; ++h) {
-            OzOperand& o = ops[2 * i + h];
-            o.x = od[h].x; o.rs = od[h].rs; o.ps = od[h].ps;
-            o.R = od[h].R; o.K = j.k;
-            o.e = od[h].e; o.out = od[h].out;
-            o.kp = j.kp; o.plane = static_cast<size_t>(od[h].R) * j.kp;
-            o.exp_gx = (o.ps == 1) ? (o.R + 7) / 8 : (o.R + 255) / 256;
-            o.slice_gx = skb;
-            o.exp_start = exp_blocks;
-            o.slice_start = slice_blocks;
-            exp_blocks += o.exp_gx * ((o.ps == 1) ? kb : k32);
-            slice_blocks += skb * ((o.R + kTile - 1) / kTile);
-        }
+        ops[2 * i] = {j.a, ars, aps, 0, j.m, j.k, ea, sla, j.kp, static_cast<size_t>(j.m) * j.kp, 0, 0, 0, 0};
+        ops[2 * i + 1] = {j.b, brs, bps, 0, j.n, j.k, eb, slb, j.kp, static_cast<size_t>(j.n) * j.kp, 0, 0, 0, 0};
+        for (int h = 0; h < 2; ++h) oz_operand_blocks(&ops[2 * i + h], &exp_blocks, &slice_blocks);
         OzGroupEntry g{};  // 64-byte aligned here; copied into the image below
         r = make_tmap_planes(&g.tmA, sla, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, j.k, j.m, slices, j.kp, kUM);
         if (r == CUDA_SUCCESS)
@@ -3697,17 +3695,9 @@ extern "C" rb_status rb_dgemm_ozaki_noalloc(rb_layout layout, rb_transpose trans
         int8_t* slb = sla + round_up(slices * pa, 256);
         size_t ars, aps, brs, bps;
         operand_views(cta, ctb, clda, cldb, ars, aps, brs, bps);
-        fill_int_kernel<<<64, 256, 0, st>>>(ea, M + N, kExpSentinel);
-        const int kb = (K + 1023) / 1024, k32 = (K + 31) / 32;
-        if (aps == 1) row_exp_kcontig_kernel<<<dim3((M + 7) / 8, kb), 256, 0, st>>>(ca, ars, M, K, ea);
-        else          row_exp_rcontig_kernel<<<dim3((M + 255) / 256, k32), 256, 0, st>>>(ca, aps, M, K, ea);
-        if (bps == 1) row_exp_kcontig_kernel<<<dim3((N + 7) / 8, kb), 256, 0, st>>>(cb, brs, N, K, eb);
-        else          row_exp_rcontig_kernel<<<dim3((N + 255) / 256, k32), 256, 0, st>>>(cb, bps, N, K, eb);
-        const dim3 ga((kp + kTile - 1) / kTile, (M + kTile - 1) / kTile);
-        const dim3 gb((kp + kTile - 1) / kTile, (N + kTile - 1) / kTile);
-        launch_ozaki_slices(ga, st, ca, ars, aps, 0, M, K, ea, slices, sla, kp, pa);
-        launch_ozaki_slices(gb, st, cb, brs, bps, 0, N, K, eb, slices, slb, kp, pb);
-        count_launch(5);
+        launch_ozaki_prepass(OzPair{{{ca, ars, aps, 0, M, K, ea, sla, kp, pa, 0, 0, 0, 0},
+                                     {cb, brs, bps, 0, N, K, eb, slb, kp, pb, 0, 0, 0, 0}}},
+                             slices, st);
         CUtensorMap tma, tmb;
         CUresult r = make_tmap_planes(&tma, sla, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, K, M, slices, kp, kUM);
         if (r == CUDA_SUCCESS) r = make_tmap_planes(&tmb, slb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, K, N, slices, kp, 256);
