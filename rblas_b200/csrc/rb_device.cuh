@@ -145,20 +145,12 @@ __device__ __forceinline__ bool elect_one() {
         : "=r"(p));
     return p != 0;
 }
-// Arrive once on CTA `rank`'s copy of `bar` (same offset in both CTAs).
-__device__ __forceinline__ void mbar_arrive_rank(uint64_t* bar, uint32_t rank) {
-    asm volatile(
-        "{\n\t.reg .b32 ra;\n\t"
-        "mapa.shared::cluster.u32 ra, %0, %1;\n\t"
-        "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}" ::"r"(smem_u32(bar)),
-        "r"(rank)
-        : "memory");
-}
-// The same without the release, for an arrival with no memory write of this
-// thread to publish: TMEM columns handed over after tcgen05.wait::ld, or the
-// word that a TMA stage (written by the async proxy before its barrier's phase
-// completed) has landed. (A cluster-scope release first waits for outstanding
-// stores, ~1000 clocks and more beside an epilogue's.)
+// Arrive once on CTA `rank`'s copy of `bar` (same offset in both CTAs), without
+// release semantics: for an arrival with no memory write of this thread to
+// publish -- TMEM columns handed over after tcgen05.wait::ld or ::st, or the word
+// that a stage has landed here (written by the async proxy, or by threads whose
+// arrivals completed its barrier's phase). A cluster-scope release first waits
+// for outstanding stores, ~1000 clocks and more beside an epilogue's.
 __device__ __forceinline__ void mbar_arrive_rank_relaxed(uint64_t* bar, uint32_t rank) {
     asm volatile(
         "{\n\t.reg .b32 ra;\n\t"
