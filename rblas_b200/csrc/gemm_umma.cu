@@ -387,14 +387,15 @@ __global__ void __launch_bounds__(UCfg<MODE>::THREADS, 1)
 // products. The hi planes then outlive the others of their stage and have a
 // ring of their own. Within each accumulator the products keep umma_body's
 // order, so the results are its bits.
-// Per CTA: warp 0 TMA producer; warp 1 TMEM owner and, in the even CTA, MMA
-// issuer (in the odd one it passes on to the even CTA that a stage has
-// landed); warps 2..17 epilogue (four per TMEM lane quarter, 64 columns each).
+// Per CTA: warp 0 TMA producer (both CTAs' loads of a stage complete on the even
+// CTA's barrier); warp 1 TMEM owner and, in the even CTA, MMA issuer; warps
+// 2..17 epilogue (four per TMEM lane quarter, 64 columns each).
 // 8192^3, us a call (split pass included), 128 x 128 tiles -> pairs: 3xBF16
-// 3316 -> 2404, BF16X6 5256 -> 4482; the GEMMs then run at 1.48 and 1.55
-// PFLOP/s of bf16 products (cuBLAS's burst 1.68), held by the power cap (SM
-// clock 1.55 GHz). A cluster-scope release in the epilogue's arrival, which
-// waits for the thread's stores, had cost BF16X6 850 us of that.
+// 3316 -> 2319, BF16X6 5256 -> 4320; held by the power cap (SM clock 1.55 GHz).
+// A cluster-scope release in the epilogue's arrival, which waits for the
+// thread's stores, cost BF16X6 850 us; a word passed on by the odd CTA that its
+// stage has landed, in place of loads that complete on the even CTA's barrier,
+// 160 (without a release, which cost more still, it ordered nothing).
 // ------------------------------------------------------------------------------
 // KB: K bytes per stage row. Ring H holds the hi planes (HP of them per
 // stage; every plane for 3xBF16), ring L the others.
@@ -415,13 +416,13 @@ static_assert(pair_smem_bytes<kModeBf16x3>() <= 232448 && pair_smem_bytes<kModeB
               "the pair kernels' rings must fit one CTA's shared memory");
 
 struct PairBar {
-    uint64_t h_full[6], h_empty[6];
+    uint64_t h_full[6], h_empty[6];  // (full: even CTA, a stage of both CTAs has landed)
     uint64_t l_full[4], l_empty[4];
-    uint64_t peer_full[4];  // even CTA: the odd CTA's stage has landed
     uint64_t acc_full[2];
     uint64_t acc_empty[2];  // even CTA: both CTAs' epilogue warps
     uint64_t drain;
     uint32_t tmem_base;
+    PairExit exit;
 };
 static_assert(sizeof(PairBar) <= kPairBarBytes, "shared memory reserved for the pair kernels' barriers");
 
@@ -443,12 +444,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     constexpr int HSTAGE = 2 * HP * PL;     // A's planes, then B's
     constexpr int LSTAGE = 2 * Pc::LP * PL;
     constexpr bool TWO = LS > 0;            // two rings
-    constexpr int PS = TWO ? LS : HS;       // slots of peer_full
     constexpr int SUB = kRowBytes / KB;     // stages per 64-element K tile
     constexpr int KSTEPS = KB / 32;
     constexpr uint32_t IDESC = umma_idesc(1, 1, 256, kPairN);  // f32 <- bf16
     constexpr bool SPLIT_ACC = (MODE == kModeBf16x6);
-    static_assert(Cfg::NB == NP && HP + Pc::LP == NP && HS <= 6 && LS <= 4 && PS <= 4 && SPLIT_ACC == TWO, "rings");
+    static_assert(Cfg::NB == NP && HP + Pc::LP == NP && HS <= 6 && LS <= 4 && SPLIT_ACC == TWO, "rings");
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -458,19 +458,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     const uint32_t rank = cluster_rank();
     if (threadIdx.x == 0) {
         for (int s = 0; s < HS; ++s) {
-            mbar_init(&bar->h_full[s], 1);
+            mbar_init(&bar->h_full[s], 2);
             mbar_init(&bar->h_empty[s], 1);
         }
         for (int s = 0; s < 4; ++s) {
-            mbar_init(&bar->l_full[s], 1);
+            mbar_init(&bar->l_full[s], 2);
             mbar_init(&bar->l_empty[s], 1);
-            mbar_init(&bar->peer_full[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&bar->acc_full[b], 1);
             mbar_init(&bar->acc_empty[b], 2 * kPairEpiWarps);
         }
         mbar_init(&bar->drain, 1);
+        bar->exit = PairExit{};
         fence_barrier_init();
     }
     if (warp == 1) tmem_alloc_pair(&bar->tmem_base, 512);
@@ -501,11 +501,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
                     break;
                 }
                 uint8_t* sh = smem + hs * HSTAGE;
-                mbar_arrive_expect_tx(&bar->h_full[hs], HSTAGE);
+                const uint32_t hf = cluster_addr(&bar->h_full[hs], 0);
+                mbar_arrive_expect_tx_cluster(hf, HSTAGE);
 #pragma unroll
-                for (int q = 0; q < HP; ++q) tma_load_3d(sh + q * PL, &tmA, &bar->h_full[hs], k0, m0, q);
+                for (int q = 0; q < HP; ++q) tma_load_3d_pair(sh + q * PL, &tmA, hf, k0, m0, q);
 #pragma unroll
-                for (int q = 0; q < HP; ++q) tma_load_3d(sh + (HP + q) * PL, &tmB, &bar->h_full[hs], k0, n0, q);
+                for (int q = 0; q < HP; ++q) tma_load_3d_pair(sh + (HP + q) * PL, &tmB, hf, k0, n0, q);
                 ++nh;
                 if constexpr (TWO) {
                     const uint32_t ls = nl % LS;
@@ -514,49 +515,27 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
                         break;
                     }
                     uint8_t* sl = lring + ls * LSTAGE;
-                    mbar_arrive_expect_tx(&bar->l_full[ls], LSTAGE);
+                    const uint32_t lf = cluster_addr(&bar->l_full[ls], 0);
+                    mbar_arrive_expect_tx_cluster(lf, LSTAGE);
 #pragma unroll
-                    for (int q = 0; q < Pc::LP; ++q) tma_load_3d(sl + q * PL, &tmA, &bar->l_full[ls], k0, m0, HP + q);
+                    for (int q = 0; q < Pc::LP; ++q) tma_load_3d_pair(sl + q * PL, &tmA, lf, k0, m0, HP + q);
 #pragma unroll
                     for (int q = 0; q < Pc::LP; ++q)
-                        tma_load_3d(sl + (Pc::LP + q) * PL, &tmB, &bar->l_full[ls], k0, n0, HP + q);
+                        tma_load_3d_pair(sl + (Pc::LP + q) * PL, &tmB, lf, k0, n0, HP + q);
                     ++nl;
                 }
             }
         }
-        if (!ok) {  // this CTA's copies land before it exits
-            for (uint32_t j = nh > (uint32_t)HS ? nh - HS : 0; j < nh; ++j)
-                mbar_wait_drain(&bar->h_full[j % HS], (j / HS) & 1);
-            if constexpr (TWO)
-                for (uint32_t j = nl > (uint32_t)LS ? nl - LS : 0; j < nl; ++j)
-                    mbar_wait_drain(&bar->l_full[j % LS], (j / LS) & 1);
-        }
-    } else if (warp == 1 && lane == 0 && rank == 1) {
-        // ------------------- odd CTA: landed stages, told to the even one -------------------
-        uint32_t it = 0;
-        for (int item = first; ok && item < items; item += step)
-            for (int kt = 0; kt < stages; ++kt, ++it) {
-                if (!mbar_wait(&bar->h_full[it % HS], (it / HS) & 1, err, 0x222)) {
-                    ok = false;
-                    break;
-                }
-                if constexpr (TWO) {
-                    if (!mbar_wait(&bar->l_full[it % LS], (it / LS) & 1, err, 0x22a)) {
-                        ok = false;
-                        break;
-                    }
-                }
-                mbar_arrive_rank_relaxed(&bar->peer_full[it % PS], 0);
-            }
-    } else if (warp == 1 && lane == 0) {
+        st_cluster(&bar->exit.issued[0][rank], 0, nh);
+        st_cluster(&bar->exit.issued[1][rank], 0, nl);
+    } else if (warp == 1 && lane == 0 && rank == 0) {
         // ------------------------- even CTA: MMA issuer -------------------------
         uint32_t it = 0, uc = 0;
         auto landed = [&](uint32_t i) -> bool {  // stage i, in both CTAs
-            if (!mbar_wait(&bar->h_full[i % HS], (i / HS) & 1, err, 0x223)) return false;
+            if (!mbar_wait_cluster(&bar->h_full[i % HS], (i / HS) & 1, err, 0x223)) return false;
             if constexpr (TWO) {
-                if (!mbar_wait(&bar->l_full[i % LS], (i / LS) & 1, err, 0x22b)) return false;
+                if (!mbar_wait_cluster(&bar->l_full[i % LS], (i / LS) & 1, err, 0x22b)) return false;
             }
-            if (!mbar_wait_cluster(&bar->peer_full[i % PS], (i / PS) & 1, err, 0x224)) return false;
             tc_fence_after();
             return true;
         };
@@ -702,9 +681,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
         }
     }
 
+    if (!ok) pair_fail(&bar->exit);
     tc_fence_before();
     __syncthreads();
     cluster_sync();  // no CTA leaves while the other may still reach its memory
+    if (bar->exit.failed) {  // in both CTAs
+        if (rank == 0 && threadIdx.x == 0) {
+            pair_drain(bar->h_full, HS, bar->exit.issued[0]);
+            if constexpr (TWO) pair_drain(bar->l_full, LS, bar->exit.issued[1]);
+        }
+        cluster_sync();
+    }
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc_pair(tmem_base, 512);
@@ -732,17 +719,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 // columns to each CTA.
 // Rings: A's f32 tiles (released as soon as the splitters hold them in
 // registers); stages of A's planes and B's planes, released together by the
-// MMAs' one commit.
+// MMAs' one commit. B's loads and the splitter warps of both CTAs arrive on the
+// even CTA's barriers.
 // Warps: 0 producer of A's tiles; 1 TMEM owner and, in the even CTA, MMA issuer
-// for both (the odd one's tells it of full stages); 2 producer of B's planes;
-// 3..18 splitter and epilogue: tile row quarter * 32 + lane (quarter = warp % 4,
-// the TMEM lanes the warp may use) in both roles; K values 32 half .. + 31 of
-// every second K tile to split (so that one tile's loads overlap the other's
-// stores), columns 32 part .. + 31 of the tile to promote and write.
+// for both; 2 producer of B's planes; 3..18 splitter and epilogue: tile row
+// quarter * 32 + lane (quarter = warp % 4, the TMEM lanes the warp may use) in
+// both roles; K values 32 half .. + 31 of every second K tile to split (so that
+// one tile's loads overlap the other's stores), columns 32 part .. + 31 of the
+// tile to promote and write.
 // Bound: A's bytes from memory. 65536 x 128 x 8192 back to back, 3xBF16: 430 us
-// (A at 5.1 TB/s, its four waves 86 % full), BF16X6 693 (24 MMAs of 64 clocks a
+// (A at 5.1 TB/s, its four waves 86 % full), BF16X6 765 (24 MMAs of 64 clocks a
 // K tile); on single CTAs with planes in shared memory, one splitter group and
 // one issuing lane, 634 and 900: the issuing lane took ~110 clocks an MMA.
+// BF16X6's planes of the odd CTA are read by the even one's MMAs, so its
+// splitters release them to the cluster, ~1000 clocks that two stages hide only
+// in part: each half of a stage's K is handed over and freed by itself (805
+// whole).
 // Splitting with 16 warps a tile instead of two groups of 8: 523 and 768. Tiles
 // of 112 rows, which fill the fourth wave, took longer (471): their columns
 // start inside 128-byte lines.
@@ -766,11 +758,15 @@ static_assert(fz_smem_bytes<kModeBf16x3>() <= 232448 && fz_smem_bytes<kModeBf16x
 
 struct FzBar {
     uint64_t f_full[4], f_empty[4];  // A's f32 tiles
-    uint64_t full[4];                // plane stages: A's split here and B's landed
-    uint64_t peer_full[4];           // (even CTA) the same of the odd one's
-    uint64_t empty[4];               // the pair's MMAs have read them
+    uint64_t a_full[4];              // plane stages (even CTA): both CTAs' splits of A are there (each half of K by itself
+                                     // where the planes are in shared memory)
+    uint64_t b_full[4];              // and loads of B
+    uint64_t empty[4];               // the pair's MMAs have read them (of A, the first half of K: empty0)
+    uint64_t empty0[2];
     uint64_t acc_full[2], acc_empty[2], drain;
     uint32_t tmem_base;
+    uint32_t issued_f;  // f32 tiles that this CTA's producer issued
+    PairExit exit;
 };
 static_assert(sizeof(FzBar) <= 256, "the fused kernels reserve 256 bytes of shared memory for their barriers");
 
@@ -786,6 +782,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFzThreads, 1)
     // every phase (copies may land out of order)
     static_assert(FS % 2 == 0 && RS % 2 == 0, "even rings");
     constexpr int KSTEPS = 4;
+    constexpr int KH = A_TMEM ? 1 : 2;  // parts of a stage that A's planes are handed over in
+    static_assert(RS * KH <= 4 && (KH == 1 || RS <= 2), "FzBar holds the parts' barriers");
     constexpr uint32_t IDESC = umma_idesc(1, 1, 256, kFzN);  // f32 <- bf16
     // BF16X6 keeps hi*hi in an accumulator of its own, as umma_body does
     constexpr bool SPLIT_ACC = (MODE == kModeBf16x6);
@@ -808,15 +806,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFzThreads, 1)
             mbar_init(&bar->f_empty[s], kFzEpiWarps / 2);
         }
         for (int s = 0; s < RS; ++s) {
-            mbar_init(&bar->full[s], 1 + kFzEpiWarps / 2);
-            mbar_init(&bar->peer_full[s], 1);
+            for (int h = 0; h < KH; ++h) mbar_init(&bar->a_full[s * KH + h], 2 * (kFzEpiWarps / 2) / KH);
+            mbar_init(&bar->b_full[s], 2);
             mbar_init(&bar->empty[s], 1);
+            if (KH == 2) mbar_init(&bar->empty0[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&bar->acc_full[b], 1);
             mbar_init(&bar->acc_empty[b], 2 * kFzEpiWarps);
         }
         mbar_init(&bar->drain, 1);
+        bar->exit = PairExit{};
         fence_barrier_init();
     }
     if (warp == 1) tmem_alloc_pair(&bar->tmem_base, 512);
@@ -850,10 +850,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFzThreads, 1)
                 }
             }
         }
-        if (!ok) {  // this CTA's copies land before it exits
-            for (uint32_t j = it > (uint32_t)FS ? it - FS : 0; j < it; ++j)
-                mbar_wait_drain(&bar->f_full[j % FS], (j / FS) & 1);
-        }
+        bar->issued_f = it;
     } else if (warp == 2 && lane == 0) {
         prefetch_tmap(&tmB);
         uint32_t it = 0, rs = 0, ph = 1;
@@ -866,24 +863,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFzThreads, 1)
                     ok = false;
                     break;
                 }
-                mbar_arrive_expect_tx(&bar->full[rs], NP * kFzBTile);
+                const uint32_t bf = cluster_addr(&bar->b_full[rs], 0);
+                mbar_arrive_expect_tx_cluster(bf, NP * kFzBTile);
 #pragma unroll
-                for (int q = 0; q < NP; ++q)
-                    tma_load_3d(bps + (rs * NP + q) * kFzBTile, &tmB, &bar->full[rs], kt * 64, n0, q);
+                for (int q = 0; q < NP; ++q) tma_load_3d_pair(bps + (rs * NP + q) * kFzBTile, &tmB, bf, kt * 64, n0, q);
                 if (++rs == RS) {
                     rs = 0;
                     ph ^= 1;
                 }
             }
         }
-        // this CTA's copies land before it exits (a stage whose split of A does
-        // not come ends the wait by its time limit)
-        if (!ok) {
-            for (uint32_t j = it > (uint32_t)RS ? it - RS : 0; j < it; ++j)
-                if (!mbar_wait_drain(&bar->full[j % RS], (j / RS) & 1)) break;
-        }
-    } else if (warp == 1) {
-        // ---------- odd CTA: full stages, told to the even one; even CTA: MMA issuer ----------
+        st_cluster(&bar->exit.issued[0][rank], 0, it);
+    } else if (warp == 1 && rank == 0) {
+        // ------------------------- even CTA: MMA issuer -------------------------
         // (the whole warp runs the loop, one lane issues: see elect_one)
         const bool lead = elect_one();
         const uint64_t d0 = sw128_kmajor_desc(smem_u32(bps));  // (see umma_pair_kernel on descriptors)
@@ -894,32 +886,28 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFzThreads, 1)
             for (int u = 0; ok && u < p.kchunks; ++u, ++uc) {
                 const int kt0 = u * kFzUnit, kt1 = min(p.num_kt, kt0 + kFzUnit);
                 const uint32_t b = uc & 1;
-                if (rank == 0) {
-                    if (uc >= 2) ok = mbar_wait_cluster(&bar->acc_empty[b], ((uc >> 1) - 1) & 1, err, 0x213);
-                    if (!__all_sync(0xffffffffu, ok)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
+                if (uc >= 2) ok = mbar_wait_cluster(&bar->acc_empty[b], ((uc >> 1) - 1) & 1, err, 0x213);
+                if (!__all_sync(0xffffffffu, ok)) {
+                    ok = false;
+                    break;
                 }
+                tc_fence_after();
                 const uint32_t d_tmem = tmem_base + b * ACC_COLS;         // the products (all, or all but hi*hi)
                 const uint32_t d_big = SPLIT_ACC ? d_tmem + kFzN : d_tmem;  // hi*hi
                 for (int kt = kt0; kt < kt1; ++kt) {
-                    ok = mbar_wait_inline(&bar->full[rs], ph, err, 0x214);
-                    if (rank == 0 && ok) ok = mbar_wait_cluster(&bar->peer_full[rs], ph, err, 0x215);
-                    if (!__all_sync(0xffffffffu, ok)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    if (rank != 0) {
-                        tc_fence_before();
-                        if (lead) mbar_arrive_rank_relaxed(&bar->peer_full[rs], 0);
-                    } else {
-                        const uint32_t sb = b_lo + rs * (NP * kFzBTile / 16), sa = a_lo + rs * (NP * kATile / 16);
-                        const uint32_t ta = tmem_base + A_COL + rs * (NP * 32);
+                    ok = mbar_wait_cluster(&bar->b_full[rs], ph, err, 0x214);
+                    const uint32_t sb = b_lo + rs * (NP * kFzBTile / 16), sa = a_lo + rs * (NP * kATile / 16);
+                    const uint32_t ta = tmem_base + A_COL + rs * (NP * 32);
 #pragma unroll
-                        for (int kk = 0; kk < KSTEPS; ++kk)
+                    for (int h = 0; h < KH; ++h) {
+                        if (ok) ok = mbar_wait_cluster(&bar->a_full[rs * KH + h], ph, err, 0x215);
+                        if (!__all_sync(0xffffffffu, ok)) {
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after();
+#pragma unroll
+                        for (int kk = h * (KSTEPS / KH); kk < (h + 1) * (KSTEPS / KH); ++kk)
 #pragma unroll
                             for (int q = 0; q < Cfg::NPROD; ++q) {
                                 const bool big = SPLIT_ACC && q == Cfg::NPROD - 1;
@@ -933,22 +921,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFzThreads, 1)
                                         umma_f16_pair(d, d_hi | (sa + Cfg::pa(q) * (kATile / 16) + 2 * kk), db, IDESC, acc);
                                 }
                             }
-                        if (lead) tc_commit_pair(&bar->empty[rs]);  // free, in both CTAs, once these MMAs complete
+                        // free, in both CTAs, once these MMAs complete
+                        if (lead) tc_commit_pair(h + 1 < KH ? &bar->empty0[rs] : &bar->empty[rs]);
                     }
+                    if (!ok) break;
                     if (++rs == RS) {
                         rs = 0;
                         ph ^= 1;
                     }
                 }
-                if (ok && rank == 0 && lead) tc_commit_pair(&bar->acc_full[b]);
+                if (ok && lead) tc_commit_pair(&bar->acc_full[b]);
             }
         }
         // nothing of ours is in flight before TMEM is released (arrives on the
         // odd CTA's copy too, which nobody waits on)
-        if (rank == 0) {
-            if (lead) tc_commit_pair(&bar->drain);
-            mbar_wait_drain(&bar->drain, 0);
-        }
+        if (lead) tc_commit_pair(&bar->drain);
+        mbar_wait_drain(&bar->drain, 0);
     } else if (warp >= 3) {
         // ------------------------- splitter and epilogue -------------------------
         constexpr int HC = kFzN / 4;  // columns per warp
@@ -968,7 +956,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFzThreads, 1)
             // add unit `promoted`'s FP32 partial (TMEM) into sum, as umma_body does
             auto promote = [&]() -> bool {
                 const uint32_t b = uc & 1;
-                const bool got = mbar_wait_inline(&bar->acc_full[b], (uc >> 1) & 1, err, 0x216);
+                const bool got = mbar_wait_cluster(&bar->acc_full[b], (uc >> 1) & 1, err, 0x216);
                 if (!__all_sync(0xffffffffu, got)) return false;
                 tc_fence_after();
                 // the smaller products first, then hi*hi (SPLIT_ACC)
@@ -1006,7 +994,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFzThreads, 1)
                 // the f32 stage is free: every lane's reads are done
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&bar->f_empty[fs]);
-                got = mbar_wait_inline(&bar->empty[rs], (i / RS + 1) & 1, err, 0x217);  // (a fresh slot's wait passes)
+                // (a fresh slot's wait passes)
+                got = mbar_wait_cluster(half + 1 < KH ? &bar->empty0[rs] : &bar->empty[rs], (i / RS + 1) & 1, err, 0x217);
                 if (!__all_sync(0xffffffffu, got)) {
                     ok = false;
                     break;
@@ -1056,7 +1045,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFzThreads, 1)
                     fence_proxy_async_smem();  // the planes' generic stores, visible to the tensor cores
                 }
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&bar->full[rs]);
+                if (lane == 0) {
+                    if constexpr (A_TMEM) mbar_arrive_rank_relaxed(&bar->a_full[rs], 0);
+                    else if (rank == 0)   mbar_arrive(&bar->a_full[rs * KH + half]);
+                    else                  mbar_arrive_rank_release(&bar->a_full[rs * KH + half], 0);
+                }
                 // once this group's part of unit u is split, unit u - 1 is promoted:
                 // the MMAs of unit u + 1 wait for that buffer
                 if (kt >= kFzUnit && !promote()) {
@@ -1092,9 +1085,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFzThreads, 1)
         }
     }
 
+    if (!ok) pair_fail(&bar->exit);
     tc_fence_before();
     __syncthreads();
     cluster_sync();  // no CTA leaves while the other may still reach its memory
+    if (bar->exit.failed) {  // in both CTAs
+        if (threadIdx.x == 0)  // this CTA's own tiles of A
+            for (uint32_t n = bar->issued_f, j = n > (uint32_t)FS ? n - FS : 0; j < n; ++j)
+                mbar_wait_drain(&bar->f_full[j % FS], (j / FS) & 1);
+        if (rank == 0 && threadIdx.x == 0) pair_drain(bar->b_full, RS, bar->exit.issued[0]);
+        cluster_sync();
+    }
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc_pair(tmem_base, 512);
@@ -1649,9 +1650,9 @@ __global__ void __launch_bounds__(kOzThreads, 1)
 // Tail: the tiles of the partial last wave run as items of one group over a
 // part of K each, which write the exact sums S_d0 * 256 + S_d1 to workspace
 // planes; ozaki_pair_reduce_kernel adds the parts (exactly) and folds.
-// Warps per CTA: 0 TMA producer, 1 TMEM owner and MMA issuer (even CTA; odd:
-// passes on that a stage landed), 2.. epilogue (two or four per TMEM lane
-// quarter).
+// Warps per CTA: 0 TMA producer (both CTAs' loads of a stage complete on the even
+// CTA's barrier), 1 TMEM owner and, in the even CTA, MMA issuer, 2.. epilogue
+// (two or four per TMEM lane quarter).
 // ------------------------------------------------------------------------------
 constexpr int kPzN = 128;
 // Epilogue warps EW: 8 (64 columns each) for one problem, 16 (32 columns) in
@@ -1672,10 +1673,11 @@ constexpr int kPzSmem = kPzAS * kATile + kPzBS * kPzBTile + 512 + kPzTabs + 1024
 static_assert(kPzSmem <= 232448, "the pair kernel's rings must fit one CTA's shared memory");
 
 struct PzBar {
-    uint64_t full[kPzAS], done[kPzAS];  // stage landed; its MMAs complete
-    uint64_t peer_full[kPzAS];          // even CTA: the odd CTA's stage has landed
+    uint64_t full[kPzAS];  // even CTA: a stage of both CTAs has landed
+    uint64_t done[kPzAS];  // its MMAs are complete
     uint64_t acc_full, acc_empty, drain;
     uint32_t tmem_base;
+    PairExit exit;
 };
 static_assert(sizeof(PzBar) <= 512, "shared memory reserved for the pair kernel's barriers");
 
@@ -1787,13 +1789,13 @@ __device__ __forceinline__ void ozaki_pair_body(const Src& src) {
     const uint32_t rank = cluster_rank();
     if (threadIdx.x == 0) {
         for (int i = 0; i < AS; ++i) {
-            mbar_init(&bar->full[i], 1);
+            mbar_init(&bar->full[i], 2);
             mbar_init(&bar->done[i], 1);
-            mbar_init(&bar->peer_full[i], 1);
         }
         mbar_init(&bar->acc_full, 1);
         mbar_init(&bar->acc_empty, 2 * EW);
         mbar_init(&bar->drain, 1);
+        bar->exit = PairExit{};
         fence_barrier_init();
     }
     if (warp == 1) tmem_alloc_pair(&bar->tmem_base, 512);
@@ -1833,18 +1835,16 @@ __device__ __forceinline__ void ozaki_pair_body(const Src& src) {
                             ok = false;
                             break;
                         }
-                        mbar_arrive_expect_tx(&bar->full[as], kATile + kPzBTile);
-                        tma_load_3d(smem + as * kATile, w.ta, &bar->full[as], kt * 128, m0, top - st);
-                        tma_load_3d(bring + bs * kPzBTile, w.tb, &bar->full[as], kt * 128, n0, st);
+                        const uint32_t full = cluster_addr(&bar->full[as], 0);
+                        mbar_arrive_expect_tx_cluster(full, kATile + kPzBTile);
+                        tma_load_3d_pair(smem + as * kATile, w.ta, full, kt * 128, m0, top - st);
+                        tma_load_3d_pair(bring + bs * kPzBTile, w.tb, full, kt * 128, n0, st);
                     }
             }
         }
-        if (!ok) {  // this CTA's copies land before it exits
-            for (uint32_t j = it > (uint32_t)AS ? it - AS : 0; j < it; ++j)
-                mbar_wait_drain(&bar->full[j % AS], (j / AS) & 1);
-        }
-    } else if (warp == 1) {
-        // ---------- odd CTA: landed stages, told to the even one; even CTA: MMA issuer ----------
+        st_cluster(&bar->exit.issued[0][rank], 0, it);
+    } else if (warp == 1 && rank == 0) {
+        // ------------------------- even CTA: MMA issuer -------------------------
         // (the whole warp runs the loop, one lane issues: see elect_one)
         const bool lead = elect_one();
         const uint64_t d0 = sw128_kmajor_desc(smem_u32(smem));  // (see umma_pair_kernel on descriptors)
@@ -1873,42 +1873,32 @@ __device__ __forceinline__ void ozaki_pair_body(const Src& src) {
                 int kt0, kt1;
                 pz_kt(w, u, groups, kt0, kt1);
                 const uint32_t d = tmem_base + (nd - 1) * kPzN;
-                if (rank == 0) {
-                    if (uc >= 1 &&
-                        !__all_sync(0xffffffffu, mbar_wait_cluster(&bar->acc_empty, (uc - 1) & 1, err, 0x313))) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
+                if (uc >= 1 &&
+                    !__all_sync(0xffffffffu, mbar_wait_cluster(&bar->acc_empty, (uc - 1) & 1, err, 0x313))) {
+                    ok = false;
+                    break;
                 }
+                tc_fence_after();
                 for (int kt = kt0; ok && kt < kt1; ++kt)
                     for (int st = 0; st <= top; ++st) {
                         if (!__all_sync(0xffffffffu, mbar_wait_cluster(&bar->full[as], ph, err, 0x314))) {
                             ok = false;
                             break;
                         }
-                        if (rank == 1) {
-                            if (lead) mbar_arrive_rank_relaxed(&bar->peer_full[as], 0);
-                        } else {
-                            if (!__all_sync(0xffffffffu, mbar_wait_cluster(&bar->peer_full[as], ph, err, 0x316))) {
-                                ok = false;
-                                break;
-                            }
-                            tc_fence_after();
-                            const uint32_t a = a_lo + as * (kATile / 16);
-                            uint32_t b[4];
+                        tc_fence_after();
+                        const uint32_t a = a_lo + as * (kATile / 16);
+                        uint32_t b[4];
 #pragma unroll
-                            for (int l = 0; l < 4; ++l)
-                                b[l] = b_lo + (bs >= (uint32_t)l ? bs - l : bs + BS - l) * (kPzBTile / 16);
-                            const int nl = min(st + 1, nd);
-                            const bool fresh = kt == kt0 && st == nl - 1;
-                            if (lead) {
-                                if (nl == 4)      stage(std::integral_constant<int, 4>{}, a, b, d, fresh);
-                                else if (nl == 3) stage(std::integral_constant<int, 3>{}, a, b, d, fresh);
-                                else if (nl == 2) stage(std::integral_constant<int, 2>{}, a, b, d, fresh);
-                                else              stage(std::integral_constant<int, 1>{}, a, b, d, fresh);
-                                tc_commit_pair(&bar->done[as]);
-                            }
+                        for (int l = 0; l < 4; ++l)
+                            b[l] = b_lo + (bs >= (uint32_t)l ? bs - l : bs + BS - l) * (kPzBTile / 16);
+                        const int nl = min(st + 1, nd);
+                        const bool fresh = kt == kt0 && st == nl - 1;
+                        if (lead) {
+                            if (nl == 4)      stage(std::integral_constant<int, 4>{}, a, b, d, fresh);
+                            else if (nl == 3) stage(std::integral_constant<int, 3>{}, a, b, d, fresh);
+                            else if (nl == 2) stage(std::integral_constant<int, 2>{}, a, b, d, fresh);
+                            else              stage(std::integral_constant<int, 1>{}, a, b, d, fresh);
+                            tc_commit_pair(&bar->done[as]);
                         }
                         if (++as == AS) {
                             as = 0;
@@ -1916,10 +1906,10 @@ __device__ __forceinline__ void ozaki_pair_body(const Src& src) {
                         }
                         if (++bs == BS) bs = 0;
                     }
-                if (ok && rank == 0 && lead) tc_commit_pair(&bar->acc_full);
+                if (ok && lead) tc_commit_pair(&bar->acc_full);
             }
         }
-        if (rank == 0 && lead) {  // nothing of ours is in flight before TMEM is released
+        if (lead) {  // nothing of ours is in flight before TMEM is released
             tc_commit_pair(&bar->drain);
             mbar_wait_drain(&bar->drain, 0);
         }
@@ -2060,9 +2050,14 @@ __device__ __forceinline__ void ozaki_pair_body(const Src& src) {
         }
     }
 
+    if (!ok) pair_fail(&bar->exit);
     tc_fence_before();
     __syncthreads();
     cluster_sync();  // no CTA leaves while the other may still reach its memory
+    if (bar->exit.failed) {  // in both CTAs
+        if (rank == 0 && threadIdx.x == 0) pair_drain(bar->full, AS, bar->exit.issued[0]);
+        cluster_sync();
+    }
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc_pair(tmem_base, 512);

@@ -145,19 +145,35 @@ __device__ __forceinline__ bool elect_one() {
         : "=r"(p));
     return p != 0;
 }
-// Arrive once on CTA `rank`'s copy of `bar` (same offset in both CTAs), without
-// release semantics: for an arrival with no memory write of this thread to
-// publish -- TMEM columns handed over after tcgen05.wait::ld or ::st, or the word
-// that a stage has landed here (written by the async proxy, or by threads whose
-// arrivals completed its barrier's phase). A cluster-scope release first waits
-// for outstanding stores, ~1000 clocks and more beside an epilogue's.
+// The shared::cluster address of CTA `rank`'s copy of p (same offset in both CTAs).
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
+    uint32_t ra;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(smem_u32(p)), "r"(rank));
+    return ra;
+}
+__device__ __forceinline__ void st_cluster(const uint32_t* p, uint32_t rank, uint32_t v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr(p, rank)), "r"(v) : "memory");
+}
+// Arrive once on CTA `rank`'s copy of `bar`. Two forms:
+// - relaxed: hands over TMEM columns only, after tcgen05.wait::ld or ::st and
+//   tcgen05.fence::before_thread_sync; the waiter's tcgen05.fence::after_thread_sync
+//   completes that order, and no release is needed for it. (A cluster-scope
+//   release first waits for outstanding stores, ~1000 clocks and more beside an
+//   epilogue's.)
+// - release: publishes shared memory that this thread's warp wrote (or saw
+//   written). Data that TMA writes needs neither: its loads complete on the
+//   waiting CTA's barrier themselves (tma_load_3d_pair).
 __device__ __forceinline__ void mbar_arrive_rank_relaxed(uint64_t* bar, uint32_t rank) {
-    asm volatile(
-        "{\n\t.reg .b32 ra;\n\t"
-        "mapa.shared::cluster.u32 ra, %0, %1;\n\t"
-        "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [ra];\n\t}" ::"r"(smem_u32(bar)),
-        "r"(rank)
-        : "memory");
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr(bar, rank)) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_rank_release(uint64_t* bar, uint32_t rank) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr(bar, rank)) : "memory");
+}
+// Arrive on a barrier of either CTA (cluster_addr) and add `bytes` to what its
+// phase waits for. Relaxed: the thread has written nothing.
+__device__ __forceinline__ void mbar_arrive_expect_tx_cluster(uint32_t bar_addr, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(bar_addr), "r"(bytes)
+                 : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
@@ -214,6 +230,42 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, u
         : "memory");
 }
 
+
+// The same into this CTA's shared memory, completing on a barrier of either CTA
+// of the pair (cluster_addr).
+__device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* map, uint32_t bar_addr,
+                                                 int32_t c0, int32_t c1, int32_t c2) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2"
+        " [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_addr), "r"(c0), "r"(c1), "r"(c2)
+        : "memory");
+}
+
+// What a pair needs to end safely when a wait gives up. A stage's loads of both
+// CTAs complete on the even CTA's barrier (two arrivals, each with its CTA's
+// bytes), so the even CTA waits for them; each producer leaves its number of
+// stages issued there, per ring.
+struct PairExit {
+    uint32_t failed;
+    uint32_t issued[2][2];  // [ring][CTA]
+};
+// Called by any thread that gives up; both CTAs read it after their cluster_sync.
+__device__ __forceinline__ void pair_fail(PairExit* x) {
+    st_cluster(&x->failed, 0, 1u);
+    st_cluster(&x->failed, 1, 1u);
+}
+// Even CTA, one thread: waits until every stage that either CTA issued has
+// landed, arriving in the place of a CTA that did not issue it.
+static __device__ __noinline__ void pair_drain(uint64_t* full, uint32_t stages, const uint32_t (&issued)[2]) {
+    const uint32_t end = issued[0] > issued[1] ? issued[0] : issued[1];
+    for (uint32_t j = end > stages ? end - stages : 0; j < end; ++j) {
+        uint64_t* bar = &full[j % stages];
+        for (int c = 0; c < 2; ++c)
+            if (j >= issued[c]) mbar_arrive(bar);
+        mbar_wait_drain(bar, (j / stages) & 1);
+    }
+}
 
 // ---- tcgen05 / TMEM --------------------------------------------------------------
 
