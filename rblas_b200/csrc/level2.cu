@@ -441,6 +441,13 @@ __global__ void __launch_bounds__(kL2Threads)
     }
 }
 
+// Whether [p, p + pn) and [q, q + qn) (elements) share memory.
+template <typename E>
+bool overlap(const E* p, size_t pn, const E* q, size_t qn) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p), b = reinterpret_cast<uintptr_t>(q);
+    return a < b + qn * sizeof(E) && b < a + pn * sizeof(E);
+}
+
 int blocks_for(long long n) { return static_cast<int>((n + kL2Threads - 1) / kL2Threads); }
 
 int fail(cudaError_t e, int32_t* ce) {
@@ -511,9 +518,14 @@ int gemv_dev(int layout, int trans, size_t m, size_t n, T ar, T ai, const T* A, 
         S = (R + chunk - 1) / chunk;
         grid = dim3(cb, S);
     }
+    // A single range writes y in the kernel that reads x and A: where y shares
+    // memory with either, its sums go through the workspace too.
+    const size_t lenx = tr ? m : n, ny = (leny - 1) * static_cast<size_t>(incy) + 1;
+    const bool through_ws = S > 1 || overlap<E>(yv, ny, xv, (lenx - 1) * static_cast<size_t>(incx) + 1) ||
+                            overlap<E>(yv, ny, Av, static_cast<size_t>(Cc - 1) * lda + static_cast<size_t>(R));
     E* ws = nullptr;
     cudaError_t e;
-    if (S > 1 && (e = scratch_alloc(&ws, static_cast<size_t>(S) * len * sizeof(E), st)) != cudaSuccess)
+    if (through_ws && (e = scratch_alloc(&ws, static_cast<size_t>(S) * len * sizeof(E), st)) != cudaSuccess)
         return fail(e, ce);
     const GemvOut<E> o{yv, incy, ea, eb, ws, len};
     if (split) {
@@ -535,7 +547,7 @@ int gemv_dev(int layout, int trans, size_t m, size_t n, T ar, T ai, const T* A, 
 #undef RB_DOT
     }
     count_launch();
-    if (S > 1) {
+    if (through_ws) {
         gemv_finalize<E><<<(len + 31) / 32, kL2Threads, 0, st>>>(o, S);
         count_launch();
     }
