@@ -18,14 +18,16 @@
 //     on timing.
 // Within one range the terms are added in rblas's order (fma(a, x, acc) for
 // real, acc + a*x with rblas's complex multiply for complex), so a NoTrans
-// column-major call of fewer than kSweepSplit columns reproduces rblas's gemv
-// exactly; other shapes differ from rblas's order within rounding.
+// column-major call of fewer than kSweepSplit columns, or of more than
+// kSweepFullRows rows, reproduces rblas's gemv exactly; other shapes differ from
+// rblas's order within rounding.
 // The rank-1 update computes each element as rblas does (alpha*x_i rounded,
 // then fma / complex multiply-add), so it matches rblas bit for bit.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 #include "../../include/rblas_b200.h"
 #include "rb_internal.h"
@@ -147,41 +149,52 @@ __device__ __forceinline__ void put(const GemvOut<E>& o, int i, int s, E acc) {
     else      finish_y(o.y + static_cast<long long>(i) * o.incy, acc, o.alpha, o.beta);
 }
 
-// y_r over few columns, in column order. A CTA covers
-// kSweepRows consecutive rows (each thread kRowsPerThread of them, 256 apart,
-// so every warp load stays one contiguous 256-byte run and the CTA reads
-// 8 KB contiguous per f64 column); the accumulators are independent.
+// Rows that a thread of the sweeps below and of the rank-1 updates takes, a CTA's
+// threads apart, so that every warp load stays one contiguous run.
 constexpr int kRowsPerThread = 4;
 constexpr int kSweepRows = kL2Threads * kRowsPerThread;
 
+// y_r in column order, a thread for four rows: few columns, or so many rows that
+// they fill the GPU. Bound by memory, with few loads in flight: in a whole tile
+// no test stands between them, so those of eight columns go out together, and
+// CTAs of two warps leave a short last wave. f64 1.3M x 100: 157 us (256 threads,
+// four columns, tests: 268; gemv_split_kernel, which is as good there and keeps
+// another order, 162); 1.3M x 20: 41 (62); f32 1.3M x 100: 105 (146; split 92).
+constexpr int kColThreads = 64;
+constexpr int kColRows = kColThreads * kRowsPerThread;
+
 template <typename E>
-__global__ void __launch_bounds__(kL2Threads)
+__global__ void __launch_bounds__(kColThreads)
     gemv_sweep_kernel(const E* __restrict__ A, size_t ld, int R, int C, const E* __restrict__ x, long long incx,
                       int conj, GemvOut<E> o) {
-    const int rbase = blockIdx.x * kSweepRows + threadIdx.x;
+    const int rbase = blockIdx.x * kColRows + threadIdx.x;
     E acc[kRowsPerThread];
     bool live[kRowsPerThread];
 #pragma unroll
     for (int q = 0; q < kRowsPerThread; ++q) {
         acc[q] = zero_el(static_cast<E*>(nullptr));
-        live[q] = rbase + q * kL2Threads < R;
+        live[q] = rbase + q * kColThreads < R;
     }
-#pragma unroll 4
-    for (int c = 0; c < C; ++c) {
-        const E xc = ld_el(x + static_cast<long long>(c) * incx);
-        const E* col = A + static_cast<size_t>(c) * ld + rbase;
+    auto columns = [&](auto whole) {
+#pragma unroll 8
+        for (int c = 0; c < C; ++c) {
+            const E xc = ld_el(x + static_cast<long long>(c) * incx);
+            const E* col = A + static_cast<size_t>(c) * ld + rbase;
 #pragma unroll
-        for (int q = 0; q < kRowsPerThread; ++q) {
-            if (live[q]) {
-                E v = ld_el(col + q * kL2Threads);
-                if (conj) v = conj_el(v);
-                acc[q] = mac(acc[q], v, xc);
+            for (int q = 0; q < kRowsPerThread; ++q) {
+                if (decltype(whole)::value || live[q]) {
+                    E v = ld_el(col + q * kColThreads);
+                    if (conj) v = conj_el(v);
+                    acc[q] = mac(acc[q], v, xc);
+                }
             }
         }
-    }
+    };
+    if (R - static_cast<int>(blockIdx.x) * kColRows >= kColRows) columns(std::true_type{});
+    else                                                             columns(std::false_type{});
 #pragma unroll
     for (int q = 0; q < kRowsPerThread; ++q)
-        if (live[q]) put(o, rbase + q * kL2Threads, 0, acc[q]);
+        if (live[q]) put(o, rbase + q * kColThreads, 0, acc[q]);
 }
 
 // Column dot: y_c over rows [r0, r1) of range s. The CTA takes two columns at
@@ -274,6 +287,9 @@ __global__ void __launch_bounds__(kL2Threads)
 // before; 256 x 16384: 98 -> 15).
 constexpr int kSweepPack = 2;
 constexpr int kSweepSplit = 32;  // fewer columns: gemv_sweep_kernel in one range, rblas's own order
+// More rows than these fill the GPU with four to a thread, and keep rblas's own
+// order too.
+constexpr int kSweepFullRows = 148 * 8 * kSweepRows - kSweepRows;
 constexpr int kSplitRows = 32 * kSweepPack;
 
 template <typename E>
@@ -501,7 +517,7 @@ int gemv_dev(int layout, int trans, size_t m, size_t n, T ar, T ai, const T* A, 
     // ranges (S) so that the grid fills the GPU, each with enough work
     int S = 1, chunk = 0;
     dim3 grid;
-    const bool split = sweep && Cc >= kSweepSplit;
+    const bool split = sweep && Cc >= kSweepSplit && R <= kSweepFullRows;
     const bool short_cols = !sweep && R <= kShortRows && Cc >= 148 * 4 * (kL2Threads / 32);
     if (split) {
         const int rb = (R + kSplitRows - 1) / kSplitRows;
@@ -510,7 +526,7 @@ int gemv_dev(int layout, int trans, size_t m, size_t n, T ar, T ai, const T* A, 
         S = (Cc + chunk - 1) / chunk;
         grid = dim3(rb, S);
     } else if (sweep) {
-        grid = dim3((R + kSweepRows - 1) / kSweepRows);
+        grid = dim3((R + kColRows - 1) / kColRows);
     } else {
         const int cols = short_cols ? kL2Threads / 32 : kDotCols, cb = (Cc + cols - 1) / cols;
         if (!short_cols) S = std::max(1, std::min((148 * 4 + cb - 1) / cb, R / 1024));
@@ -531,7 +547,7 @@ int gemv_dev(int layout, int trans, size_t m, size_t n, T ar, T ai, const T* A, 
     if (split) {
         gemv_split_kernel<E><<<grid, kL2Threads, 0, st>>>(Av, lda, R, Cc, xv, incx, conj, chunk, o);
     } else if (sweep) {
-        gemv_sweep_kernel<E><<<grid, kL2Threads, 0, st>>>(Av, lda, R, Cc, xv, incx, conj, o);
+        gemv_sweep_kernel<E><<<grid, kColThreads, 0, st>>>(Av, lda, R, Cc, xv, incx, conj, o);
     } else {
 #define RB_DOT(W, COLS, VA, VX) \
     gemv_dot_kernel<E, W, COLS, VA, VX><<<grid, kL2Threads, 0, st>>>(Av, lda, R, Cc, xv, incx, conj, chunk, o)
