@@ -210,11 +210,13 @@ constexpr int kShortRows = 1024;
 template <typename E, int W, int COLS, bool VA, bool VX>
 __global__ void __launch_bounds__(kL2Threads)
     gemv_dot_kernel(const E* __restrict__ A, size_t ld, int R, int C, const E* __restrict__ x, long long incx,
-                    int conj, int rchunk, GemvOut<E> o) {
+                    int conj, unsigned rchunk, GemvOut<E> o) {
     constexpr int V = kVecLen<E>, LANES = W * 32;
     const int t = threadIdx.x % LANES, s = blockIdx.y;
+    // rows are counted unsigned: an index past the last row may exceed INT_MAX
     const int c0 = (blockIdx.x * (kL2Threads / LANES) + threadIdx.x / LANES) * COLS;
-    const int r0 = s * rchunk, r1 = min(R, r0 + rchunk);  // rchunk: a multiple of V
+    const unsigned r0 = static_cast<unsigned>(s) * rchunk;  // rchunk: a multiple of V
+    const unsigned r1 = min(static_cast<unsigned>(R), r0 + rchunk);
     const E* a[COLS];
 #pragma unroll
     for (int q = 0; q < COLS; ++q) a[q] = A + static_cast<size_t>(min(c0 + q, C - 1)) * ld;
@@ -225,7 +227,7 @@ __global__ void __launch_bounds__(kL2Threads)
         for (int i = 0; i < V; ++i) acc[q][i] = zero_el(static_cast<E*>(nullptr));
     if (c0 < C) {
 #pragma unroll 2
-        for (int r = r0 + t * V; r + V <= r1; r += LANES * V) {
+        for (unsigned r = r0 + t * V; r + V <= r1; r += LANES * V) {
             Pack<E, V> v[COLS], xv;
 #pragma unroll
             for (int q = 0; q < COLS; ++q) v[q] = ld_pack<VA, V>(a[q] + r);
@@ -241,7 +243,7 @@ __global__ void __launch_bounds__(kL2Threads)
                 for (int i = 0; i < V; ++i)
                     acc[q][i] = mac(acc[q][i], conj ? conj_el(v[q].e[i]) : v[q].e[i], xv.e[i]);
         }
-        const int rl = r0 + (r1 - r0) / V * V + t;  // fewer than V rows are left
+        const unsigned rl = r0 + (r1 - r0) / V * V + t;  // fewer than V rows are left
         if (t < V && rl < r1) {
             const E xv = ld_el(x + static_cast<long long>(rl) * incx);
 #pragma unroll
@@ -295,11 +297,12 @@ constexpr int kSplitRows = 32 * kSweepPack;
 template <typename E>
 __global__ void __launch_bounds__(kL2Threads)
     gemv_split_kernel(const E* __restrict__ A, size_t ld, int R, int C, const E* __restrict__ x, long long incx,
-                      int conj, int cchunk, GemvOut<E> o) {
+                      int conj, unsigned cchunk, GemvOut<E> o) {
     constexpr int WARPS = kL2Threads / 32;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, s = blockIdx.y;
     const int rb = blockIdx.x * kSplitRows + lane;
-    const int c0 = s * cchunk, c1 = min(C, c0 + cchunk);
+    // (columns unsigned, as the rows of gemv_dot_kernel)
+    const unsigned c0 = static_cast<unsigned>(s) * cchunk, c1 = min(static_cast<unsigned>(C), c0 + cchunk);
     E acc[kSweepPack];
     bool live[kSweepPack];
 #pragma unroll
@@ -308,7 +311,7 @@ __global__ void __launch_bounds__(kL2Threads)
         live[q] = rb + q * 32 < R;
     }
 #pragma unroll 4
-    for (int c = c0 + warp; c < c1; c += WARPS) {
+    for (unsigned c = c0 + warp; c < c1; c += WARPS) {
         const E* col = A + static_cast<size_t>(c) * ld + rb;
         const E xc = ld_el(x + static_cast<long long>(c) * incx);
 #pragma unroll
@@ -515,24 +518,25 @@ int gemv_dev(int layout, int trans, size_t m, size_t n, T ar, T ai, const T* A, 
     const bool va = reinterpret_cast<uintptr_t>(A) % 16 == 0 && (lda * sizeof(E)) % 16 == 0;
     const bool vx = incx == 1 && reinterpret_cast<uintptr_t>(x) % 16 == 0;
     // ranges (S) so that the grid fills the GPU, each with enough work
-    int S = 1, chunk = 0;
+    long long S = 1, chunk = 0;
+    const long long rows = R, columns = Cc;
     dim3 grid;
     const bool split = sweep && Cc >= kSweepSplit && R <= kSweepFullRows;
     const bool short_cols = !sweep && R <= kShortRows && Cc >= 148 * 4 * (kL2Threads / 32);
     if (split) {
-        const int rb = (R + kSplitRows - 1) / kSplitRows;
-        S = std::max(1, std::min(148 * 8 / rb, Cc / 32));
-        chunk = (Cc + S - 1) / S;
-        S = (Cc + chunk - 1) / chunk;
-        grid = dim3(rb, S);
+        const long long rb = (rows + kSplitRows - 1) / kSplitRows;
+        S = std::max(1ll, std::min(148 * 8 / rb, columns / 32));
+        chunk = (columns + S - 1) / S;
+        S = (columns + chunk - 1) / chunk;
+        grid = dim3(static_cast<unsigned>(rb), static_cast<unsigned>(S));
     } else if (sweep) {
-        grid = dim3((R + kColRows - 1) / kColRows);
+        grid = dim3(static_cast<unsigned>((rows + kColRows - 1) / kColRows));
     } else {
-        const int cols = short_cols ? kL2Threads / 32 : kDotCols, cb = (Cc + cols - 1) / cols;
-        if (!short_cols) S = std::max(1, std::min((148 * 4 + cb - 1) / cb, R / 1024));
-        chunk = ((R + S - 1) / S + V - 1) / V * V;
-        S = (R + chunk - 1) / chunk;
-        grid = dim3(cb, S);
+        const long long cols = short_cols ? kL2Threads / 32 : kDotCols, cb = (columns + cols - 1) / cols;
+        if (!short_cols) S = std::max(1ll, std::min((148 * 4 + cb - 1) / cb, rows / 1024));
+        chunk = ((rows + S - 1) / S + V - 1) / V * V;
+        S = (rows + chunk - 1) / chunk;
+        grid = dim3(static_cast<unsigned>(cb), static_cast<unsigned>(S));
     }
     // A single range writes y in the kernel that reads x and A: where y shares
     // memory with either, its sums go through the workspace too.
@@ -545,12 +549,12 @@ int gemv_dev(int layout, int trans, size_t m, size_t n, T ar, T ai, const T* A, 
         return fail(e, ce);
     const GemvOut<E> o{yv, incy, ea, eb, ws, len};
     if (split) {
-        gemv_split_kernel<E><<<grid, kL2Threads, 0, st>>>(Av, lda, R, Cc, xv, incx, conj, chunk, o);
+        gemv_split_kernel<E><<<grid, kL2Threads, 0, st>>>(Av, lda, R, Cc, xv, incx, conj, static_cast<unsigned>(chunk), o);
     } else if (sweep) {
         gemv_sweep_kernel<E><<<grid, kColThreads, 0, st>>>(Av, lda, R, Cc, xv, incx, conj, o);
     } else {
 #define RB_DOT(W, COLS, VA, VX) \
-    gemv_dot_kernel<E, W, COLS, VA, VX><<<grid, kL2Threads, 0, st>>>(Av, lda, R, Cc, xv, incx, conj, chunk, o)
+    gemv_dot_kernel<E, W, COLS, VA, VX><<<grid, kL2Threads, 0, st>>>(Av, lda, R, Cc, xv, incx, conj, static_cast<unsigned>(chunk), o)
         if (short_cols) {
             if (va && vx)      RB_DOT(1, 1, true, true);
             else if (va)       RB_DOT(1, 1, true, false);
@@ -564,7 +568,7 @@ int gemv_dev(int layout, int trans, size_t m, size_t n, T ar, T ai, const T* A, 
     }
     count_launch();
     if (through_ws) {
-        gemv_finalize<E><<<(len + 31) / 32, kL2Threads, 0, st>>>(o, S);
+        gemv_finalize<E><<<static_cast<unsigned>((leny + 31) / 32), kL2Threads, 0, st>>>(o, static_cast<int>(S));
         count_launch();
     }
     e = cudaGetLastError();
