@@ -411,26 +411,33 @@ __device__ __forceinline__ void simt_epilogue(const SimtOut<T>& o, const T (&acc
         // DMMA accumulators: acc[mb * 2 + nb][q], placed by dmma_row / dmma_col
         const int g = lane >> 2, tq = lane & 3;
         const int wm0 = wm * 64, wn0 = wn * 16;
+        if (m0 + wm0 >= o.m || n0 + wn0 >= o.n) return;
+        // 16 C0 values requested at a time. Each store stands behind its own
+        // tests, and the reads behind one of beta: with one test of both (and the
+        // stores' addresses formed with the reads') beta == 0 took 2-3 % longer.
 #pragma unroll
-        for (int ig = 0; ig < 8; ig += 4) {  // 16 C0 values requested at a time
-            T cv[4][4];
+        for (int ig = 0; ig < 8; ig += 4) {
+            T cv[4][4] = {};
+            if (o.beta_mode != 0) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int r = m0 + wm0 + dmma_row<A_K>((ig + i) >> 1, q, g);
+                        const int cidx = n0 + wn0 + dmma_col<B_K>((ig + i) & 1, q, tq);
+                        cv[i][q] = simt_live(o, r, cidx) ? o.cin[r + static_cast<size_t>(cidx) * o.ldcin] : T(0);
+                    }
+            }
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const int r = m0 + wm0 + dmma_row<A_K>((ig + i) >> 1, q, g);
                     const int cidx = n0 + wn0 + dmma_col<B_K>((ig + i) & 1, q, tq);
-                    cv[i][q] = (o.beta_mode != 0 && simt_live(o, r, cidx))
-                                   ? o.cin[r + static_cast<size_t>(cidx) * o.ldcin] : T(0);
-                }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int r = m0 + wm0 + dmma_row<A_K>((ig + i) >> 1, q, g);
-                    const int cidx = n0 + wn0 + dmma_col<B_K>((ig + i) & 1, q, tq);
-                    if (!simt_live(o, r, cidx)) continue;
-                    const T tv = (o.beta_mode == 2) ? o.beta * cv[i][q] : cv[i][q];
+                    if (r >= o.m || cidx >= o.n) continue;
+                    if ((o.tri == 1 && r > cidx) || (o.tri == 2 && r < cidx)) continue;
+                    T tv = T(0);
+                    if (o.beta_mode != 0) tv = (o.beta_mode == 1) ? cv[i][q] : o.beta * cv[i][q];
                     o.c[r + static_cast<size_t>(cidx) * o.ldc] = fma(o.alpha, acc[ig + i][q], tv);
                 }
         }
@@ -445,27 +452,34 @@ __device__ __forceinline__ void simt_epilogue(const SimtOut<T>& o, const T (&acc
         return n0 + (B_K ? (wn0 + lane_n * TN + j) : (wn0 + (j / VEC) * 4 * VEC + lane_n * VEC + (j % VEC)));
     };
     // two rows at a time: their C0 values are requested together, before the
-    // stores (which might alias them, so the compiler keeps that order)
+    // stores (which might alias them, so the compiler keeps that order); tests as
+    // above
 #pragma unroll
     for (int ig = 0; ig < 8; ig += 2) {
-        T cv[2][TN];
+        T cv[2][TN] = {};
+        if (o.beta_mode != 0) {
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) {
+                    const int r = row(ig + i), cidx = col(j);
+                    cv[i][j] = simt_live(o, r, cidx) ? o.cin[r + static_cast<size_t>(cidx) * o.ldcin] : T(0);
+                }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int r = row(ig + i);
+            if (r >= o.m) continue;
 #pragma unroll
             for (int j = 0; j < TN; ++j) {
-                const int r = row(ig + i), cidx = col(j);
-                cv[i][j] = (o.beta_mode != 0 && simt_live(o, r, cidx))
-                               ? o.cin[r + static_cast<size_t>(cidx) * o.ldcin] : T(0);
-            }
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < TN; ++j) {
-                const int r = row(ig + i), cidx = col(j);
-                if (!simt_live(o, r, cidx)) continue;
-                const T t = (o.beta_mode == 2) ? o.beta * cv[i][j] : cv[i][j];
+                const int cidx = col(j);
+                if (cidx >= o.n) continue;
+                if ((o.tri == 1 && r > cidx) || (o.tri == 2 && r < cidx)) continue;
+                T t = T(0);
+                if (o.beta_mode != 0) t = (o.beta_mode == 1) ? cv[i][j] : o.beta * cv[i][j];
                 o.c[r + static_cast<size_t>(cidx) * o.ldc] = fma(o.alpha, acc[ig + i][j], t);
             }
+        }
     }
 }
 
