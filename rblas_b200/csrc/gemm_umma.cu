@@ -41,6 +41,7 @@
 #include <mutex>
 #include <vector>
 #include <type_traits>
+#include <utility>
 
 #include "../../include/rblas_b200.h"
 #include "rb_device.cuh"
@@ -3098,12 +3099,6 @@ int bf16_grouped_dev(int planes, const rb_gemm_problem* probs, size_t count, con
     return RB_OK;
 }
 
-// Tail tiles to run unit by unit (OzParams::tail_tiles): the tiles of the
-// partial last wave (all tiles when there are fewer than SMs), when dealing
-// their units as oz_item does finishes clearly before one more whole tile
-// would, counting the reduce pass over their planes and C; else 0. Times are
-// modelled from the products per unit (a diagonal d has d + 1) at the B200's
-// INT8 rate per SM and its copy rate; only their ratio matters.
 // Dynamic shared memory of both Ozaki tile widths, set once per process.
 cudaError_t ozaki_kernel_attributes() {
     static std::once_flag once;
@@ -3129,6 +3124,12 @@ cudaError_t ozaki_kernel_attributes() {
     return result;
 }
 
+// Tail tiles to run unit by unit (OzParams::tail_tiles): the tiles of the
+// partial last wave (all tiles when there are fewer than SMs), when dealing
+// their units as oz_item does finishes clearly before one more whole tile
+// would, counting the reduce pass over their planes and C; else 0. Times are
+// modelled from the products per unit (a diagonal d has d + 1) at the B200's
+// INT8 rate per SM and its copy rate; only their ratio matters.
 int ozaki_tail_tiles(int num_tiles, int slices, int kchunks, int k, int sms, int un) {
     const int upc = (slices + 1) / 2;
     if (kchunks != 1 || upc < 2 || sms < 1) return 0;
@@ -3151,6 +3152,47 @@ int ozaki_tail_tiles(int num_tiles, int slices, int kchunks, int k, int sms, int
     const double reduce_s = 4e-6 + tail * (upc + 2.0) * tile_elems * sizeof(double) / 6.5e12;
     const bool fits = tail * upc * tile_elems * sizeof(double) <= static_cast<double>(size_t(512) << 20);
     return (fits && product_s * max_load + reduce_s < 0.9 * whole_tile_s) ? tail : 0;
+}
+
+// Time (us) of the fullest pair when the tail's items are dealt as pz_item does:
+// ranks in order of cost, G to a pass, every other pass mirrored. A (group, part)
+// is `tail` ranks of one cost, so a pass takes each as one run of pairs; dealing
+// item by item took up to 45 us of every call.
+double ozaki_pair_tail_load(const OzParams& p, const int (&cost)[kOzGroups], int pairs, double prod_us) {
+    const int groups = (p.slices + 3) / 4;
+    int total = 0;
+    for (int g = 0; g < groups; ++g) total += p.tail_tiles * p.parts[g];
+    std::vector<std::pair<long long, int>> step(pairs + 1);  // products, items: from this pair on
+    int rank = 0;
+    for (int i = 0; i < groups; ++i) {
+        const int g = p.order[i], parts = p.parts[g];
+        for (int part = 0; part < parts; ++part) {
+            const long long nkt = p.num_kt, kts = nkt * (part + 1) / parts - nkt * part / parts;
+            for (const int end = rank + p.tail_tiles; rank < end;) {
+                const int pass = rank / pairs, len = std::min(pairs, total - pass * pairs);
+                const int to = std::min(end, (pass + 1) * pairs);
+                int lo = rank - pass * pairs, hi = to - pass * pairs;
+                if (pass & 1) {
+                    const int l = len - hi;
+                    hi = len - lo;
+                    lo = l;
+                }
+                step[lo].first += cost[g] * kts;
+                step[hi].first -= cost[g] * kts;
+                ++step[lo].second;
+                --step[hi].second;
+                rank = to;
+            }
+        }
+    }
+    double load = 0;
+    long long products = 0, items = 0;
+    for (int q = 0; q < pairs; ++q) {
+        products += step[q].first;
+        items += step[q].second;
+        load = std::max(load, products * prod_us + 3.0 * items);
+    }
+    return load;
 }
 
 // The pair kernel's tail (OzParams::tail_tiles, parts, order, plane0, planes):
@@ -3202,19 +3244,7 @@ void ozaki_pair_tail(OzParams& p, int pairs) {
         cand.planes = planes;
         const size_t bytes = static_cast<size_t>(tail) * planes * kPzTileElems * sizeof(double);
         if (bytes > (size_t(512) << 20)) break;
-        // the snake's fullest pair: the items' costs in rank order, one per pass
-        const int total = pz_items(cand) - (p.num_tiles - tail);
-        double load = 0;
-        for (int q = 0; q < std::min(total, pairs); ++q) {
-            double l = 0;
-            for (int j = q; j < total; j += pairs) {
-                PzWork w{};
-                pz_item(cand, pairs, p.num_tiles - tail + j, w);
-                const int g = groups - 1 - w.u_lo;
-                l += cost[g] * (w.kt1 - w.kt0) * prod_us + 3.0;
-            }
-            load = std::max(load, l);
-        }
+        const double load = ozaki_pair_tail_load(cand, cost, pairs, prod_us);
         const double t = load + 10.0 + (bytes + 2.0 * tail * kPzTileElems * sizeof(double)) / 5e6;
         if (t < best) {
             best = t;
