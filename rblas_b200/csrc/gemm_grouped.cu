@@ -331,7 +331,6 @@ void set_tuned_ozaki_widths(std::shared_ptr<const std::map<uint32_t, int>> table
 }
 
 void force_ozaki_width(int w) { t_forced_oz_width = w; }
-bool ozaki_width_forced() { return t_forced_oz_width != 0; }
 
 int ozaki_tile_n(size_t m, size_t n, size_t k) {
     if (t_forced_oz_width) return t_forced_oz_width;

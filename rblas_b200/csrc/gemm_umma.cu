@@ -3262,10 +3262,9 @@ void ozaki_pair_tail(OzParams& p, int pairs) {
 // Whether an m x n product takes the pair kernel: unless one tile row of 128 is
 // all it has, or a pair's 256 rows pad so much more than 128 that the wide
 // tiles' larger cost (per 128 x 256 C of one SM 1 against 0.85 for a pair's
-// 256 x 128) is the smaller one. A width that the autotuner forces while it
-// times the other kernels wins.
+// 256 x 128) is the smaller one.
 bool ozaki_pair_tiles(int m, int n) {
-    if (m <= 128 || ozaki_width_forced()) return false;
+    if (m <= 128) return false;
     const double wide = static_cast<double>((m + 127) / 128) * ((n + 255) / 256);
     return n <= 128 || 0.85 * ((m + 255) / 256) * ((n + 127) / 128) <= wide;
 }

@@ -11,11 +11,12 @@
 //     larger factor must win by 3% to be kept. Buckets with a full wave of C
 //     tiles, or too short a K for two ranges of four K-tiles, are left to
 //     the built-in rule.
-//   - the tile width of the Ozaki tensor-core kernels, 128 x 256 or
+//   - the tile width of the Ozaki kernels on single CTAs, 128 x 256 or
 //     128 x 128 (f64 buckets with n below 2048): the narrow tile pads less
 //     and deals more tiles to the SMs, the wide one lands fewer operand bytes
 //     per MAC. The narrow one must win by 3%. The width changes no result
-//     bit.
+//     bit. Timed on a shape of the bucket that does not run on CTA pairs;
+//     a bucket without one has no width.
 // The table is written as text:
 //
 //   rblas_b200 grouped autotune v2
@@ -60,6 +61,32 @@ std::string device_tag() {
 }
 
 constexpr int kLoBucket = 5, kHiBucket = 12;  // 32 .. 4096
+
+// The m x n of bucket (lm, ln) to time the Ozaki tile widths on: the
+// representative one or, where that runs on CTA pairs, the nearest to it (in
+// the product of the ratios) of the largest sizes per number of 128-wide tiles
+// that does not. False: every shape of the bucket runs on pairs.
+bool ozaki_width_shape(int lm, int ln, int* m, int* n) {
+    const int rm = static_cast<int>(std::ldexp(1.41, lm)), rn = static_cast<int>(std::ldexp(1.41, ln));
+    auto sizes = [](int l, int r) {
+        std::vector<int> v{r, 1 << l};
+        for (int x = (1 << l) / 128 * 128 + 128; x < 2 << l; x += 128) v.push_back(x);
+        v.push_back((2 << l) - 1);
+        return v;
+    };
+    double best = 0;
+    for (int x : sizes(lm, rm))
+        for (int y : sizes(ln, rn)) {
+            if (ozaki_pair_tiles(x, y)) continue;
+            const double far = std::fabs(std::log2(static_cast<double>(x) / rm)) +
+                               std::fabs(std::log2(static_cast<double>(y) / rn));
+            if (best != 0 && far + 1 >= best) continue;
+            best = far + 1;
+            *m = x;
+            *n = y;
+        }
+    return best != 0;
+}
 
 }  // namespace
 
@@ -161,10 +188,10 @@ rb_status rb_autotune_grouped(const char* cache_path, int* buckets_tuned) {
     // Ozaki tile width per f64 bucket (n below 2048)
     auto oz_table = std::make_shared<std::map<uint32_t, int>>();
     for (int lm = kLoBucket; lm <= kHiBucket && status == RB_OK; ++lm)
-        for (int ln = kLoBucket; ln <= 10 && status == RB_OK; ++ln)
+        for (int ln = kLoBucket; ln <= 10 && status == RB_OK; ++ln) {
+            int m, n;
+            if (!ozaki_width_shape(lm, ln, &m, &n)) continue;
             for (int lk = kLoBucket; lk <= kHiBucket && status == RB_OK; ++lk) {
-                const int m = static_cast<int>(std::ldexp(1.41, lm));
-                const int n = static_cast<int>(std::ldexp(1.41, ln));
                 const int k = static_cast<int>(std::ldexp(1.41, lk));
                 float ms[2] = {0, 0};
                 for (int w = 0; w < 2 && status == RB_OK; ++w) {
@@ -188,6 +215,7 @@ rb_status rb_autotune_grouped(const char* cache_path, int* buckets_tuned) {
                 (*oz_table)[tune_key(1, m, n, k)] = (ms[1] < 0.97f * ms[0]) ? 128 : 256;
                 ++tuned;
             }
+        }
     force_ozaki_width(0);
     if (status == RB_OK) {
         if (cache_path && *cache_path) {
