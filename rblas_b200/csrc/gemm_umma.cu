@@ -3355,13 +3355,108 @@ cudaError_t launch_ozaki_gemm(bool ta, bool tb, int m, int n, int k, double alph
     return e;
 }
 
-// Many f64 GEMMs in the Ozaki form with three launches for the whole batch:
-// one exponent pass and one slice pass over every operand, then one
-// persistent ozaki_grouped_kernel over every problem's tiles. probs[i] is
+// The problems of one kind of tile (0: pairs; 1, 2: 256- and 128-wide tiles of
+// one CTA) in a grouped Ozaki launch, longest K first.
+struct OzGroupKind {
+    std::vector<std::pair<int, int>> jobs;  // tiles, K tiles
+    double per_kt, per_tile;                // us: one tile's K tile, the rest of it
+    // of `workers` (pairs, CTAs), each with every workers-th tile: the first's time
+    double time(int workers) const {
+        double t = 0;
+        long long at = 0;
+        for (const auto& j : jobs) {
+            const long long end = at + j.first;
+            t += ((end + workers - 1) / workers - (at + workers - 1) / workers) * (j.second * per_kt + per_tile);
+            at = end;
+        }
+        return t;
+    }
+    int workers_for(double us, int cap) const {  // the fewest that finish in `us` (cap + 1: none do)
+        if (jobs.empty()) return 0;
+        int lo = 1, hi = cap + 1;
+        while (lo < hi) {
+            const int mid = (lo + hi) / 2;
+            if (time(mid) <= us) hi = mid;
+            else                 lo = mid + 1;
+        }
+        return lo;
+    }
+};
+
+// Workers of each kind's launch when the kinds share the SMs and start together:
+// the split that ends first, or false where one after the other does about as
+// well. A persistent CTA holds its SM, so launches of the whole GPU each run one
+// after the other however few tiles they have, and each ends in its longest
+// chain. 40 mixed requests up to 512 a side took 155 us in two kinds of tile, 208
+// with pairs as a third, 148 sharing; 24 up to 2048 a side 358, 458 and 270. Costs
+// as fitted to 41 sets: a product of a pair's tile 250 clocks, of a 128 x 256 one
+// 540, of a 128 x 128 one 450; a tile's drains 10, 50 and 20 us. What the split
+// leaves over goes to the kind that ends last.
+bool ozaki_share_sms(OzGroupKind (&kinds)[3], int slices, int sms, int (&workers)[3]) {
+    const double prod_us = slices * (slices + 1) / 2 / 1.7e3;
+    const double clocks[3] = {250, 540, 450}, tile_us[3] = {10, 50, 20};
+    const int sm[3] = {2, 1, 1};
+    int cap[3] = {sms / 2, sms, sms};
+    double lo = 0, hi = 0;
+    int used = 0;
+    for (int q = 0; q < 3; ++q) {
+        workers[q] = 0;
+        if (kinds[q].jobs.empty()) continue;
+        kinds[q].per_kt = clocks[q] * prod_us;
+        kinds[q].per_tile = tile_us[q];
+        long long tiles = 0;
+        for (const auto& j : kinds[q].jobs) tiles += j.first;
+        cap[q] = static_cast<int>(std::min<long long>(cap[q], tiles));
+        const double t = kinds[q].time(cap[q]);
+        lo = std::max(lo, t);
+        hi += t;
+        ++used;
+    }
+    hi *= 0.95;
+    int left = 0;
+    auto fits = [&](double us) {
+        left = sms;
+        bool all = true;
+        for (int q = 0; q < 3; ++q) {
+            workers[q] = kinds[q].workers_for(us, cap[q]);
+            left -= sm[q] * workers[q];
+            all = all && workers[q] <= cap[q];
+        }
+        return all && left >= 0;
+    };
+    if (used < 2 || !fits(hi)) return false;
+    for (int i = 0; i < 7; ++i) {
+        const double mid = 0.5 * (lo + hi);
+        if (fits(mid)) hi = mid;
+        else           lo = mid;
+    }
+    fits(hi);
+    for (;;) {
+        int last = -1;
+        double end = 0;
+        for (int q = 0; q < 3; ++q) {
+            if (workers[q] >= cap[q] || left < sm[q]) continue;
+            const double t = kinds[q].time(workers[q]);
+            if (t > end) {
+                end = t;
+                last = q;
+            }
+        }
+        if (last < 0) return true;
+        const int more = std::min(cap[last] - workers[last], std::max(1, left / sm[last] / 4));
+        workers[last] += more;
+        left -= sm[last] * more;
+    }
+}
+
+// Many f64 GEMMs in the Ozaki form: one exponent pass and one slice pass over
+// every operand, then a persistent launch per kind of tile
+// (ozaki_pair_grouped_kernel, ozaki_grouped_kernel of either width) over the
+// problems of that kind. probs[i] is
 // column-major or row-major like rb_gemm_problem; its C0 is read from
 // cin[i] (leading dimension ldcin[i]; probs[i].c itself when cin is null) and
-// the result goes to probs[i].c. Every tile runs the fused epilogue of
-// ozaki_gemm_kernel, so each result equals that problem's own
+// the result goes to probs[i].c. Every tile folds its terms in the order of the
+// single call, so each result equals that problem's own
 // rb_dgemm_dev(..., RB_PREC_OZAKI, ...) bit for bit.
 int ozaki_grouped_dev(const rb_gemm_problem* probs, size_t count, const void* const* cin, const size_t* ldcin,
                       cudaStream_t st, int32_t* ce) {
@@ -3473,6 +3568,7 @@ int ozaki_grouped_dev(const rb_gemm_problem* probs, size_t count, const void* co
     uint32_t* err_word = device_error_word();
     int exp_blocks = 0, slice_blocks = 0;
     int kind_first[3] = {}, kind_count[3] = {}, kind_tiles[3] = {};  // problems and tiles of each launch
+    OzGroupKind group_kinds[3];
     for (const Job& j : jobs) ++kind_count[j.kind];
     for (int q = 1; q < 3; ++q) kind_first[q] = kind_first[q - 1] + kind_count[q - 1];
     double work = 0;
@@ -3515,6 +3611,7 @@ int ozaki_grouped_dev(const rb_gemm_problem* probs, size_t count, const void* co
         // [kind_first[q] + q, kind_first[q] + kind_count[q] + q]
         starts[i + j.kind] = kind_tiles[j.kind];
         kind_tiles[j.kind] += p.num_tiles;
+        group_kinds[j.kind].jobs.emplace_back(p.num_tiles, j.num_kt);
         work += 2.0 * j.m * j.n * static_cast<double>(j.k) * slices * (slices + 1) / 2;
     }
     for (int q = 0; q < 3; ++q) starts[kind_first[q] + kind_count[q] + q] = kind_tiles[q];
@@ -3543,29 +3640,35 @@ int ozaki_grouped_dev(const rb_gemm_problem* probs, size_t count, const void* co
         kernel_timing_begin("umma_ozaki_grouped_i8", work, st, &tmr);
         const OzGroupEntry* dtab = reinterpret_cast<const OzGroupEntry*>(mem);
         const int* dstarts = reinterpret_cast<const int*>(mem + ent_bytes);
-        // with more than one kind, the first goes on st and the others on a
-        // forked stream: their CTAs take the SMs that the first launch's leave
-        // as they finish (each persistent CTA holds a whole SM), instead of
-        // waiting for its last tile
+        // With more than one kind, the first goes on st and the others on forked
+        // streams. Where they share the SMs each has one of its own; else the
+        // others have one together, and their CTAs take the SMs that the first
+        // launch's leave as they finish. (Pairs first: they need both SMs of a
+        // TPC.)
         const int kinds = (kind_count[0] > 0) + (kind_count[1] > 0) + (kind_count[2] > 0);
+        int workers[3] = {};
         ForkedStream fk;
-        const bool fork = kinds > 1 && fork_stream(st, &fk) == cudaSuccess;
-        bool started = false;
+        const bool share = kinds > 1 && ozaki_share_sms(group_kinds, slices, sms, workers);
+        const bool fork = kinds > 1 && fork_stream(st, &fk, share && kinds == 3) == cudaSuccess;
+        if (!share || !fork) {
+            workers[0] = sms / 2;
+            workers[1] = workers[2] = sms;
+        }
+        int started = 0;
         for (int q = 0; q < 3; ++q) {
             if (kind_count[q] == 0) continue;
-            const cudaStream_t ks = started && fork ? fk.s : st;
-            started = true;
+            const cudaStream_t ks = !started || !fork ? st : started == 2 && fk.s2 ? fk.s2 : fk.s;
+            ++started;
             const OzGroupEntry* kt = dtab + kind_first[q];
             const int* ks0 = dstarts + kind_first[q] + q;
+            const int grid = std::min(kind_tiles[q], workers[q]);
             if (q == 0)
-                ozaki_pair_grouped_kernel<<<2 * std::min(kind_tiles[0], sms / 2), pz_threads(kPzGroupEpiWarps), kPzSmem, ks>>>(
-                    kt, ks0, kind_count[0], err_word);
+                ozaki_pair_grouped_kernel<<<2 * grid, pz_threads(kPzGroupEpiWarps), kPzSmem, ks>>>(kt, ks0, kind_count[0],
+                                                                                                   err_word);
             else if (q == 1)
-                ozaki_grouped_kernel<256><<<std::min(kind_tiles[1], sms), kOzThreads, OzCfg<256>::SMEM, ks>>>(
-                    kt, ks0, kind_count[1], err_word);
+                ozaki_grouped_kernel<256><<<grid, kOzThreads, OzCfg<256>::SMEM, ks>>>(kt, ks0, kind_count[1], err_word);
             else
-                ozaki_grouped_kernel<128><<<std::min(kind_tiles[2], sms), kOzThreads, OzCfg<128>::SMEM, ks>>>(
-                    kt, ks0, kind_count[2], err_word);
+                ozaki_grouped_kernel<128><<<grid, kOzThreads, OzCfg<128>::SMEM, ks>>>(kt, ks0, kind_count[2], err_word);
         }
         e = cudaGetLastError();
         if (fork) {

@@ -876,13 +876,13 @@ constexpr int kAuxStreams = 4;
 struct AuxSlot {
     std::mutex mu;
     bool init = false;
-    cudaStream_t s = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
+    cudaStream_t s = nullptr, s2 = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr, join2 = nullptr;
 };
 AuxSlot g_aux[kMaxDevices][kAuxStreams];
 }  // namespace
 
-cudaError_t fork_stream(cudaStream_t st, ForkedStream* f) {
+cudaError_t fork_stream(cudaStream_t st, ForkedStream* f, bool two) {
     const int d = current_device();
     if (d < 0 || d >= kMaxDevices) return cudaErrorInvalidDevice;
     const int slot = static_cast<int>((reinterpret_cast<uintptr_t>(st) >> 4) % kAuxStreams);
@@ -895,13 +895,19 @@ cudaError_t fork_stream(cudaStream_t st, ForkedStream* f) {
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&a.join, cudaEventDisableTiming);
         a.init = e == cudaSuccess;
     }
+    if (two && !a.s2 && e == cudaSuccess) {
+        e = cudaEventCreateWithFlags(&a.join2, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&a.s2, cudaStreamNonBlocking);
+    }
     if (e == cudaSuccess) e = cudaEventRecord(a.fork, st);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(a.s, a.fork, 0);
+    if (e == cudaSuccess && two) e = cudaStreamWaitEvent(a.s2, a.fork, 0);
     if (e != cudaSuccess) {
         a.mu.unlock();
         return e;
     }
     f->s = a.s;
+    f->s2 = two ? a.s2 : nullptr;
     f->slot = d * kAuxStreams + slot;
     return cudaSuccess;
 }
@@ -911,8 +917,13 @@ cudaError_t join_stream(cudaStream_t st, ForkedStream* f) {
     AuxSlot& a = g_aux[f->slot / kAuxStreams][f->slot % kAuxStreams];
     cudaError_t e = cudaEventRecord(a.join, a.s);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(st, a.join, 0);
+    if (f->s2) {
+        cudaError_t e2 = cudaEventRecord(a.join2, f->s2);
+        if (e2 == cudaSuccess) e2 = cudaStreamWaitEvent(st, a.join2, 0);
+        if (e == cudaSuccess) e = e2;
+    }
     f->slot = -1;
-    f->s = nullptr;
+    f->s = f->s2 = nullptr;
     a.mu.unlock();
     return e;
 }

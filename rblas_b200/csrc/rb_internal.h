@@ -73,15 +73,16 @@ uint32_t* device_error_word();
 
 // A second stream for work that may overlap the caller's stream st: after
 // fork_stream, f->s starts behind everything queued on st so far; after
-// join_stream, st waits for everything queued on f->s. The pair holds one
+// join_stream, st waits for everything queued on f->s; with `two`, the same
+// for a third stream f->s2. The pair holds one
 // of a few per-device auxiliary streams (picked by st) locked in between,
 // so concurrent callers never interleave their fork and join records.
 // Both also work while st is being captured into a CUDA graph.
 struct ForkedStream {
-    cudaStream_t s = nullptr;
+    cudaStream_t s = nullptr, s2 = nullptr;
     int slot = -1;
 };
-cudaError_t fork_stream(cudaStream_t st, ForkedStream* f);
+cudaError_t fork_stream(cudaStream_t st, ForkedStream* f, bool two = false);
 cudaError_t join_stream(cudaStream_t st, ForkedStream* f);
 
 // ---- device allocations ---------------------------------------------------------
