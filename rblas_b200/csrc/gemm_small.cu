@@ -323,38 +323,67 @@ cudaError_t launch_small_gemm(int cfg, bool a_kmajor, bool b_kmajor, int m, int 
 
 // Which small tile (1: 32 x 32; 2: 64 x 64, f32 only) an m x n x k product
 // runs fastest on, or 0: the 128-wide tiles, given the grouped kernel's split
-// factor for them (1: not split). Times in us: a launch, and a time per k that
-// a CTA alone on its SM takes (a chain of latencies) or its tiles per SM times
-// what each costs there. From calls (us, 128-wide -> small): SGEMM 256^3 32.8
-// -> 10.3, 512^3 54.7 -> 20.5, 768^3 75.9 -> 36.9 (64 x 64), 1000 x 700 x 333
-// 48 -> 26, 1024^3 59.8 against 72 (left); DGEMM 256^3 26.2 -> 10.3, 512^3
-// 34.9 -> 20.5, 1000 x 700 x 333 37.9 -> 33.5, 1024^3 96 against 108 (left);
-// 300 x 300 x 3000 split in K 72 (f32), 63 (f64), small 63-90, 57-72.
+// factor for them (1: not split). Times in us: a launch, what a wave of tiles
+// costs beside its k (C's stores above all: 3000^2 of k = 16 is four waves of
+// wide tiles, 60 of small ones), and a time per k that a CTA alone on its SM
+// takes (a chain of latencies) or its tiles per SM times what each costs there,
+// by how each operand is stored: K-major or off 16 bytes it is copied element by
+// element (the wide tiles repack what is off 16 bytes first). Fitted to 1669 calls
+// of k 8 .. 2900, all transposes, leading dimensions on and off 16 bytes: the
+// choice is 0.9 % (f64 0.2 %) off the best one in the mean; by k and the numbers
+// of tiles alone it was 2.0 and 1.7 %.
+// us, 128-wide -> small: SGEMM 256^3 32.8 -> 10.3, 512^3 54.7 -> 20.5, 768^3 75.9
+// -> 36.9 (64 x 64); DGEMM 256^3 26.2 -> 10.3, 512^3 34.9 -> 20.5; left: SGEMM
+// 1024^3 59.8 against 72, A^T B^T 1200^2 of k = 32 8.4 against 12, 3000^2 of k =
+// 16 29 against 37; DGEMM 1024^3 96 against 108, A^T B 1700^2 of k = 16 12.4
+// against 18.5.
 template <typename T>
-int small_gemm_cfg(size_t m, size_t n, size_t k, int splits, int sms) {
+int small_gemm_cfg(size_t m, size_t n, size_t k, int splits, int sms, const SmallOperands& op) {
     auto waves = [&](size_t bm, size_t bn, int s = 1) {
         return std::ceil(static_cast<double>((m + bm - 1) / bm) * static_cast<double>((n + bn - 1) / bn) * s / sms);
     };
     const double K = static_cast<double>(k);
+    const int a = op.a_k, b = op.b_k;  // (as numbers)
+    const int rows = (!op.a_k && !op.a_vec) + (!op.b_k && !op.b_vec);  // MN-major operands copied by element
+    const int packed = !op.a_vec + !op.b_vec;
+    const double packed_mega = 1e-6 * K * ((op.a_vec ? 0.0 : static_cast<double>(m)) + (op.b_vec ? 0.0 : static_cast<double>(n)));
     if (sizeof(T) == 4) {
-        const double t1 = 5.0 + K * std::max(0.023, 0.0125 * waves(32, 32));
-        const double t2 = 6.2 + K * std::max(0.040, 0.034 * waves(64, 64));
-        const double wide = splits > 1             ? 20.0 + 0.085 * K / splits * waves(128, 128, splits)
-                            : simt_narrow_f32(m, n) ? 8.0 + 0.050 * K * waves(128, 64)
-                                                    : 11.0 + 0.085 * K * waves(128, 128);
+        const double w1 = waves(32, 32), w2 = waves(64, 64);
+        const double t1 =
+            std::max(8.5, 5.0 + 0.44 * w1 + K * std::max(0.0175 + 0.0018 * a + 0.0016 * b + 0.0040 * rows,
+                                                         (0.0107 + 0.0008 * a + 0.0006 * b + 0.0032 * rows) * w1));
+        const double t2 =
+            std::max(8.5, 5.1 + 1.64 * w2 + K * std::max(0.0305 + 0.0045 * a + 0.0060 * b + 0.0084 * rows,
+                                                         (0.0255 + 0.0020 * a + 0.0026 * b + 0.0068 * rows) * w2));
+        double wide = 4.2 * packed + 4.6 * packed_mega;
+        if (splits > 1) {
+            const double w = waves(128, 128, splits);
+            wide += 18.2 + 9.2 * w + (0.0587 + 0.0142 * a + 0.0144 * b) * K / splits * w;
+        } else if (simt_narrow_f32(m, n)) {
+            const double w = waves(128, 64);
+            wide += 5.1 + 1.57 * w + (0.0437 + 0.0034 * a + 0.0084 * b) * K * w;
+        } else {
+            const double w = waves(128, 128);
+            wide += 1.6 + 6.4 * w + (0.0728 + 0.0043 * a + 0.0120 * b) * K * w;
+        }
+        wide = std::max(7.8, wide);
         return std::min(t1, t2) >= wide ? 0 : t1 <= t2 ? 1 : 2;
     }
-    const double t1 = 4.5 + K * std::max(0.022, 0.0165 * waves(32, 32));
-    const double wide = splits > 1 ? 15.0 + 0.078 * K / splits * waves(128, 64, splits)
-                                   : 6.4 + 0.078 * K * waves(128, 64);
-    return t1 < wide ? 1 : 0;
+    const double w1 = waves(32, 32), w = waves(128, 64, splits);
+    const double t1 =
+        std::max(8.5, 4.1 + 0.55 * w1 + K * std::max(0.0226 - 0.001 * a + 0.001 * b + 0.0033 * rows,
+                                                     (0.0134 + 0.0008 * a + 0.0032 * b + 0.0019 * rows) * w1));
+    const double wide = 4.4 * packed + 7.3 * packed_mega +
+                        (splits > 1 ? 9.3 + 6.1 * w + 0.069 * K / splits * w
+                                    : 2.9 + 3.5 * w + (0.068 - 0.004 * a - 0.0014 * b) * K * w);
+    return t1 < std::max(7.8, wide) ? 1 : 0;
 }
 
 template cudaError_t launch_small_gemm<float>(int, bool, bool, int, int, int, float, const float*, size_t, const float*,
                                               size_t, float, float*, size_t, cudaStream_t, int, int);
 template cudaError_t launch_small_gemm<double>(int, bool, bool, int, int, int, double, const double*, size_t,
                                                const double*, size_t, double, double*, size_t, cudaStream_t, int, int);
-template int small_gemm_cfg<float>(size_t, size_t, size_t, int, int);
-template int small_gemm_cfg<double>(size_t, size_t, size_t, int, int);
+template int small_gemm_cfg<float>(size_t, size_t, size_t, int, int, const SmallOperands&);
+template int small_gemm_cfg<double>(size_t, size_t, size_t, int, int, const SmallOperands&);
 
 }  // namespace rb

@@ -358,7 +358,8 @@ int plain_small(const ColProblem<T>& p, int splits) {
             return 0;
         sms.store(n, std::memory_order_relaxed);
     }
-    return small_gemm_cfg<T>(p.m, p.n, p.k, splits, n);
+    auto vec = [](const T* x, size_t ld) { return reinterpret_cast<uintptr_t>(x) % 16 == 0 && ld * sizeof(T) % 16 == 0; };
+    return small_gemm_cfg<T>(p.m, p.n, p.k, splits, n, {p.ta, !p.tb, vec(p.a, p.lda), vec(p.b, p.ldb)});
 }
 
 template <typename T>

@@ -121,8 +121,12 @@ bool simt_narrow_f32(size_t m, size_t n);
 // 128-wide tiles (with the grouped kernel's K split `splits`). k_range: where
 // the grouped kernel splits K, the k of its ranges (0: unsplit), whose sums
 // are then formed apart and added in order, as there.
+struct SmallOperands {
+    bool a_k, b_k;      // K-major
+    bool a_vec, b_vec;  // base and leading dimension on 16 bytes
+};
 template <typename T>
-int small_gemm_cfg(size_t m, size_t n, size_t k, int splits, int sms);
+int small_gemm_cfg(size_t m, size_t n, size_t k, int splits, int sms, const SmallOperands& op);
 template <typename T>
 cudaError_t launch_small_gemm(int cfg, bool a_kmajor, bool b_kmajor, int m, int n, int k, T alpha, const T* A, size_t lda,
                               const T* B, size_t ldb, T beta, T* C, size_t ldc, cudaStream_t st, int tri, int k_range);
