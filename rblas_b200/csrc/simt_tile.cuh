@@ -412,34 +412,37 @@ __device__ __forceinline__ void simt_epilogue(const SimtOut<T>& o, const T (&acc
         const int g = lane >> 2, tq = lane & 3;
         const int wm0 = wm * 64, wn0 = wn * 16;
         if (m0 + wm0 >= o.m || n0 + wn0 >= o.n) return;
-        // 16 C0 values requested at a time. Each store stands behind its own
-        // tests, and the reads behind one of beta: with one test of both (and the
-        // stores' addresses formed with the reads') beta == 0 took 2-3 % longer.
+        auto row = [&](int i, int q) { return m0 + wm0 + dmma_row<A_K>(i >> 1, q, g); };
+        auto col = [&](int i, int q) { return n0 + wn0 + dmma_col<B_K>(i & 1, q, tq); };
+        auto put = [&](int i, int q, T tv) {
+            const int r = row(i, q), cidx = col(i, q);
+            if (r >= o.m || cidx >= o.n) return;
+            if ((o.tri == 1 && r > cidx) || (o.tri == 2 && r < cidx)) return;
+            o.c[r + static_cast<size_t>(cidx) * o.ldc] = fma(o.alpha, acc[i][q], tv);
+        };
+        // 16 C0 values requested at a time; without C0 a loop of its own (in one
+        // loop with the reads behind a test, A^T B^T without C0 took 4 % longer)
+        if (o.beta_mode == 0) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) put(i, q, T(0));
+            return;
+        }
 #pragma unroll
         for (int ig = 0; ig < 8; ig += 4) {
-            T cv[4][4] = {};
-            if (o.beta_mode != 0) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const int r = m0 + wm0 + dmma_row<A_K>((ig + i) >> 1, q, g);
-                        const int cidx = n0 + wn0 + dmma_col<B_K>((ig + i) & 1, q, tq);
-                        cv[i][q] = simt_live(o, r, cidx) ? o.cin[r + static_cast<size_t>(cidx) * o.ldcin] : T(0);
-                    }
-            }
+            T cv[4][4];
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    const int r = m0 + wm0 + dmma_row<A_K>((ig + i) >> 1, q, g);
-                    const int cidx = n0 + wn0 + dmma_col<B_K>((ig + i) & 1, q, tq);
-                    if (r >= o.m || cidx >= o.n) continue;
-                    if ((o.tri == 1 && r > cidx) || (o.tri == 2 && r < cidx)) continue;
-                    T tv = T(0);
-                    if (o.beta_mode != 0) tv = (o.beta_mode == 1) ? cv[i][q] : o.beta * cv[i][q];
-                    o.c[r + static_cast<size_t>(cidx) * o.ldc] = fma(o.alpha, acc[ig + i][q], tv);
+                    const int r = row(ig + i, q), cidx = col(ig + i, q);
+                    cv[i][q] = simt_live(o, r, cidx) ? o.cin[r + static_cast<size_t>(cidx) * o.ldcin] : T(0);
                 }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) put(ig + i, q, (o.beta_mode == 1) ? cv[i][q] : o.beta * cv[i][q]);
         }
         return;
     }
@@ -451,34 +454,38 @@ __device__ __forceinline__ void simt_epilogue(const SimtOut<T>& o, const T (&acc
     auto col = [&](int j) {
         return n0 + (B_K ? (wn0 + lane_n * TN + j) : (wn0 + (j / VEC) * 4 * VEC + lane_n * VEC + (j % VEC)));
     };
+    auto put = [&](int i, int j, T tv) {
+        const int r = row(i), cidx = col(j);
+        if (r >= o.m || cidx >= o.n) return;
+        if ((o.tri == 1 && r > cidx) || (o.tri == 2 && r < cidx)) return;
+        o.c[r + static_cast<size_t>(cidx) * o.ldc] = fma(o.alpha, acc[i][j], tv);
+    };
+    if (o.beta_mode == 0) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (row(i) >= o.m) continue;
+#pragma unroll
+            for (int j = 0; j < TN; ++j) put(i, j, T(0));
+        }
+        return;
+    }
     // two rows at a time: their C0 values are requested together, before the
-    // stores (which might alias them, so the compiler keeps that order); tests as
-    // above
+    // stores (which might alias them, so the compiler keeps that order)
 #pragma unroll
     for (int ig = 0; ig < 8; ig += 2) {
-        T cv[2][TN] = {};
-        if (o.beta_mode != 0) {
+        T cv[2][TN];
 #pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j) {
-                    const int r = row(ig + i), cidx = col(j);
-                    cv[i][j] = simt_live(o, r, cidx) ? o.cin[r + static_cast<size_t>(cidx) * o.ldcin] : T(0);
-                }
-        }
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int r = row(ig + i);
-            if (r >= o.m) continue;
+        for (int i = 0; i < 2; ++i)
 #pragma unroll
             for (int j = 0; j < TN; ++j) {
-                const int cidx = col(j);
-                if (cidx >= o.n) continue;
-                if ((o.tri == 1 && r > cidx) || (o.tri == 2 && r < cidx)) continue;
-                T t = T(0);
-                if (o.beta_mode != 0) t = (o.beta_mode == 1) ? cv[i][j] : o.beta * cv[i][j];
-                o.c[r + static_cast<size_t>(cidx) * o.ldc] = fma(o.alpha, acc[ig + i][j], t);
+                const int r = row(ig + i), cidx = col(j);
+                cv[i][j] = simt_live(o, r, cidx) ? o.cin[r + static_cast<size_t>(cidx) * o.ldcin] : T(0);
             }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            if (row(ig + i) >= o.m) continue;
+#pragma unroll
+            for (int j = 0; j < TN; ++j) put(ig + i, j, (o.beta_mode == 1) ? cv[i][j] : o.beta * cv[i][j]);
         }
     }
 }
