@@ -875,6 +875,21 @@ __global__ void __launch_bounds__(kTbThreads, 1)
     }
 }
 
+// Whether 32-wide slices (one CTA per SM) finish before 16-wide ones (two per
+// SM). In units of a wave of the latter, 2 sms slices: their last wave takes 0.7
+// of one where it leaves each SM one CTA at most; a wave of wide slices takes
+// 0.78, and up to a tenth more where the order is padded to blocks of 64. Over
+// 1912 calls the choice is 0.3 % off the better one in the mean (always wide
+// 1.5 %, always 16-wide 6.6 %). us, 16-wide / 32-wide: 600 x 48, 75 members (225
+// slices against 150 on 148 SMs) 127 / 195, 200 x 100, 40 members 38 / 50, 512 x
+// 100, 150 members 342 / 290.
+bool trsm_wide_slices(int q, int nrhs, size_t batch, int sms) {
+    const size_t n16 = batch * ((nrhs + 15) / 16), n32 = batch * ((nrhs + 31) / 32), rest = n16 % (2 * sms);
+    const double padded = 64.0 * ((q + 63) / 64) / q;
+    const double t16 = static_cast<double>(n16 / (2 * sms)) + (rest == 0 ? 0.0 : rest <= static_cast<size_t>(sms) ? 0.7 : 1.0);
+    return 0.78 * std::min(1.1, padded * padded) * static_cast<double>((n32 + sms - 1) / sms) < t16;
+}
+
 size_t tw_smem(int q) {
     return (static_cast<size_t>(q) + 2 * kInvNB) * kTwYS * sizeof(double);
 }
@@ -982,15 +997,12 @@ int trsm_batched_dev(int side, int uplo, int trans, int diag, size_t m, size_t n
     bool alloc_failed = false;
     int td_rb = 0;  // f64: slice width of the tensor-core path (0: not used)
     if constexpr (sizeof(T) == 8) {
-        // 16-wide slices while two CTAs fit an SM, then 8-wide, then one CTA per SM
-        // 32-wide ones where 16-wide ones would put a second CTA on some SM
-        // (one 16-wide CTA per SM finishes first: 512 x 512, us: 59 against
-        // 70; 512 x 4096 of a 1024 system: 274 against 227)
+        // 16-wide slices while two CTAs fit an SM, then 8-wide, then one CTA per SM;
+        // 32-wide ones where their waves take less time
         int dev = 0, sms = 148;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const size_t slices16 = static_cast<size_t>((p.nrhs + 15) / 16) * batch;
-        if (p.nrhs > 16 && slices16 > static_cast<size_t>(sms) && tw_smem(p.q) <= kTbSmemMax) td_rb = 32;
+        if (tw_smem(p.q) <= kTbSmemMax && trsm_wide_slices(p.q, p.nrhs, batch, sms)) td_rb = 32;
         else if (td_smem<16>(p.q) <= kTbSmemMax / 2) td_rb = 16;
         else if (td_smem<8>(p.q) <= kTbSmemMax / 2) td_rb = 8;
         else if (td_smem<16>(p.q) <= kTbSmemMax) td_rb = 16;
