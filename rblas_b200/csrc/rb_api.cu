@@ -892,13 +892,10 @@ cudaError_t fork_stream(cudaStream_t st, ForkedStream* f, bool two) {
     cudaError_t e = cudaSuccess;
     if (!a.init) {
         e = cudaStreamCreateWithFlags(&a.s, cudaStreamNonBlocking);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&a.fork, cudaEventDisableTiming);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&a.join, cudaEventDisableTiming);
-        a.init = e == cudaSuccess;
-    }
-    if (two && !a.s2 && e == cudaSuccess) {
-        e = cudaEventCreateWithFlags(&a.join2, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&a.s2, cudaStreamNonBlocking);
+        for (cudaEvent_t* ev : {&a.fork, &a.join, &a.join2})
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+        a.init = e == cudaSuccess;
     }
     if (e == cudaSuccess) e = cudaEventRecord(a.fork, st);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(a.s, a.fork, 0);
