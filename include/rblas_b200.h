@@ -437,11 +437,13 @@ rb_status rb_dtrmm_dev(rb_side side, rb_uplo uplo, rb_transpose trans, rb_diag d
  * solves one problem per call: trsm, src/level3.rs:390-520). Problem i solves
  * with A_i = a + i*stride_a and B_i = b + i*stride_b (elements), all sharing
  * side, uplo, trans, diag, m, n, alpha, lda, ldb; column-major like rblas.
- * One launch for the batch: each CTA keeps a slice of B_i's right-hand sides
- * in shared memory for the whole solve (32 right-hand sides per CTA up to
- * order 632 f64 / 1512 f32, 16 or 8 up to 2318 f64 / 5546 f32; larger orders
- * fall back to the single-problem path per member). The B_i must not
- * overlap. Enqueued on `stream`. */
+ * Each CTA keeps a slice of B_i's right-hand sides in shared memory for the
+ * whole solve. f32: one launch for the batch, 32 right-hand sides per CTA up to
+ * order 1512, 16 or 8 up to 5546. f64: two launches (the inverses of the
+ * diagonal blocks, in chunks of members of at most 256 MB, then the solve), 32
+ * right-hand sides per CTA up to order 679 where their waves take less time than
+ * those of 16, 16 or 8 up to 2421. Larger orders fall back to the single-problem
+ * path per member. The B_i must not overlap. Enqueued on `stream`. */
 rb_status rb_strsm_batched_dev(rb_side side, rb_uplo uplo, rb_transpose trans, rb_diag diag, size_t m,
                                size_t n, float alpha, const float* a, size_t lda, size_t stride_a, float* b,
                                size_t ldb, size_t stride_b, size_t batch, void* stream, rb_error* err);
@@ -515,9 +517,10 @@ rb_status rb_gemm_grouped_plan_create(const rb_gemm_problem* problems, size_t co
 rb_status rb_gemm_grouped_plan_launch(void* plan, void* stream, rb_error* err);
 rb_status rb_gemm_grouped_plan_destroy(void* plan);
 
-/* Split-K autotuner of the grouped kernel. Times the candidate split
- * factors of every shape bucket (floor(log2) of m, n, k in 32..4096, per
- * dtype) on the current device, installs the winners process-wide and, if
+/* Autotuner of the grouped kernel's split-K factor and of the tile width of the
+ * Ozaki kernels on single CTAs. Times the candidates of every shape bucket
+ * (floor(log2) of m, n, k in 32..4096, per dtype; widths: f64 buckets that hold
+ * a shape whose call reads one) on the current device, installs the winners process-wide and, if
  * cache_path is not NULL, writes them there; *buckets_tuned = buckets timed.
  * Takes seconds and about 1.5 GB of device memory while it runs. Launches
  * planned after the call use the table, so a problem's result depends on its

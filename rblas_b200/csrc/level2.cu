@@ -8,14 +8,15 @@
 // A is the column-major view of its transpose, which swaps the two gemv
 // kernels and the roles of x and y in the rank-1 update.
 //   * "column sweep" gemv (y_r = sum_c A[r,c] x_c): a CTA per (row tile, range
-//     of columns), its warps on every eighth column; few columns: one thread
-//     per row.
-//   * "column dot" gemv (y_c = sum_r A[r,c] x_r): four columns at a time per
-//     CTA (per warp, for short ones) and row range, a fixed-order reduction.
+//     of columns), its warps on every eighth column; few columns, or rows
+//     enough to fill the GPU: one thread per four rows, all columns in order.
+//   * "column dot" gemv (y_c = sum_r A[r,c] x_r): two columns at a time per
+//     CTA and row range, one per warp where columns are short and many; a
+//     fixed-order reduction.
 //   * the ranges (S of them, only when there are too few tiles to fill the
 //     GPU) go through a workspace and a finalize pass in range order; a single
-//     range applies rblas's beta pass and alpha itself. Results do not depend
-//     on timing.
+//     range applies rblas's beta pass and alpha itself, unless y shares memory
+//     with x or A. Results do not depend on timing.
 // Within one range the terms are added in rblas's order (fma(a, x, acc) for
 // real, acc + a*x with rblas's complex multiply for complex), so a NoTrans
 // column-major call of fewer than kSweepSplit columns, or of more than

@@ -434,9 +434,9 @@ rb_status run_dev(const ColProblem<T>& p, rb_precision prec, cudaStream_t st, rb
         return run_precision_form(p, prec, st, err);
     }
     // Few C tiles of 128: small tiles, or with a long K the grouped kernel's
-    // deterministic split-K, fill the GPU. Either depends on the shape alone,
-    // and the small tiles sum K in the ranges that the other would split it
-    // into, so a call's bits repeat from call to call.
+    // deterministic split-K, fill the GPU. The split depends on the shape alone,
+    // and the small tiles sum K in the ranges that it would cut, so a call's bits
+    // depend neither on the route nor on how its operands are aligned.
     rb_gemm_problem gq;
     int k_range = 0;
     const int splits = p.split_ok ? plain_splits(p, &gq, &k_range) : 1;
