@@ -81,7 +81,7 @@ int main() {
                             }
                 }
     std::printf("%%.1f us\n", slowest);
-    return slowest < 15 ? 0 : 2;
+    return slowest < 25 ? 0 : 2;
 }
 """
 
